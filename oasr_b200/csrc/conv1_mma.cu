@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv1_mma_kernel(const __grid_con
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(t_empty + 2);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform for the compiler
   const int lane = threadIdx.x & 31;
   const int slots_per_b = p.TH * 4 * p.FH;
 
@@ -206,7 +206,8 @@ __global__ void __launch_bounds__(kThreads, 1) conv1_mma_kernel(const __grid_con
 
   if (warp == 0) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0) {
+    {
+      const bool issuer = ptx::elect_one();   // whole warp, one elected lane issues: see gemm.cu
       bool ok = true;
       int n = 0;
       const uint32_t b_addr = ptx::smem_u32(sB);
@@ -221,17 +222,16 @@ __global__ void __launch_bounds__(kThreads, 1) conv1_mma_kernel(const __grid_con
           const int acc = u & 1;
           if (!ptx::mbar_wait(&t_empty[acc], ((u >> 1) & 1) ^ 1u, abort_flag)) { ok = false; break; }
           ptx::tc_fence_after_sync();
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const uint64_t adesc = ptx::smem_desc_kmajor_sw128(a_addr + k * 32);
-            const uint64_t bdesc = ptx::smem_desc_kmajor_sw128(b_addr + half * 256 * kRowBytes + k * 32);
-            ptx::umma_f16(tmem_base + acc * 256, adesc, bdesc, kIdesc, k != 0 ? 1u : 0u);
+          const uint64_t ad = ptx::smem_desc_kmajor_sw128(a_addr), bd = ptx::smem_desc_kmajor_sw128(b_addr + half * 256 * kRowBytes);
+          if (issuer) {
+            ptx::umma_f16(tmem_base + acc * 256, ad, bd, kIdesc, 0u);
+            ptx::umma_f16(tmem_base + acc * 256, ad + 2, bd + 2, kIdesc, 1u);
+            ptx::umma_commit(&t_full[acc]);
           }
-          ptx::umma_commit(&t_full[acc]);
         }
-        if (ok) ptx::umma_commit(&a_empty[s]);
+        if (ok && issuer) ptx::umma_commit(&a_empty[s]);
       }
-      if (!ok && p.status) atomicOr(p.status, kStatusGemmMma);
+      if (!ok && issuer && p.status) atomicOr(p.status, kStatusGemmMma);
     }
     __syncwarp();
   } else if (warp <= kProdWarps) {

@@ -118,7 +118,7 @@ conv2_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 1);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform for the compiler
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -152,8 +152,9 @@ conv2_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const uint32_t a_box_bytes = static_cast<uint32_t>(p.conv_tpt * p.conv_f2 * 128);
 
   if (warp == 0) {
-    // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    // ------------------------------ TMA producer (whole warp, one elected lane issues: see gemm.cu) ------------------
+    {
+      const bool issuer = ptx::elect_one();
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -164,28 +165,31 @@ conv2_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         if (!mine.valid) mine = lead;
         for (int kb = 0; kb < p.num_k_blocks; ++kb) {
           if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
-          const uint32_t lead_full = ptx::map_to_cta(&full_bar[stage], 0);
-          if (cta_rank == 0) ptx::mbar_expect_tx(&full_bar[stage], 2 * (a_box_bytes + S::kBBytes));
           // K block kb = (tap, 64-channel block).  Tap (kh, kw) of output (t2, f2) reads input frame 2*t2 + kh, feature
           // 2*f2 + kw: parity plane (kh&1)*2 + (kw&1), rows (t2 + kh/2, f2 + kw/2) -- one dense box of tpt x f2 rows x 64
           // channels.  Rows past the box stay stale in shared memory: they only feed accumulator rows never stored.
           const int tap = kb / p.conv_cblocks, cb = kb - tap * p.conv_cblocks;
           const int kh = tap / 3, kw = tap - 3 * kh;
-          ptx::tma_load_5d_pair(sA + stage * S::kABytes, &tmap_a, cb * BK, kw >> 1, (kh & 1) * 2 + (kw & 1),
-                                mine.t0 + (kh >> 1), mine.b, lead_full);
+          if (issuer) {
+            const uint32_t lead_full = ptx::map_to_cta(&full_bar[stage], 0);
+            if (cta_rank == 0) ptx::mbar_expect_tx(&full_bar[stage], 2 * (a_box_bytes + S::kBBytes));
+            ptx::tma_load_5d_pair(sA + stage * S::kABytes, &tmap_a, cb * BK, kw >> 1, (kh & 1) * 2 + (kw & 1),
+                                  mine.t0 + (kh >> 1), mine.b, lead_full);
 #pragma unroll
-          for (int j = 0; j < kHalves; ++j)
-            ptx::tma_load_3d_pair(sB + stage * S::kBBytes + j * S::kBHalfBytes, &tmap_b, kb * BK,
-                                  j * kNI + static_cast<int>(cta_rank) * (kNI / 2), 0, lead_full);
+            for (int j = 0; j < kHalves; ++j)
+              ptx::tma_load_3d_pair(sB + stage * S::kBBytes + j * S::kBHalfBytes, &tmap_b, kb * BK,
+                                    j * kNI + static_cast<int>(cta_rank) * (kNI / 2), 0, lead_full);
+          }
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
       }
-      if (!ok && p.status) atomicOr(p.status, kStatusGemmProducer);
+      if (!ok && issuer && p.status) atomicOr(p.status, kStatusGemmProducer);
     }
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (leader CTA) -------------------
-    if (lane == 0 && cta_rank == 0) {
+    if (cta_rank == 0) {
+      const bool issuer = ptx::elect_one();
       int stage = 0;
       uint32_t phase = 0, acc_phase = 0;
       bool ok = true;
@@ -196,24 +200,23 @@ conv2_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         for (int kb = 0; kb < p.num_k_blocks; ++kb) {
           if (!ptx::mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
           ptx::tc_fence_after_sync();
-          const uint32_t a_addr = ptx::smem_u32(sA + stage * S::kABytes);
-          const uint32_t b_addr = ptx::smem_u32(sB + stage * S::kBBytes);
+          const uint64_t ad = ptx::smem_desc_kmajor_sw128(ptx::smem_u32(sA) + stage * S::kABytes);
+          const uint64_t bd = ptx::smem_desc_kmajor_sw128(ptx::smem_u32(sB) + stage * S::kBBytes);
+          if (issuer) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t adesc = ptx::smem_desc_kmajor_sw128(a_addr + k * UMMA_K * 2);
+            for (int k = 0; k < BK / UMMA_K; ++k) {     // 32 bytes of K per instruction = 2 descriptor units
 #pragma unroll
-            for (int j = 0; j < kHalves; ++j) {
-              const uint64_t bdesc = ptx::smem_desc_kmajor_sw128(b_addr + j * S::kBHalfBytes + k * UMMA_K * 2);
-              ptx::umma_f16_pair(tmem_base + j * kNI, adesc, bdesc, kIdesc, (kb | k) != 0 ? 1u : 0u);
+              for (int j = 0; j < kHalves; ++j)
+                ptx::umma_f16_pair(tmem_base + j * kNI, ad + 2 * k, bd + j * (S::kBHalfBytes >> 4) + 2 * k, kIdesc, (kb | k) != 0 ? 1u : 0u);
             }
+            ptx::umma_commit_pair(&empty_bar[stage], 3);
           }
-          ptx::umma_commit_pair(&empty_bar[stage], 3);
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
-        if (ok) ptx::umma_commit_pair(tfull_bar, 3);
+        if (ok && issuer) ptx::umma_commit_pair(tfull_bar, 3);
         acc_phase ^= 1u;
       }
-      if (!ok && p.status) atomicOr(p.status, kStatusGemmMma);
+      if (!ok && issuer && p.status) atomicOr(p.status, kStatusGemmMma);
     }
     __syncwarp();
   } else {

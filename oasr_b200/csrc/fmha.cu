@@ -199,7 +199,7 @@ fmha_tcgen05_kernel(const __grid_constant__ Maps maps, const Params p) {
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + S::kNumBars);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform for the compiler
   const int lane = threadIdx.x & 31;
 
   // Barrier block: q_full, kv_full[2], kv_empty[2], s_full[2], s_free[2], p_full[2], po_done[2] = 13.
@@ -229,11 +229,13 @@ fmha_tcgen05_kernel(const __grid_constant__ Maps maps, const Params p) {
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 4) {
-    // =================== TMA producer + MMA issuer (one thread) ===================
-    if (lane == 0) {
+    // =================== TMA producer + MMA issuer (whole warp, one elected lane issues: see gemm.cu) ===================
+    {
+      const bool issuer = ptx::elect_one();
       bool ok = true;
       constexpr uint32_t kKVBytes = (kAtoms + S::kVAtoms) * kAtomBytes;
       auto load_kv = [&](int t /*tile index within [0,nkv)*/, int b) {
+        if (!issuer) return;
         const int key0 = (tile_begin + t) * BKV;
         ptx::mbar_expect_tx(&kv_full[b], kKVBytes);
         uint8_t* dk = sK + b * kAtoms * kAtomBytes;
@@ -277,37 +279,41 @@ fmha_tcgen05_kernel(const __grid_constant__ Maps maps, const Params p) {
         const uint32_t a_addr = ptx::smem_u32(sQ);
         const uint32_t b_addr = ptx::smem_u32(sK + b * kAtoms * kAtomBytes);
         const uint32_t d_tmem = tmem_base + kColS + b * BKV;
+        const uint64_t ad = ptx::smem_desc_kmajor_sw128(a_addr), bd = ptx::smem_desc_kmajor_sw128(b_addr);
+        if (issuer) {
 #pragma unroll
-        for (int kk = 0; kk < kAtoms * 4; ++kk) {
-          const uint32_t off = (kk / 4) * kAtomBytes + (kk % 4) * 32;
-          ptx::umma_f16(d_tmem, ptx::smem_desc_kmajor_sw128(a_addr + off), ptx::smem_desc_kmajor_sw128(b_addr + off),
-                        kIdescQK, kk != 0 ? 1u : 0u);
+          for (int kk = 0; kk < kAtoms * 4; ++kk) {
+            const uint32_t off = ((kk / 4) * kAtomBytes + (kk % 4) * 32) >> 4;
+            ptx::umma_f16(d_tmem, ad + off, bd + off, kIdescQK, kk != 0 ? 1u : 0u);
+          }
+          ptx::umma_commit(&s_full[b]);
         }
-        ptx::umma_commit(&s_full[b]);
       };
       auto issue_pv = [&](int b) {
         const uint32_t a_addr = ptx::smem_u32(sP + b * 2 * kAtomBytes);
         const uint32_t b_addr = ptx::smem_u32(sV + b * S::kVAtoms * kAtomBytes);
         const uint32_t d_tmem = tmem_base + kColO + b * D;
+        // V tile: rows = keys (128 B each), 16 keys per MMA = 2048 B; atoms along D are kAtomBytes apart
+        const uint64_t ad = ptx::smem_desc_kmajor_sw128(a_addr), bd = ptx::smem_desc_mnmajor_sw128(b_addr, kAtomBytes, 1024);
+        if (issuer) {
 #pragma unroll
-        for (int kk = 0; kk < BKV / 16; ++kk) {
-          const uint64_t adesc = ptx::smem_desc_kmajor_sw128(a_addr + (kk / 4) * kAtomBytes + (kk % 4) * 32);
-          // V tile: rows = keys (128 B each), 16 keys per MMA = 2048 B; atoms along D are kAtomBytes apart
-          const uint64_t bdesc = ptx::smem_desc_mnmajor_sw128(b_addr + kk * 2048, kAtomBytes, 1024);
-          ptx::umma_f16(d_tmem, adesc, bdesc, kIdescPV, kk != 0 ? 1u : 0u);
+          for (int kk = 0; kk < BKV / 16; ++kk)
+            ptx::umma_f16(d_tmem, ad + (((kk / 4) * kAtomBytes + (kk % 4) * 32) >> 4), bd + ((kk * 2048) >> 4), kIdescPV, kk != 0 ? 1u : 0u);
+          ptx::umma_commit(&po_done[b]);
+          ptx::umma_commit(&kv_empty[b]);
         }
-        ptx::umma_commit(&po_done[b]);
-        ptx::umma_commit(&kv_empty[b]);
       };
 
       // Q tile (+ second atom)
-      ptx::mbar_expect_tx(q_full, kAtoms * kAtomBytes);
-      if (p.relpos) {
-        ptx::tma_load_4d(sQ, &maps.q, 0, q_row_c1, h, q_c3, q_full);
-        ptx::tma_load_4d(sQ + kAtomBytes, &maps.q2, 0, q_row_c1, h, q_c3, q_full);
-      } else {
+      if (issuer) {
+        ptx::mbar_expect_tx(q_full, kAtoms * kAtomBytes);
+        if (p.relpos) {
+          ptx::tma_load_4d(sQ, &maps.q, 0, q_row_c1, h, q_c3, q_full);
+          ptx::tma_load_4d(sQ + kAtomBytes, &maps.q2, 0, q_row_c1, h, q_c3, q_full);
+        } else {
 #pragma unroll
-        for (int a = 0; a < kAtoms; ++a) ptx::tma_load_4d(sQ + a * kAtomBytes, &maps.q, a * 64, q_row_c1, h, q_c3, q_full);
+          for (int a = 0; a < kAtoms; ++a) ptx::tma_load_4d(sQ + a * kAtomBytes, &maps.q, a * 64, q_row_c1, h, q_c3, q_full);
+        }
       }
       load_kv(0, 0);
       if (nkv > 1) load_kv(1, 1);
@@ -340,7 +346,7 @@ fmha_tcgen05_kernel(const __grid_constant__ Maps maps, const Params p) {
           load_kv(j + 2, b);
         }
       }
-      if (!ok && p.status) atomicOr(p.status, kStatusFmhaMma);
+      if (!ok && issuer && p.status) atomicOr(p.status, kStatusFmhaMma);
     }
     __syncwarp();
   } else {

@@ -173,7 +173,7 @@ fmha_relpos64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kNumBars);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // warp-uniform for the compiler
   if (threadIdx.x == 0) {
     ptx::mbar_init(q_full, 1);
     for (int i = 0; i < 2; ++i) {
@@ -234,9 +234,13 @@ fmha_relpos64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   };
   constexpr uint32_t kIdleLimit = 1u << 24;   // polls without progress before the role gives up (a sleep between polls
                                               // measured slower: 45.4 / 46.0 / 46.3 / 46.7 us per launch for 0 / 20 / 40 / 100 ns)
+  // Both run as whole warps with one elected lane issuing (see gemm.cu); a barrier counts as complete as soon as one lane
+  // has seen it, so that all lanes take the same way.
+  auto done = [&](uint64_t* bar, uint32_t parity) -> bool { return __any_sync(0xffffffffu, ptx::mbar_test(bar, parity)) != 0; };
   if (warp == 5) {
-    // =================== TMA producer (one thread) ===================
-    if (lane == 0) {
+    // =================== TMA producer ===================
+    {
+      const bool issuer = ptx::elect_one();
       bool ok = true;
       Cursor ck, cv;
       start(ck);
@@ -248,29 +252,33 @@ fmha_relpos64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
           const int gg = ck.g, b = gg & 1;
           // the stage's last user was Q.K^T of tile gg - 2; Q is single-buffered: a new item's Q waits for the
           // previous item's last Q.K^T (tile gg - 1)
-          bool ready = gg < 2 || ptx::mbar_test(&k_empty[b], ((gg - 2) >> 1) & 1u);
-          if (ready && ck.j == 0 && ck.ord > 0) ready = ptx::mbar_test(&k_empty[(gg - 1) & 1], ((gg - 1) >> 1) & 1u);
+          bool ready = gg < 2 || done(&k_empty[b], ((gg - 2) >> 1) & 1u);
+          if (ready && ck.j == 0 && ck.ord > 0) ready = done(&k_empty[(gg - 1) & 1], ((gg - 1) >> 1) & 1u);
           if (ready) {
             const Item& w = ck.w;
-            if (ck.j == 0) {
-              ptx::mbar_expect_tx(q_full, kQBytes);
-              ptx::tma_load_4d(sQ, &map_q, 0, w.row0 + w.q0, w.h, 0, q_full);
-              ptx::tma_load_4d(sQ + 128 * 128, &map_q2, 0, w.row0 + w.q0, w.h, 0, q_full);
-            }
             const int key0 = ck.j * BKV;
-            ptx::mbar_expect_tx(&k_full[b], kKBytes);
-            uint8_t* dk = sK + b * kKBytes;
-            ptx::tma_load_4d(dk, &map_k, 0, w.row0 + key0, w.h, 0, &k_full[b]);
-            ptx::tma_load_4d(dk + BKV * 128, &map_pos, 0, key0, w.h, 0, &k_full[b]);
+            if (issuer) {
+              if (ck.j == 0) {
+                ptx::mbar_expect_tx(q_full, kQBytes);
+                ptx::tma_load_4d(sQ, &map_q, 0, w.row0 + w.q0, w.h, 0, q_full);
+                ptx::tma_load_4d(sQ + 128 * 128, &map_q2, 0, w.row0 + w.q0, w.h, 0, q_full);
+              }
+              ptx::mbar_expect_tx(&k_full[b], kKBytes);
+              uint8_t* dk = sK + b * kKBytes;
+              ptx::tma_load_4d(dk, &map_k, 0, w.row0 + key0, w.h, 0, &k_full[b]);
+              ptx::tma_load_4d(dk + BKV * 128, &map_pos, 0, key0, w.h, 0, &k_full[b]);
+            }
             advance(ck);
             progress = true;
           }
         }
         if (cv.it < n_items) {
           const int gg = cv.g, b = gg & 1;
-          if (gg < 2 || ptx::mbar_test(&v_empty[b], ((gg - 2) >> 1) & 1u)) {   // P.V of tile gg - 2 finished
-            ptx::mbar_expect_tx(&v_full[b], kVBytes);
-            ptx::tma_load_4d(sV + b * kVBytes, &map_v, 0, cv.w.row0 + cv.j * BKV, cv.w.h, 0, &v_full[b]);
+          if (gg < 2 || done(&v_empty[b], ((gg - 2) >> 1) & 1u)) {   // P.V of tile gg - 2 finished
+            if (issuer) {
+              ptx::mbar_expect_tx(&v_full[b], kVBytes);
+              ptx::tma_load_4d(sV + b * kVBytes, &map_v, 0, cv.w.row0 + cv.j * BKV, cv.w.h, 0, &v_full[b]);
+            }
             advance(cv);
             progress = true;
           }
@@ -282,38 +290,41 @@ fmha_relpos64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
           else if ((idle & 63u) == 63u && *abort_flag) ok = false;
         }
       }
-      if (!ok && p.status) atomicOr(p.status, kStatusFmhaMma);
+      if (!ok && issuer && p.status) atomicOr(p.status, kStatusFmhaMma);
     }
     __syncwarp();
   } else if (warp == 4) {
-    // =================== MMA issuer (one thread) ===================
-    if (lane == 0) {
+    // =================== MMA issuer ===================
+    {
+      const bool issuer = ptx::elect_one();
       bool ok = true;
       auto issue_qk = [&](int b) {   // S[b] = [q+u | q+v] . [k | pos]^T : K = 128 in eight steps of 16
         const uint32_t a_addr = ptx::smem_u32(sQ);
         const uint32_t b_addr = ptx::smem_u32(sK + b * kKBytes);
         const uint32_t d_tmem = tmem_base + kColS + b * BKV;
+        const uint64_t ad = ptx::smem_desc_kmajor_sw128(a_addr), bd = ptx::smem_desc_kmajor_sw128(b_addr);
+        if (issuer) {
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint64_t adesc = ptx::smem_desc_kmajor_sw128(a_addr + (kk / 4) * (128 * 128) + (kk % 4) * 32);
-          const uint64_t bdesc = ptx::smem_desc_kmajor_sw128(b_addr + (kk / 4) * (BKV * 128) + (kk % 4) * 32);
-          ptx::umma_f16(d_tmem, adesc, bdesc, kIdescQK, kk != 0 ? 1u : 0u);
+          for (int kk = 0; kk < 8; ++kk)
+            ptx::umma_f16(d_tmem, ad + (((kk / 4) * (128 * 128) + (kk % 4) * 32) >> 4), bd + (((kk / 4) * (BKV * 128) + (kk % 4) * 32) >> 4),
+                          kIdescQK, kk != 0 ? 1u : 0u);
+          ptx::umma_commit(&s_full[b]);
+          ptx::umma_commit(&k_empty[b]);
         }
-        ptx::umma_commit(&s_full[b]);
-        ptx::umma_commit(&k_empty[b]);
       };
       auto issue_pv = [&](int b, bool first) {   // O (+)= P . V_b : K = 64 keys in four steps of 16
         const uint32_t a_addr = ptx::smem_u32(sP);
         const uint32_t b_addr = ptx::smem_u32(sV + b * kVBytes);
         const uint32_t d_tmem = tmem_base + kColO;
+        const uint64_t ad = ptx::smem_desc_kmajor_sw128(a_addr);
+        const uint64_t bd = ptx::smem_desc_mnmajor_sw128(b_addr, ptx::smem_u32(sOnes) - b_addr, 1024);
+        if (issuer) {
 #pragma unroll
-        for (int kk = 0; kk < BKV / 16; ++kk) {
-          const uint64_t adesc = ptx::smem_desc_kmajor_sw128(a_addr + kk * 32);
-          const uint64_t bdesc = ptx::smem_desc_mnmajor_sw128(b_addr + kk * 2048, ptx::smem_u32(sOnes) - b_addr, 1024);
-          ptx::umma_f16(d_tmem, adesc, bdesc, kIdescPV, (!first || kk != 0) ? 1u : 0u);
+          for (int kk = 0; kk < BKV / 16; ++kk)
+            ptx::umma_f16(d_tmem, ad + ((kk * 32) >> 4), bd + ((kk * 2048) >> 4), kIdescPV, (!first || kk != 0) ? 1u : 0u);
+          ptx::umma_commit(po_done);
+          ptx::umma_commit(&v_empty[b]);
         }
-        ptx::umma_commit(po_done);
-        ptx::umma_commit(&v_empty[b]);
       };
       Cursor cq, cp;   // next scores, next P.V
       start(cq);
@@ -327,8 +338,8 @@ fmha_relpos64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
           // next item too: its Q was requested when this item's last Q.K^T finished.
           const int b = cq.g & 1;
           const uint32_t ph = (cq.g >> 1) & 1u;
-          if (ptx::mbar_test(&k_full[b], ph) && ptx::mbar_test(&s_free[b], ph ^ 1u) &&
-              (cq.j != 0 || ptx::mbar_test(q_full, static_cast<uint32_t>(cq.ord) & 1u))) {
+          if (done(&k_full[b], ph) && done(&s_free[b], ph ^ 1u) &&
+              (cq.j != 0 || done(q_full, static_cast<uint32_t>(cq.ord) & 1u))) {
             ptx::tc_fence_after_sync();
             issue_qk(b);
             advance(cq);
@@ -338,8 +349,8 @@ fmha_relpos64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         if (cp.g < cq.g) {
           // P.V of tile g: P written, V landed, and (first tile of an item) every row has read the previous item's O
           const int b = cp.g & 1;
-          if (ptx::mbar_test(p_full, static_cast<uint32_t>(cp.g) & 1u) && ptx::mbar_test(&v_full[b], (cp.g >> 1) & 1u) &&
-              (cp.j != 0 || cp.ord == 0 || ptx::mbar_test(o_free, static_cast<uint32_t>(cp.ord - 1) & 1u))) {
+          if (done(p_full, static_cast<uint32_t>(cp.g) & 1u) && done(&v_full[b], (cp.g >> 1) & 1u) &&
+              (cp.j != 0 || cp.ord == 0 || done(o_free, static_cast<uint32_t>(cp.ord - 1) & 1u))) {
             ptx::tc_fence_after_sync();
             issue_pv(b, cp.j == 0);
             advance(cp);

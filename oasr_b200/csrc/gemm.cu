@@ -274,7 +274,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmap_a, const CUten
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform for the compiler
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -315,28 +315,31 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmap_a, const CUten
   Scheduler<kSched, BN, kCtas> sched(p);
   sched.rank = cta_rank;
 
+  // Producer and issuer run as whole warps with one elected lane issuing: loop state and descriptors then stay in uniform
+  // registers, which is where the TMA and MMA instructions take them from.  Under `lane == 0` every operand is moved there
+  // per instruction (0.14k clocks per MMA, more than a 128 x 256 MMA itself takes).
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      Tile t;
-      bool ok = true;
-      for (int iter = 0; ok && sched.get(iter, t); ++iter) {
-        for (int kb = 0; kb < p.num_k_blocks; ++kb) {
-          if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
+    const bool issuer = ptx::elect_one();
+    int stage = 0;
+    uint32_t phase = 0;
+    Tile t;
+    bool ok = true;
+    for (int iter = 0; ok && sched.get(iter, t); ++iter) {
+      for (int kb = 0; kb < p.num_k_blocks; ++kb) {
+        if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
+        uint8_t* a_dst = sA + stage * S::kABytes;
+        uint8_t* b_dst = sB + stage * S::kBBytes;
+        if (issuer) {
           if constexpr (kCtas == 2) {
             // both CTAs' bytes are credited to the leader's barrier; only the leader arrives on it
             const uint32_t lead_full = ptx::map_to_cta(&full_bar[stage], 0);
             if (cta_rank == 0) ptx::mbar_expect_tx(&full_bar[stage], 2 * (S::kABytes + S::kBBytes));
-            ptx::tma_load_3d_pair(sA + stage * S::kABytes, &tmap_a, kb * BK, t.a_row, t.a_batch, lead_full);
+            ptx::tma_load_3d_pair(a_dst, &tmap_a, kb * BK, t.a_row, t.a_batch, lead_full);
             int b_row = t.b_row;
             if constexpr (kEpi == kEpiGlu) b_row = (cta_rank == 0 ? 0 : p.N) + t.n0 / 2;  // value | gate rows
-            ptx::tma_load_3d_pair(sB + stage * S::kBBytes, &tmap_b, kb * BK, b_row, t.b_batch, lead_full);
-            if (++stage == kStages) { stage = 0; phase ^= 1u; }
-            continue;
-          }
-          if constexpr (kSched == kSchedConv) {
+            ptx::tma_load_3d_pair(b_dst, &tmap_b, kb * BK, b_row, t.b_batch, lead_full);
+          } else if constexpr (kSched == kSchedConv) {
             // K block kb = (tap, 64-channel block).  Tap (kh, kw) of output (t2, f2) reads input frame
             // 2*t2 + kh, feature 2*f2 + kw: parity plane (kh&1)*2 + (kw&1), rows (t2 + kh/2, f2 + kw/2) --
             // one dense box of conv_tpt x conv_f2 rows x 64 channels.  Rows past the box stay stale in
@@ -344,31 +347,30 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmap_a, const CUten
             const int tap = kb / p.conv_cblocks, cb = kb - tap * p.conv_cblocks;
             const int kh = tap / 3, kw = tap - 3 * kh;
             ptx::mbar_expect_tx(&full_bar[stage], static_cast<uint32_t>(p.conv_tpt * p.conv_f2 * 128) + S::kBBytes);
-            ptx::tma_load_5d(sA + stage * S::kABytes, &tmap_a, cb * BK, kw >> 1, (kh & 1) * 2 + (kw & 1),
-                             t.a_row + (kh >> 1), t.a_batch, &full_bar[stage]);
-            ptx::tma_load_3d(sB + stage * S::kBBytes, &tmap_b, kb * BK, t.b_row, t.b_batch, &full_bar[stage]);
-            if (++stage == kStages) { stage = 0; phase ^= 1u; }
-            continue;
-          }
-          ptx::mbar_expect_tx(&full_bar[stage], S::kABytes + S::kBBytes);
-          ptx::tma_load_3d(sA + stage * S::kABytes, &tmap_a, kb * kBKe, t.a_row, t.a_batch, &full_bar[stage]);
-          if constexpr (kEpi == kEpiGlu) {
-            // value rows [n0/2, +BN/2) and gate rows [N + n0/2, +BN/2) of the 2N-row weight
-            ptx::tma_load_3d(sB + stage * S::kBBytes, &tmap_b, kb * kBKe, t.b_row / 2, t.b_batch, &full_bar[stage]);
-            ptx::tma_load_3d(sB + stage * S::kBBytes + S::kBBytes / 2, &tmap_b, kb * kBKe, p.N + t.b_row / 2,
-                             t.b_batch, &full_bar[stage]);
+            ptx::tma_load_5d(a_dst, &tmap_a, cb * BK, kw >> 1, (kh & 1) * 2 + (kw & 1), t.a_row + (kh >> 1), t.a_batch,
+                             &full_bar[stage]);
+            ptx::tma_load_3d(b_dst, &tmap_b, kb * BK, t.b_row, t.b_batch, &full_bar[stage]);
           } else {
-            ptx::tma_load_3d(sB + stage * S::kBBytes, &tmap_b, kb * kBKe, t.b_row, t.b_batch, &full_bar[stage]);
+            ptx::mbar_expect_tx(&full_bar[stage], S::kABytes + S::kBBytes);
+            ptx::tma_load_3d(a_dst, &tmap_a, kb * kBKe, t.a_row, t.a_batch, &full_bar[stage]);
+            if constexpr (kEpi == kEpiGlu) {
+              // value rows [n0/2, +BN/2) and gate rows [N + n0/2, +BN/2) of the 2N-row weight
+              ptx::tma_load_3d(b_dst, &tmap_b, kb * kBKe, t.b_row / 2, t.b_batch, &full_bar[stage]);
+              ptx::tma_load_3d(b_dst + S::kBBytes / 2, &tmap_b, kb * kBKe, p.N + t.b_row / 2, t.b_batch, &full_bar[stage]);
+            } else {
+              ptx::tma_load_3d(b_dst, &tmap_b, kb * kBKe, t.b_row, t.b_batch, &full_bar[stage]);
+            }
           }
-          if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
+        if (++stage == kStages) { stage = 0; phase ^= 1u; }
       }
-      if (!ok && p.status) atomicOr(p.status, kStatusGemmProducer);
     }
+    if (!ok && issuer && p.status) atomicOr(p.status, kStatusGemmProducer);
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
-    if (lane == 0 && cta_rank == 0) {
+    if (cta_rank == 0) {
+      const bool issuer = ptx::elect_one();
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -381,27 +383,28 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmap_a, const CUten
         for (int kb = 0; kb < p.num_k_blocks; ++kb) {
           if (!ptx::mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
           ptx::tc_fence_after_sync();
-          const uint32_t a_addr = ptx::smem_u32(sA + stage * S::kABytes);
-          const uint32_t b_addr = ptx::smem_u32(sB + stage * S::kBBytes);
+          const uint64_t ad = ptx::smem_desc_kmajor_sw128(ptx::smem_u32(sA) + stage * S::kABytes);
+          const uint64_t bd = ptx::smem_desc_kmajor_sw128(ptx::smem_u32(sB) + stage * S::kBBytes);
+          if (issuer) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t adesc = ptx::smem_desc_kmajor_sw128(a_addr + k * UMMA_K * 2);
-            const uint64_t bdesc = ptx::smem_desc_kmajor_sw128(b_addr + k * UMMA_K * 2);
-            if constexpr (kCtas == 2) ptx::umma_f16_pair(d_tmem, adesc, bdesc, kIdesc, (kb | k) != 0 ? 1u : 0u);
-            else if constexpr (kKind == 1) ptx::umma_f8(d_tmem, adesc, bdesc, kIdesc, (kb | k) != 0 ? 1u : 0u);
-            else if constexpr (kKind == 2) ptx::umma_i8(d_tmem, adesc, bdesc, kIdesc, (kb | k) != 0 ? 1u : 0u);
-            else ptx::umma_f16(d_tmem, adesc, bdesc, kIdesc, (kb | k) != 0 ? 1u : 0u);
+            for (int k = 0; k < BK / UMMA_K; ++k) {   // 32 bytes of K per instruction = 2 descriptor units
+              const uint32_t accumulate = (kb | k) != 0 ? 1u : 0u;
+              if constexpr (kCtas == 2) ptx::umma_f16_pair(d_tmem, ad + 2 * k, bd + 2 * k, kIdesc, accumulate);
+              else if constexpr (kKind == 1) ptx::umma_f8(d_tmem, ad + 2 * k, bd + 2 * k, kIdesc, accumulate);
+              else if constexpr (kKind == 2) ptx::umma_i8(d_tmem, ad + 2 * k, bd + 2 * k, kIdesc, accumulate);
+              else ptx::umma_f16(d_tmem, ad + 2 * k, bd + 2 * k, kIdesc, accumulate);
+            }
+            if constexpr (kCtas == 2) ptx::umma_commit_pair(&empty_bar[stage], 3);  // frees the stage in both CTAs
+            else ptx::umma_commit(&empty_bar[stage]);
           }
-          if constexpr (kCtas == 2) ptx::umma_commit_pair(&empty_bar[stage], 3);  // frees the stage in both CTAs
-          else ptx::umma_commit(&empty_bar[stage]);
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
-        if (ok) {
+        if (ok && issuer) {
           if constexpr (kCtas == 2) ptx::umma_commit_pair(&tfull_bar[acc], 3);
           else ptx::umma_commit(&tfull_bar[acc]);
         }
       }
-      if (!ok && p.status) atomicOr(p.status, kStatusGemmMma);
+      if (!ok && issuer && p.status) atomicOr(p.status, kStatusGemmMma);
     }
     __syncwarp();
   } else {
