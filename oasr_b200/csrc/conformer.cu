@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "gemm_small.cuh"
 
 namespace ob {
 namespace {
@@ -31,6 +32,9 @@ struct Workspace {
 };
 
 int64_t align256(int64_t x) { return (x + 255) / 256 * 256; }
+
+constexpr Chain kFirst{0, 1};   // the executor's first GEMM, and the ones behind it (gemm_small.cuh)
+constexpr Chain kInner{1, 0};
 
 struct ChunkWorkspace {
   float* res;
@@ -208,8 +212,8 @@ int oasr_b200_conformer_encode_packed(const oasr_b200_conformer_model* model, co
 #define OB_LINEAR(label, fl, out, in, wt, bs, lay, qi, N, K, act, glu)                                              \
   do {                                                                                                              \
     if (qk == 0) {                                                                                                  \
-      if (glu) OB_STEP("gemm_glu " label, fl, oasr_b200_gemm_glu(out, in, wt, bs, M, N, K, dt, stream));              \
-      else OB_STEP("gemm " label, fl, oasr_b200_gemm(out, in, wt, bs, M, N, K, act, dt, stream));                    \
+      if (glu) OB_STEP("gemm_glu " label, fl, gemm_glu_op(out, in, wt, bs, M, N, K, dt, stream, kInner));             \
+      else OB_STEP("gemm " label, fl, gemm_op(out, in, wt, bs, M, N, K, act, dt, stream, kInner));                   \
     } else {                                                                                                        \
       OB_STEP("quantize_rows", 0, oasr_b200_quantize_rows(w.q8, w.qs, in, M, K, qk, dt, stream));                     \
       OB_STEP("gemm_q8 " label, fl, oasr_b200_gemm_q8(out, w.q8, w.qs, (lay).q_w[qi], (lay).q_s[qi], bs, M, N, K, act, glu, qk, dt, stream)); \
@@ -228,6 +232,9 @@ int oasr_b200_conformer_encode_packed(const oasr_b200_conformer_model* model, co
   const bool fills = g_fused_addnorm == 2 || pairs * 5 >= rounds * slots * 4;
   const bool fuse = qk == 0 && g_fused_addnorm != 0 && fills && oasr_b200_gemm_add_norm_supported(d, d) != 0 &&
                     oasr_b200_gemm_add_norm_supported(d, m.ffn) != 0 && oasr_b200_gemm_add_norm_supported(d, m.embed_in) != 0;
+  // Few rows: the Linear adds into the fp32 residual stream itself (its few output bytes cost nothing there) and the norm
+  // reads the sum, which is then never rounded to 16 bits.
+  const bool resid = !fuse && qk == 0 && M <= gsm::kMaxRows;
   // add + norm; with an 8-bit kind (and an unsplit h) the kernel also leaves the quantised row of h in w.q8 / w.qs for
   // the Linear that reads h next, which then skips its own quantisation launch (OB_LINEAR_H)
 #define OB_ADD_NORM(hout, rout, rin, y_, alpha, mode, wa, ba, wb, bb, eps_, split)                                      \
@@ -243,6 +250,9 @@ int oasr_b200_conformer_encode_packed(const oasr_b200_conformer_model* model, co
     if (fuse) {                                                                                                     \
       OB_STEP("gemm_addnorm " label, fl, oasr_b200_gemm_add_norm_f32(hout, w.res, rin, in, wt, bs, M, d, K, alpha, mode, wa, ba, \
                                                                     wb, bb, eps_, split, dt, stream));              \
+    } else if (resid) {                                                                                             \
+      OB_STEP("gemm " label, fl, gemm_residual_f32_op(w.res, rin, in, wt, bs, M, d, K, alpha, dt, stream, kInner));   \
+      OB_ADD_NORM(hout, (mode) == 2 ? w.res : nullptr, w.res, nullptr, 0.0, mode, wa, ba, wb, bb, eps_, split);       \
     } else {                                                                                                        \
       OB_LINEAR(label, fl, w.y, in, wt, bs, lay, qi, d, K, OASR_ACT_NONE, 0);                                        \
       OB_ADD_NORM(hout, w.res, rin, w.y, alpha, mode, wa, ba, wb, bb, eps_, split);                                   \
@@ -259,7 +269,7 @@ int oasr_b200_conformer_encode_packed(const oasr_b200_conformer_model* model, co
   } else {
   // The embedding is the first value of the fp32 residual stream: it goes there in fp32 straight from the GEMM's
   // epilogue (a 16-bit round trip here would put a rounding error on every element that all layers then carry).
-  OB_STEP("gemm embed", 2.0 * M * d * m.embed_in, oasr_b200_gemm_residual_f32(w.res, nullptr, rows, m.embed_w, m.embed_b, M, d, m.embed_in, 1.0, dt, stream));
+  OB_STEP("gemm embed", 2.0 * M * d * m.embed_in, gemm_residual_f32_op(w.res, nullptr, rows, m.embed_w, m.embed_b, M, d, m.embed_in, 1.0, dt, stream, kFirst));
   if (m.embed_ln_w) {
     OB_ADD_NORM(w.h, w.res, w.res, nullptr, 0.0, 2, m.embed_ln_w, m.embed_ln_b, ly[0].norm_ff_macaron_w, ly[0].norm_ff_macaron_b, 1e-5, 0);
   } else {
@@ -273,7 +283,7 @@ int oasr_b200_conformer_encode_packed(const oasr_b200_conformer_model* model, co
     att_plan = w.att_plan;
   }
   // linear_pos of every layer in one GEMM: (max_seg, d) x (L*d, d)^T
-  OB_STEP("gemm linear_pos", 2.0 * max_seg * L * d * d, oasr_b200_gemm(w.pos, m.pe, m.pos_w_all, nullptr, max_seg, L * d, d, OASR_ACT_NONE, dt, stream));
+  OB_STEP("gemm linear_pos", 2.0 * max_seg * L * d * d, gemm_op(w.pos, m.pe, m.pos_w_all, nullptr, max_seg, L * d, d, OASR_ACT_NONE, dt, stream, kInner));
 
   for (int64_t i = 0; i < L; ++i) {
     const oasr_b200_conformer_layer& l = ly[i];
@@ -283,7 +293,7 @@ int oasr_b200_conformer_encode_packed(const oasr_b200_conformer_model* model, co
                       l.norm_mha_b, nullptr, nullptr, m.eps, 0);
     // relative-position self-attention
     if (qkv_dup) {   // [Wq;Wk;Wv] are rows d.. of [Wq;Wq;Wk;Wv]: the query block once, stored as q+u and q+v
-      OB_STEP("gemm qkv4", 2.0 * M * 3 * d * d, oasr_b200_gemm_dup_first(w.qkv4, w.h, static_cast<const uint8_t*>(l.qkv4_w) + d * d * 2, l.qkv4_b, M, 3 * d, d, d, dt, stream));
+      OB_STEP("gemm qkv4", 2.0 * M * 3 * d * d, gemm_dup_first_op(w.qkv4, w.h, static_cast<const uint8_t*>(l.qkv4_w) + d * d * 2, l.qkv4_b, M, 3 * d, d, d, dt, stream, kInner));
     } else {
       OB_LINEAR_H("qkv4", 2.0 * M * 3 * d * d /* algorithmic: the query block is issued twice */, w.qkv4, l.qkv4_w, l.qkv4_b, l, 2, 4 * d, OASR_ACT_NONE, 0);
     }
@@ -309,8 +319,8 @@ int oasr_b200_conformer_encode_packed(const oasr_b200_conformer_model* model, co
     }
   }
   if (log_probs || argmax) {   // log_probs == NULL: token-only head, one vocabulary sweep, no log-prob write
-    OB_STEP("gemm_log_softmax", 2.0 * M * m.vocab_padded * d /* algorithmic; issued with the input split in two 16-bit terms (K = 2d) */, oasr_b200_gemm_log_softmax(log_probs, w.h3, m.ctc_w, m.ctc_b, M, m.vocab_padded, 2 * d, dt, OASR_DT_F32,
-                                       argmax, stream));
+    OB_STEP("gemm_log_softmax", 2.0 * M * m.vocab_padded * d /* algorithmic; issued with the input split in two 16-bit terms (K = 2d) */, gemm_log_softmax_op(log_probs, w.h3, m.ctc_w, m.ctc_b, M, m.vocab_padded, 2 * d, dt, OASR_DT_F32,
+                                       argmax, stream, kInner));
   }
   return OASR_OK;
 }
@@ -415,8 +425,8 @@ int oasr_b200_conformer_chunk_paged(const oasr_b200_conformer_model* model, cons
 #define OB_CHUNK_LINEAR(label, fl, out, in, wt, bs, lay, qi, R, N, K, act, glu)                                       \
   do {                                                                                                                \
     if (qk == 0) {                                                                                                    \
-      if (glu) OB_STEP("gemm_glu " label, fl, oasr_b200_gemm_glu(out, in, wt, bs, R, N, K, dt, stream));                \
-      else OB_STEP("gemm " label, fl, oasr_b200_gemm(out, in, wt, bs, R, N, K, act, dt, stream));                      \
+      if (glu) OB_STEP("gemm_glu " label, fl, gemm_glu_op(out, in, wt, bs, R, N, K, dt, stream, kInner));               \
+      else OB_STEP("gemm " label, fl, gemm_op(out, in, wt, bs, R, N, K, act, dt, stream, kInner));                     \
     } else {                                                                                                          \
       OB_STEP("quantize_rows", 0, oasr_b200_quantize_rows(w.q8, w.qs, in, R, K, qk, dt, stream));                       \
       OB_STEP("gemm_q8 " label, fl, oasr_b200_gemm_q8(out, w.q8, w.qs, (lay).q_w[qi], (lay).q_s[qi], bs, R, N, K, act, glu, qk, dt, stream)); \
@@ -429,8 +439,20 @@ int oasr_b200_conformer_chunk_paged(const oasr_b200_conformer_model* model, cons
     if (qk == 0) OB_CHUNK_LINEAR(label, fl, out, w.h, wt, bs, lay, qi, M, N, d, act, 0);                                \
     else OB_STEP("gemm_q8 " label, fl, oasr_b200_gemm_q8(out, w.q8, w.qs, (lay).q_w[qi], (lay).q_s[qi], bs, M, N, d, act, 0, qk, dt, stream)); \
   } while (0)
+  // last Linear of a sub-layer, residual step and norm; few rows: see the offline executor
+  const bool resid = qk == 0 && M <= gsm::kMaxRows;
+#define OB_CHUNK_LINEAR_ADDNORM(label, fl, hout, in, wt, bs, lay, qi, K, alpha, mode, wa, ba, wb, bb, split)          \
+  do {                                                                                                                \
+    if (resid) {                                                                                                      \
+      OB_STEP("gemm " label, fl, gemm_residual_f32_op(w.res, w.res, in, wt, bs, M, d, K, alpha, dt, stream, kInner));   \
+      OB_ADD_NORM(hout, (mode) == 2 ? w.res : nullptr, w.res, nullptr, 0.0, mode, wa, ba, wb, bb, m.eps, split);        \
+    } else {                                                                                                          \
+      OB_CHUNK_LINEAR(label, fl, w.y, in, wt, bs, lay, qi, M, d, K, OASR_ACT_NONE, 0);                                 \
+      OB_ADD_NORM(hout, w.res, w.res, w.y, alpha, mode, wa, ba, wb, bb, m.eps, split);                                 \
+    }                                                                                                                 \
+  } while (0)
   // the embedding starts the fp32 residual stream unrounded (see the offline executor)
-  OB_STEP("gemm embed", 2.0 * M * d * m.embed_in, oasr_b200_gemm_residual_f32(w.res, nullptr, rows, m.embed_w, m.embed_b, M, d, m.embed_in, 1.0, dt, stream));
+  OB_STEP("gemm embed", 2.0 * M * d * m.embed_in, gemm_residual_f32_op(w.res, nullptr, rows, m.embed_w, m.embed_b, M, d, m.embed_in, 1.0, dt, stream, kFirst));
   if (m.embed_ln_w) {
     OB_ADD_NORM(w.h, w.res, w.res, nullptr, 0.0, 2, m.embed_ln_w, m.embed_ln_b, ly[0].norm_ff_macaron_w, ly[0].norm_ff_macaron_b, 1e-5, 0);
   } else {
@@ -439,11 +461,10 @@ int oasr_b200_conformer_chunk_paged(const oasr_b200_conformer_model* model, cons
   for (int64_t i = 0; i < L; ++i) {
     const oasr_b200_conformer_layer& l = ly[i];
     OB_CHUNK_LINEAR_H("ffn_w1", 2.0 * M * m.ffn * d, w.a_ffn, l.ffm_w1, l.ffm_b1, l, 0, m.ffn, OASR_ACT_SWISH);
-    OB_CHUNK_LINEAR("ffn_w2", 2.0 * M * m.ffn * d, w.y, w.a_ffn, l.ffm_w2, l.ffm_b2, l, 1, M, d, m.ffn, OASR_ACT_NONE, 0);
-    OB_ADD_NORM(w.h, w.res, w.res, w.y, 0.5, 0, l.norm_mha_w, l.norm_mha_b, nullptr, nullptr, m.eps, 0);
+    OB_CHUNK_LINEAR_ADDNORM("ffn_w2", 2.0 * M * m.ffn * d, w.h, w.a_ffn, l.ffm_w2, l.ffm_b2, l, 1, m.ffn, 0.5, 0, l.norm_mha_w, l.norm_mha_b, nullptr, nullptr, 0);
     // attention: project, append the chunk's keys/values to the pages, attend over cache + chunk
     if (qkv_dup) {
-      OB_STEP("gemm qkv4", 2.0 * M * 3 * d * d, oasr_b200_gemm_dup_first(w.qkv4, w.h, static_cast<const uint8_t*>(l.qkv4_w) + d * d * 2, l.qkv4_b, M, 3 * d, d, d, dt, stream));
+      OB_STEP("gemm qkv4", 2.0 * M * 3 * d * d, gemm_dup_first_op(w.qkv4, w.h, static_cast<const uint8_t*>(l.qkv4_w) + d * d * 2, l.qkv4_b, M, 3 * d, d, d, dt, stream, kInner));
     } else {
       OB_CHUNK_LINEAR_H("qkv4", 2.0 * M * 3 * d * d, w.qkv4, l.qkv4_w, l.qkv4_b, l, 2, 4 * d, OASR_ACT_NONE);
     }
@@ -466,27 +487,26 @@ int oasr_b200_conformer_chunk_paged(const oasr_b200_conformer_model* model, cons
                                        pos_start, block_table, total_seqlens, B, T, m.heads, blocks_per_seq, block_size,
                                        num_blocks, scale, dt, stream));
     }
-    OB_CHUNK_LINEAR("attn_out", 2.0 * M * d * d, w.y, w.att, l.out_w, l.out_b, l, 3, M, d, d, OASR_ACT_NONE, 0);
-    OB_ADD_NORM(w.h, w.res, w.res, w.y, 1.0, 1, l.norm_conv_scale, l.norm_conv_shift, nullptr, nullptr, m.eps, 0);
+    OB_CHUNK_LINEAR_ADDNORM("attn_out", 2.0 * M * d * d, w.h, w.att, l.out_w, l.out_b, l, 3, d, 1.0, 1, l.norm_conv_scale, l.norm_conv_shift, nullptr, nullptr, 0);
     // convolution module with the cached left context
     OB_STEP("conv_state_concat", 0, oasr_b200_conv_state_concat(w.xcat, static_cast<uint8_t*>(cnn_state) + i * num_slots * SL * d * 2,
                                      num_slots, slot_ids, w.h, B, SL, T, d, dt, stream));
     OB_CHUNK_LINEAR("pw1", 2.0 * MC * 2 * d * d, w.g, w.xcat, l.pw1_w, l.pw1_b, l, 4, MC, d, d, OASR_ACT_NONE, 1);
     OB_STEP("depthwise_conv1d", 0, oasr_b200_depthwise_conv1d_affine(w.cv, w.g, l.dw_w, l.dw_b, l.conv_bn_scale, l.conv_bn_shift,
                                      B, T + SL, d, m.kernel, 0, 0, OASR_ACT_SWISH, dt, stream));
-    OB_CHUNK_LINEAR("pw2", 2.0 * M * d * d, w.y, w.cv, l.pw2_w, l.pw2_b, l, 5, M, d, d, OASR_ACT_NONE, 0);
-    OB_ADD_NORM(w.h, w.res, w.res, w.y, 1.0, 0, l.norm_ff_w, l.norm_ff_b, nullptr, nullptr, m.eps, 0);
+    OB_CHUNK_LINEAR_ADDNORM("pw2", 2.0 * M * d * d, w.h, w.cv, l.pw2_w, l.pw2_b, l, 5, d, 1.0, 0, l.norm_ff_w, l.norm_ff_b, nullptr, nullptr, 0);
     OB_CHUNK_LINEAR_H("ffn_w1", 2.0 * M * m.ffn * d, w.a_ffn, l.ff_w1, l.ff_b1, l, 6, m.ffn, OASR_ACT_SWISH);
-    OB_CHUNK_LINEAR("ffn_w2", 2.0 * M * m.ffn * d, w.y, w.a_ffn, l.ff_w2, l.ff_b2, l, 7, M, d, m.ffn, OASR_ACT_NONE, 0);
     if (i + 1 < L) {
-      OB_ADD_NORM(w.h, w.res, w.res, w.y, 0.5, 2, l.norm_final_w, l.norm_final_b, ly[i + 1].norm_ff_macaron_w, ly[i + 1].norm_ff_macaron_b, m.eps, 0);
+      OB_CHUNK_LINEAR_ADDNORM("ffn_w2", 2.0 * M * m.ffn * d, w.h, w.a_ffn, l.ff_w2, l.ff_b2, l, 7, m.ffn, 0.5, 2, l.norm_final_w,
+                              l.norm_final_b, ly[i + 1].norm_ff_macaron_w, ly[i + 1].norm_ff_macaron_b, 0);
     } else {
-      OB_ADD_NORM(w.h3, w.res, w.res, w.y, 0.5, 2, l.norm_final_w, l.norm_final_b, m.after_norm_w, m.after_norm_b, m.eps, 1);
+      OB_CHUNK_LINEAR_ADDNORM("ffn_w2", 2.0 * M * m.ffn * d, w.h3, w.a_ffn, l.ff_w2, l.ff_b2, l, 7, m.ffn, 0.5, 2, l.norm_final_w,
+                              l.norm_final_b, m.after_norm_w, m.after_norm_b, 1);
     }
   }
   if (log_probs || argmax) {   // log_probs == NULL: token-only head, one vocabulary sweep, no log-prob write
-    OB_STEP("gemm_log_softmax", 2.0 * M * m.vocab_padded * d /* algorithmic; issued with the input split in two 16-bit terms (K = 2d) */, oasr_b200_gemm_log_softmax(log_probs, w.h3, m.ctc_w, m.ctc_b, M, m.vocab_padded, 2 * d, dt, OASR_DT_F32,
-                                       argmax, stream));
+    OB_STEP("gemm_log_softmax", 2.0 * M * m.vocab_padded * d /* algorithmic; issued with the input split in two 16-bit terms (K = 2d) */, gemm_log_softmax_op(log_probs, w.h3, m.ctc_w, m.ctc_b, M, m.vocab_padded, 2 * d, dt, OASR_DT_F32,
+                                       argmax, stream, kInner));
   }
   return OASR_OK;
 }

@@ -28,6 +28,7 @@
 
 #include "common.cuh"
 #include "device_status.cuh"
+#include "gemm_small.cuh"
 #include "sm100_ptx.cuh"
 #include "tma_host.cuh"
 
@@ -1241,10 +1242,16 @@ int gemm_simt_reference(void* D, const void* A, const void* B, const void* bias,
 
 }  // namespace ob
 
-extern "C" {
+extern "C" int oasr_b200_gemm_dup_first_supported(int64_t N, int64_t K, int64_t dup_cols);
 
-int oasr_b200_gemm(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K,
-                   int activation, int dtype, void* stream) {
+namespace ob {
+
+namespace gemm {
+// Dense 16-bit problems of few rows go to gemm_small.cu; a forced tile width names a kernel of this file.
+static bool small_rows(int64_t M, int64_t N, int64_t K) { return g_force_bn == 0 && gsm::takes(M, N, K); }
+}  // namespace gemm
+
+int gemm_op(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int activation, int dtype, void* stream, Chain chain) {
   using namespace ob;
   using namespace ob::gemm;
   if (int rc = validate_common("gemm", D, A, B, bias, M, N, K)) return rc;
@@ -1252,6 +1259,12 @@ int oasr_b200_gemm(void* D, const void* A, const void* B, const void* bias, int6
   if (M == 0) return OASR_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (use_simt(M, N, K)) return gemm_simt_reference(D, A, B, bias, M, N, K, activation, dtype, s);
+  if (small_rows(M, N, K)) {
+    gsm::Args a;
+    a.D = D; a.A = A; a.B = B; a.bias = bias; a.M = M; a.N = N; a.K = K; a.act = activation;
+    a.b_static = chain.b_static; a.late_launch = chain.late_launch;
+    return gsm::run(gsm::kStore, a, dtype, s);
+  }
   Problem pr{};
   pr.sched = kSchedDense; pr.epi = kEpiStore;
   pr.M = M; pr.N = N; pr.K = K; pr.batch = 1; pr.A = A; pr.B = B;
@@ -1260,12 +1273,7 @@ int oasr_b200_gemm(void* D, const void* A, const void* B, const void* bias, int6
   return run<kSchedDense, kEpiStore>(pr, dtype, s);
 }
 
-int oasr_b200_gemm_dup_first_supported(int64_t N, int64_t K, int64_t dup_cols) {
-  return N > 0 && K >= 16 && K % 8 == 0 && dup_cols > 0 && dup_cols <= N && N % 256 == 0 && dup_cols % 256 == 0 ? 1 : 0;
-}
-
-int oasr_b200_gemm_dup_first(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K,
-                             int64_t dup_cols, int dtype, void* stream) {
+int gemm_dup_first_op(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int64_t dup_cols, int dtype, void* stream, Chain chain) {
   using namespace ob;
   using namespace ob::gemm;
   if (int rc = validate_common("gemm_dup_first", D, A, B, bias, M, N, K)) return rc;
@@ -1274,6 +1282,12 @@ int oasr_b200_gemm_dup_first(void* D, const void* A, const void* B, const void* 
              (long long)N, (long long)dup_cols);
   if (M == 0) return OASR_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (small_rows(M, N, K)) {
+    gsm::Args a;
+    a.D = D; a.A = A; a.B = B; a.bias = bias; a.M = M; a.N = N; a.K = K; a.dup_cols = dup_cols;
+    a.b_static = chain.b_static; a.late_launch = chain.late_launch;
+    return gsm::run(gsm::kDup, a, dtype, s);
+  }
   Problem pr{};
   pr.sched = kSchedDense; pr.epi = kEpiStore;
   pr.M = M; pr.N = N; pr.K = K; pr.batch = 1; pr.A = A; pr.B = B;
@@ -1310,6 +1324,107 @@ int oasr_b200_gemm_dup_first(void* D, const void* A, const void* B, const void* 
   });
 }
 
+int gemm_residual_f32_op(float* R_out, const float* R_in, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, double alpha, int dtype, void* stream, Chain chain) {
+  using namespace ob;
+  using namespace ob::gemm;
+  if (int rc = validate_common("gemm_residual_f32", R_out, A, B, bias, M, N, K)) return rc;
+  OB_REQUIRE(M == 0 || !R_in || is_aligned(R_in, 16), OASR_ERR_ALIGN, "gemm_residual_f32: residual pointer unaligned");
+  if (M == 0) return OASR_OK;
+  if (small_rows(M, N, K)) {
+    gsm::Args a;
+    a.D = R_out; a.R_in = R_in; a.A = A; a.B = B; a.bias = bias; a.M = M; a.N = N; a.K = K; a.alpha = static_cast<float>(alpha);
+    a.b_static = chain.b_static; a.late_launch = chain.late_launch;
+    return gsm::run(gsm::kResid, a, dtype, static_cast<cudaStream_t>(stream));
+  }
+  Problem pr{};
+  pr.sched = kSchedDense; pr.epi = kEpiResid;
+  pr.M = M; pr.N = N; pr.K = K; pr.batch = 1; pr.A = A; pr.B = B;
+  pr.p.M = (int)M; pr.p.N = (int)N; pr.p.K = (int)K; pr.p.batch = 1;
+  pr.p.D = R_out; pr.p.R_in = R_in; pr.p.bias = bias; pr.p.act = OASR_ACT_NONE; pr.p.alpha = (float)alpha;
+  return run<kSchedDense, kEpiResid>(pr, dtype, static_cast<cudaStream_t>(stream));
+}
+
+int gemm_glu_op(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int dtype, void* stream, Chain chain) {
+  using namespace ob;
+  using namespace ob::gemm;
+  if (int rc = validate_common("gemm_glu", D, A, B, bias, M, N, K)) return rc;
+  if (M == 0) return OASR_OK;
+  if (g_force_bn == 0 && gsm::takes_glu(M, N, K)) {
+    gsm::Args a;
+    a.D = D; a.A = A; a.B = B; a.bias = bias; a.M = M; a.N = N; a.K = K;
+    a.b_static = chain.b_static; a.late_launch = chain.late_launch;
+    return gsm::run(gsm::kGlu, a, dtype, static_cast<cudaStream_t>(stream));
+  }
+  Problem pr{};
+  pr.sched = kSchedDense; pr.epi = kEpiGlu;
+  pr.M = M; pr.N = N; pr.K = K; pr.batch = 1; pr.A = A; pr.B = B;
+  pr.p.M = (int)M; pr.p.N = (int)N; pr.p.K = (int)K; pr.p.batch = 1;
+  pr.p.D = D; pr.p.bias = bias; pr.p.act = OASR_ACT_NONE; pr.p.alpha = 1.f;
+  return run<kSchedDense, kEpiGlu>(pr, dtype, static_cast<cudaStream_t>(stream));
+}
+
+int gemm_log_softmax_op(void* out, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int dtype, int out_dtype, int32_t* argmax, void* stream, Chain chain) {
+  using namespace ob;
+  using namespace ob::gemm;
+  // out == NULL with argmax != NULL: only the per-row index of the first maximum is wanted (greedy CTC search);
+  // one sweep over the vocabulary, nothing but 4 bytes per row is written
+  const bool tokens_only = out == nullptr && argmax != nullptr;
+  if (int rc = validate_common("gemm_log_softmax", tokens_only ? static_cast<const void*>(A) : out, A, B, bias, M, N, K)) return rc;
+  OB_REQUIRE(out_dtype == OASR_DT_F32 || out_dtype == dtype, OASR_ERR_DTYPE,
+             "gemm_log_softmax: out dtype must be fp32 or the activation dtype");
+  if (M == 0) return OASR_OK;
+  // Two forms.  The fused kernel sweeps the vocabulary twice per 128-row tile (statistics, then the same products
+  // written normalised) and never writes logits; it keeps one CTA per row tile, so it needs about as many row tiles
+  // as SMs.  The split form writes fp32 logits into `out` with the dense scheduler (every SM busy at any M) and
+  // normalises the rows in place: one GEMM instead of two for a second pass over the output.
+  const bool split_ok = out_dtype == OASR_DT_F32 && !use_simt(M, N, K) && !tokens_only;
+  const bool split = split_ok && (g_lsm_path == 2 || (g_lsm_path == 0 && lsm_split_wins(M, N, K)));
+  if (split) {
+    if (small_rows(M, N, K)) {
+      gsm::Args a;
+      a.D = out; a.A = A; a.B = B; a.bias = bias; a.M = M; a.N = N; a.K = K;
+      a.b_static = chain.b_static; a.late_launch = chain.late_launch;
+      if (int rc = gsm::run(gsm::kResid, a, dtype, static_cast<cudaStream_t>(stream))) return rc;
+    } else {
+    Problem pg{};
+    pg.sched = kSchedDense; pg.epi = kEpiResid;
+    pg.M = M; pg.N = N; pg.K = K; pg.batch = 1; pg.A = A; pg.B = B;
+    pg.p.M = (int)M; pg.p.N = (int)N; pg.p.K = (int)K; pg.p.batch = 1;
+    pg.p.D = out; pg.p.R_in = nullptr; pg.p.bias = bias; pg.p.act = OASR_ACT_NONE; pg.p.alpha = 1.f;
+    if (int rc = run<kSchedDense, kEpiResid>(pg, dtype, static_cast<cudaStream_t>(stream))) return rc;
+    }
+    int64_t g = M < static_cast<int64_t>(sm_count()) * 8 ? M : static_cast<int64_t>(sm_count()) * 8;
+    log_softmax_rows_f32_kernel<<<static_cast<unsigned>(g), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<float*>(out), argmax, (int)M, (int)N);
+    return check_launch("log_softmax_rows launch");
+  }
+  Problem pr{};
+  pr.sched = kSchedSweep; pr.epi = kEpiLsm;
+  pr.M = M; pr.N = N; pr.K = K; pr.batch = 1; pr.A = A; pr.B = B;
+  pr.p.M = (int)M; pr.p.N = (int)N; pr.p.K = (int)K; pr.p.batch = 1;
+  pr.p.D = out; pr.p.bias = bias; pr.p.act = OASR_ACT_NONE; pr.p.alpha = 1.f;
+  pr.p.out_f32 = out_dtype == OASR_DT_F32 ? 1 : 0;
+  pr.p.lsm_passes = tokens_only ? 1 : 2;
+  pr.p.argmax = argmax;
+  return run<kSchedSweep, kEpiLsm>(pr, dtype, static_cast<cudaStream_t>(stream));
+}
+
+}  // namespace ob
+
+extern "C" {
+
+int oasr_b200_gemm(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int activation, int dtype, void* stream) {
+  return ob::gemm_op(D, A, B, bias, M, N, K, activation, dtype, stream, ob::Chain{});
+}
+
+int oasr_b200_gemm_dup_first_supported(int64_t N, int64_t K, int64_t dup_cols) {
+  return N > 0 && K >= 16 && K % 8 == 0 && dup_cols > 0 && dup_cols <= N && N % 256 == 0 && dup_cols % 256 == 0 ? 1 : 0;
+}
+
+int oasr_b200_gemm_dup_first(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int64_t dup_cols, int dtype, void* stream) {
+  return ob::gemm_dup_first_op(D, A, B, bias, M, N, K, dup_cols, dtype, stream, ob::Chain{});
+}
+
 int oasr_b200_gemm_q8(void* D, const void* A_q, const float* a_scale, const void* B_q, const float* b_scale,
                       const void* bias, int64_t M, int64_t N, int64_t K, int activation, int glu, int kind,
                       int out_dtype, void* stream) {
@@ -1342,33 +1457,12 @@ int oasr_b200_gemm_q8(void* D, const void* A_q, const float* a_scale, const void
   });
 }
 
-int oasr_b200_gemm_residual_f32(float* R_out, const float* R_in, const void* A, const void* B, const void* bias,
-                                int64_t M, int64_t N, int64_t K, double alpha, int dtype, void* stream) {
-  using namespace ob;
-  using namespace ob::gemm;
-  if (int rc = validate_common("gemm_residual_f32", R_out, A, B, bias, M, N, K)) return rc;
-  OB_REQUIRE(M == 0 || !R_in || is_aligned(R_in, 16), OASR_ERR_ALIGN, "gemm_residual_f32: residual pointer unaligned");
-  if (M == 0) return OASR_OK;
-  Problem pr{};
-  pr.sched = kSchedDense; pr.epi = kEpiResid;
-  pr.M = M; pr.N = N; pr.K = K; pr.batch = 1; pr.A = A; pr.B = B;
-  pr.p.M = (int)M; pr.p.N = (int)N; pr.p.K = (int)K; pr.p.batch = 1;
-  pr.p.D = R_out; pr.p.R_in = R_in; pr.p.bias = bias; pr.p.act = OASR_ACT_NONE; pr.p.alpha = (float)alpha;
-  return run<kSchedDense, kEpiResid>(pr, dtype, static_cast<cudaStream_t>(stream));
+int oasr_b200_gemm_residual_f32(float* R_out, const float* R_in, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, double alpha, int dtype, void* stream) {
+  return ob::gemm_residual_f32_op(R_out, R_in, A, B, bias, M, N, K, alpha, dtype, stream, ob::Chain{});
 }
 
-int oasr_b200_gemm_glu(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K,
-                       int dtype, void* stream) {
-  using namespace ob;
-  using namespace ob::gemm;
-  if (int rc = validate_common("gemm_glu", D, A, B, bias, M, N, K)) return rc;
-  if (M == 0) return OASR_OK;
-  Problem pr{};
-  pr.sched = kSchedDense; pr.epi = kEpiGlu;
-  pr.M = M; pr.N = N; pr.K = K; pr.batch = 1; pr.A = A; pr.B = B;
-  pr.p.M = (int)M; pr.p.N = (int)N; pr.p.K = (int)K; pr.p.batch = 1;
-  pr.p.D = D; pr.p.bias = bias; pr.p.act = OASR_ACT_NONE; pr.p.alpha = 1.f;
-  return run<kSchedDense, kEpiGlu>(pr, dtype, static_cast<cudaStream_t>(stream));
+int oasr_b200_gemm_glu(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int dtype, void* stream) {
+  return ob::gemm_glu_op(D, A, B, bias, M, N, K, dtype, stream, ob::Chain{});
 }
 
 int oasr_b200_bmm(void* D, const void* A, const void* B, int64_t batch, int64_t M, int64_t N, int64_t K, int dtype,
@@ -1484,44 +1578,8 @@ int oasr_b200_subsample_conv2(void* out, const void* x1, const void* w2, const v
   });
 }
 
-int oasr_b200_gemm_log_softmax(void* out, const void* A, const void* B, const void* bias, int64_t M, int64_t N,
-                               int64_t K, int dtype, int out_dtype, int32_t* argmax, void* stream) {
-  using namespace ob;
-  using namespace ob::gemm;
-  // out == NULL with argmax != NULL: only the per-row index of the first maximum is wanted (greedy CTC search);
-  // one sweep over the vocabulary, nothing but 4 bytes per row is written
-  const bool tokens_only = out == nullptr && argmax != nullptr;
-  if (int rc = validate_common("gemm_log_softmax", tokens_only ? static_cast<const void*>(A) : out, A, B, bias, M, N, K)) return rc;
-  OB_REQUIRE(out_dtype == OASR_DT_F32 || out_dtype == dtype, OASR_ERR_DTYPE,
-             "gemm_log_softmax: out dtype must be fp32 or the activation dtype");
-  if (M == 0) return OASR_OK;
-  // Two forms.  The fused kernel sweeps the vocabulary twice per 128-row tile (statistics, then the same products
-  // written normalised) and never writes logits; it keeps one CTA per row tile, so it needs about as many row tiles
-  // as SMs.  The split form writes fp32 logits into `out` with the dense scheduler (every SM busy at any M) and
-  // normalises the rows in place: one GEMM instead of two for a second pass over the output.
-  const bool split_ok = out_dtype == OASR_DT_F32 && !use_simt(M, N, K) && !tokens_only;
-  const bool split = split_ok && (g_lsm_path == 2 || (g_lsm_path == 0 && lsm_split_wins(M, N, K)));
-  if (split) {
-    Problem pg{};
-    pg.sched = kSchedDense; pg.epi = kEpiResid;
-    pg.M = M; pg.N = N; pg.K = K; pg.batch = 1; pg.A = A; pg.B = B;
-    pg.p.M = (int)M; pg.p.N = (int)N; pg.p.K = (int)K; pg.p.batch = 1;
-    pg.p.D = out; pg.p.R_in = nullptr; pg.p.bias = bias; pg.p.act = OASR_ACT_NONE; pg.p.alpha = 1.f;
-    if (int rc = run<kSchedDense, kEpiResid>(pg, dtype, static_cast<cudaStream_t>(stream))) return rc;
-    int64_t g = M < static_cast<int64_t>(sm_count()) * 8 ? M : static_cast<int64_t>(sm_count()) * 8;
-    log_softmax_rows_f32_kernel<<<static_cast<unsigned>(g), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<float*>(out), argmax, (int)M, (int)N);
-    return check_launch("log_softmax_rows launch");
-  }
-  Problem pr{};
-  pr.sched = kSchedSweep; pr.epi = kEpiLsm;
-  pr.M = M; pr.N = N; pr.K = K; pr.batch = 1; pr.A = A; pr.B = B;
-  pr.p.M = (int)M; pr.p.N = (int)N; pr.p.K = (int)K; pr.p.batch = 1;
-  pr.p.D = out; pr.p.bias = bias; pr.p.act = OASR_ACT_NONE; pr.p.alpha = 1.f;
-  pr.p.out_f32 = out_dtype == OASR_DT_F32 ? 1 : 0;
-  pr.p.lsm_passes = tokens_only ? 1 : 2;
-  pr.p.argmax = argmax;
-  return run<kSchedSweep, kEpiLsm>(pr, dtype, static_cast<cudaStream_t>(stream));
+int oasr_b200_gemm_log_softmax(void* out, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int dtype, int out_dtype, int32_t* argmax, void* stream) {
+  return ob::gemm_log_softmax_op(out, A, B, bias, M, N, K, dtype, out_dtype, argmax, stream, ob::Chain{});
 }
 
 }  // extern "C"
