@@ -13,6 +13,7 @@ from dataclasses import dataclass
 from functools import lru_cache
 from typing import Optional, Tuple
 
+import numpy as np
 import torch
 
 from . import _lib
@@ -100,12 +101,15 @@ def batched_fbank(waveforms: torch.Tensor, lengths: torch.Tensor, cfg: FbankConf
     dev = waveforms.device
     L, hop = cfg.frame_length_samples, cfg.frame_shift_samples
     num_frames = max(0, (T - L) // hop + 1)
-    feat_len = feature_lengths(lengths.cpu() if isinstance(lengths, torch.Tensor) else lengths, cfg).to(dev, non_blocking=True)
+    # sample counts and frame counts in one small host array, one copy to the device
+    counts = np.empty((2, B), dtype=np.int32)
+    counts[0] = lengths.cpu().numpy() if isinstance(lengths, torch.Tensor) else np.asarray(lengths)
+    counts[1] = np.maximum((counts[0].astype(np.int64) - L) // hop + 1, 0)
+    len_dev, feat_len = torch.from_numpy(counts).to(dev, non_blocking=True)
     out = torch.empty(B, num_frames, cfg.num_mel_bins, device=dev, dtype=torch.float32)
     if B == 0 or num_frames == 0:
         return out, feat_len
     window, mel, lo, hi = _tables(cfg, dev)
-    len_dev = torch.as_tensor(lengths).to(torch.int32).to(dev, non_blocking=True)
     mean = istd = None
     if cmvn is not None:
         mean, istd = (t.to(dev, torch.float32).contiguous() for t in cmvn)

@@ -97,3 +97,25 @@ def test_audio_to_tokens_through_fbank_and_encoder():
     assert torch.equal(ol_a, ol_b)
     valid = (torch.arange(lp_a.shape[1])[None, :] < ol_a.cpu()[:, None])
     assert (lp_a.cpu() - lp_b.cpu())[valid].abs().max().item() < 2e-2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("length_ms,shift_ms", [(25.0, 10.0), (32.0, 16.0), (20.0, 7.0), (17.0, 10.0)])
+def test_512_point_kernel_at_other_framings_and_odd_frame_counts(length_ms, shift_ms):
+    """Frame pairs of the n_fft = 512 kernel: a last frame without a partner, an utterance that ends inside a pair, frame
+    lengths that fill the transform, shifts that are no multiple of a warp, more samples than a lane holds ahead."""
+    import oasr_b200 as ob
+    from oasr_b200 import features as F
+
+    cfg = F.FbankConfig(frame_length_ms=length_ms, frame_shift_ms=shift_ms)
+    L, hop = cfg.frame_length_samples, cfg.frame_shift_samples
+    assert cfg.n_fft == 512
+    lengths = torch.tensor([L + 4 * hop, L, L + hop + 1, L + 3 * hop - 1, L - 1])
+    wave = torch.randn(5, L + 4 * hop, generator=torch.Generator().manual_seed(8)) * 0.2
+    got, glen = F.batched_fbank(wave.cuda(), lengths, cfg)
+    want, wlen = OFE.fbank(wave, lengths, OFE.FbankConfig(frame_length_ms=length_ms, frame_shift_ms=shift_ms))
+    assert ob.device_status() == 0 and glen.cpu().tolist() == wlen.tolist() == [5, 1, 2, 3, 0]
+    for b, n in enumerate(wlen.tolist()):
+        if n:
+            assert (got[b, :n].cpu() - want[b, :n]).abs().max().item() < 3e-3     # fp32 FFT and summation order, as above
+        assert torch.count_nonzero(got[b, n:]) == 0
