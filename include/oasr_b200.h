@@ -652,6 +652,38 @@ OASR_API int oasr_b200_paged_kv_gather(void* k_out, void* v_out, const void* k_p
                                        int64_t block_size, int64_t num_blocks, int elem_bytes,
                                        void* stream);
 
+/* ---- windowed relative-position attention (FastConformer) ------------------ */
+/* 1 when a chunked-limited window of `left_chunks` whole chunks of `chunk` frames
+ * before a frame's own chunk fits the kernels below (head_dim 64 or 128, at most
+ * 64 different distances), else 0. */
+OASR_API int oasr_b200_fmha_window_supported(int64_t head_dim, int64_t chunk, int64_t left_chunks);
+/* Self-attention of packed segments inside that window with the Transformer-XL
+ * position term: scores ((q+u).k_j + (q+v).r_{i-j}) * scale over the keys j of the
+ * chunks [chunk(i) - left_chunks, chunk(i)] of the segment
+ * (oasr/models/nemotron/encoder.py:82-149, 300-359), linear in the frames: no
+ * (T, T) scores or bias exist.  qkv4 (total, 4*heads*head_dim) = [q+u|q+v|k|v];
+ * rel_k (table_rows, heads*head_dim): row center - d is relative_k_proj of
+ * distance d (rows outside the table are never needed by a visible key);
+ * out (total, heads*head_dim). */
+OASR_API int oasr_b200_fmha_window_packed(void* out, const void* qkv4, const void* rel_k, int64_t table_rows,
+                                          int64_t center, const int32_t* cu_seqlens, int64_t num_segs,
+                                          int64_t max_seg, int64_t total, int64_t heads, int64_t head_dim,
+                                          int64_t chunk, int64_t left_chunks, double scale, int dtype,
+                                          void* stream);
+/* The same for the Tq new frames of B streams over their paged keys / values
+ * (NemotronEncoderLayer.forward_chunk, oasr/models/nemotron/encoder.py:269-326):
+ * qkv4 (B*Tq, 4*heads*head_dim); cached (B) frames already in the pages,
+ * pos_start (B) absolute frame of each stream's key 0.  The chunk's own keys and
+ * values are taken from qkv4 and WRITTEN to the pages at positions cached + t (the
+ * rule of oasr_b200_paged_kv_write), so no page write is needed before. */
+OASR_API int oasr_b200_fmha_window_paged(void* out, const void* qkv4, void* k_pool, void* v_pool,
+                                         const void* rel_k, int64_t table_rows, int64_t center,
+                                         const int32_t* block_table, const int32_t* cached,
+                                         const int32_t* pos_start, int64_t B, int64_t Tq, int64_t heads,
+                                         int64_t head_dim, int64_t blocks_per_seq, int64_t block_size,
+                                         int64_t num_blocks, int64_t chunk, int64_t left_chunks, double scale,
+                                         int dtype, void* stream);
+
 /* ---- packed-layout glue ------------------------------------------------ */
 /* out[i, :] = in[index[i], :] for i < n_out (rows of `row_bytes` bytes,
  * multiple of 16; index int64; `in` has `in_rows` rows and an index outside
@@ -873,6 +905,9 @@ typedef struct oasr_b200_fastconformer_model {
   double mask_floor;       /* finite additive floor of a masked key (-1e4, encoder.py:80) */
   const oasr_b200_fastconformer_layer* layers;   /* HOST array of num_layers entries */
   int32_t quant_kind;      /* 0 = 16-bit Linear GEMMs; OASR_Q8_FP8_E4M3 / OASR_Q8_INT8 = per-token quantised inputs x q_w */
+  const void* rel_window;                    /* nullable: (num_layers, 64, hidden), row y of a layer = relative_k_proj of distance
+                                                off - y, off = left_chunks * chunk + chunk - 1: what windowed attention needs of
+                                                the projected table, the same for every batch */
 } oasr_b200_fastconformer_model;
 
 /* Bytes of device scratch oasr_b200_fastconformer_layers_packed needs for `total` packed frames, a relative-position
@@ -895,6 +930,27 @@ OASR_API int oasr_b200_fastconformer_layers_packed(const oasr_b200_fastconformer
                                                    int64_t bias_numel, int64_t num_segs, int64_t total,
                                                    int64_t max_seg, void* workspace, int64_t workspace_bytes,
                                                    void* stream);
+
+/* Bytes of device scratch oasr_b200_fastconformer_chunk_paged needs. */
+OASR_API int64_t oasr_b200_fastconformer_chunk_workspace_bytes(const oasr_b200_fastconformer_model* model, int64_t B,
+                                                               int64_t Tq);
+/* The layer stack for one chunk of B streams in one host call
+ * (NemotronEncoder.forward_chunk_paged, oasr/models/nemotron/encoder.py:269-326,
+ * 585-650): rows (B*Tq, hidden) post-subsampling states (16-bit, or fp32 with
+ * rows_f32), out (B*Tq, hidden) fp32.  Pools and block_table as in
+ * oasr_b200_fmha_window_paged, one pool pair per layer (HOST arrays of pointers);
+ * cnn_state (num_layers, num_slots, kernel-1, hidden) the post-GLU conv tails,
+ * updated in place for the rows' slot_ids.  Needs rel_window, a supported window
+ * and 16-bit Linears (quant_kind 0). */
+OASR_API int oasr_b200_fastconformer_chunk_paged(const oasr_b200_fastconformer_model* model, const void* rows,
+                                                 int rows_f32, float* out, int64_t B, int64_t Tq,
+                                                 void* const* k_pools, void* const* v_pools,
+                                                 const int32_t* block_table, const int32_t* cached,
+                                                 const int32_t* pos_start, int64_t blocks_per_seq,
+                                                 int64_t block_size, int64_t num_blocks, void* cnn_state,
+                                                 int64_t num_slots, const int64_t* slot_ids, void* workspace,
+                                                 int64_t workspace_bytes, void* stream);
+
 
 #ifdef __cplusplus
 }

@@ -86,6 +86,9 @@ _SIGNATURES = {
     "oasr_b200_depthwise_conv1d_packed_causal": [P, P, P, P, P, I, I, I, I, c_int, c_int, P],
     "oasr_b200_relshift_bias_packed": [P, P, P, P, I, I, I, I, I, c_double, I, I, c_double, c_int, P],
     "oasr_b200_fmha_varlen_strided": [P, P, P, P, I, I, I, P, P, c_int, c_int, P, P, I, I, I, I, I, I, I, c_double, c_int, P],
+    "oasr_b200_fmha_window_supported": [I, I, I],
+    "oasr_b200_fmha_window_packed": [P, P, P, I, I, P, I, I, I, I, I, I, I, c_double, c_int, P],
+    "oasr_b200_fmha_window_paged": [P, P, P, P, P, I, I, P, P, P, I, I, I, I, I, I, I, I, I, c_double, c_int, P],
     "oasr_b200_bmm_strided": [P, P, P, I, I, I, I, I, I, I, I, c_int, P],
     "oasr_b200_fmha_bthd": [P, P, P, P, P, P, P, P, I, I, I, P, P, P, I, I, I, I, I, I, I, I, I, c_double, c_int, c_int, P],
     "oasr_b200_fmha_varlen": [P, P, P, P, P, P, c_int, P, P, I, I, I, I, I, I, I, c_double, c_int, P],
@@ -134,10 +137,13 @@ class FastConformerModel(ctypes.Structure):
 
     _fields_ = [(n, ctypes.c_int32) for n in (
         "hidden", "heads", "ffn", "kernel", "num_layers", "dtype", "left_context", "right_context")] + [
-        ("eps", c_double), ("mask_floor", c_double), ("layers", POINTER(FastConformerLayer)), ("quant_kind", ctypes.c_int32)]
+        ("eps", c_double), ("mask_floor", c_double), ("layers", POINTER(FastConformerLayer)), ("quant_kind", ctypes.c_int32),
+        ("rel_window", c_void_p)]
 
 
 _SIGNATURES["oasr_b200_fastconformer_layers_packed"] = [POINTER(FastConformerModel), P, c_int, P, P, I, P, P, I, I, I, I, P, I, P]
+_SIGNATURES["oasr_b200_fastconformer_chunk_paged"] = [POINTER(FastConformerModel), P, c_int, P, I, I, POINTER(c_void_p), POINTER(c_void_p),
+                                                     P, P, P, I, I, I, P, I, P, P, I, P]
 _SIGNATURES["oasr_b200_conformer_encode_packed"] = [POINTER(ConformerModel), P, P, P, I, I, I, P, I, P, P, P]
 
 _SIGNATURES["oasr_b200_conformer_encode_packed_noalloc"] = [POINTER(ConformerModel), P, P, P, I, I, I, P, P, P]
@@ -183,6 +189,8 @@ def load() -> ctypes.CDLL:
     lib.oasr_b200_fmha_relpos_plan_bytes.argtypes = [I, I, I]
     lib.oasr_b200_fastconformer_workspace_bytes.restype = c_int64
     lib.oasr_b200_fastconformer_workspace_bytes.argtypes = [POINTER(FastConformerModel), I, I, I]
+    lib.oasr_b200_fastconformer_chunk_workspace_bytes.restype = c_int64
+    lib.oasr_b200_fastconformer_chunk_workspace_bytes.argtypes = [POINTER(FastConformerModel), I, I]
     for name, argtypes in _SIGNATURES.items():
         try:
             fn = getattr(lib, name)
@@ -196,7 +204,8 @@ def load() -> ctypes.CDLL:
 def exported_names() -> list[str]:
     return list(_STRING_FUNCS) + ["oasr_b200_launch_count", "oasr_b200_conformer_workspace_bytes", "oasr_b200_profile_count",
                                   "oasr_b200_conformer_noalloc_capacity_bytes", "oasr_b200_conformer_chunk_workspace_bytes",
-                                  "oasr_b200_fastconformer_workspace_bytes", "oasr_b200_fmha_relpos_plan_bytes"] + list(_SIGNATURES)
+                                  "oasr_b200_fastconformer_workspace_bytes", "oasr_b200_fastconformer_chunk_workspace_bytes",
+                                  "oasr_b200_fmha_relpos_plan_bytes"] + list(_SIGNATURES)
 
 
 def launch_count() -> int:

@@ -368,9 +368,7 @@ class ConformerCTC:
             self._workspace = torch.empty(int(need * 1.25) + 256, dtype=torch.uint8, device=xs.device)
         ws = self._workspace
         off = (-ws.data_ptr()) % 256
-        L = self.cfg.layers
-        kp = (ctypes.c_void_p * L)(*[cache.k_pool[i].data_ptr() for i in range(L)])
-        vp = (ctypes.c_void_p * L)(*[cache.v_pool[i].data_ptr() for i in range(L)])
+        kp, vp = cache.pool_pointers()
         log_probs = torch.empty(B, T, self.cfg.vocab_padded, device=xs.device, dtype=torch.float32)
         argmax = torch.empty(B, T, device=xs.device, dtype=torch.int32)
         _lib.call("oasr_b200_conformer_chunk_paged", ctypes.byref(self._native_model), _p(rows), B, T, kp, vp, _p(table),

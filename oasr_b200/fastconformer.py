@@ -76,6 +76,7 @@ class FastConformerLayers:
                 lw[n] = (w(params[p + n + ".weight"]), w(params[p + n + ".bias"]))
             self.layers.append(lw)
         self._workspace = None
+        self._rel_window = None           # (L, 64, C): see _window_table
         self.native = True                # packed batches run through the one-call native executor
         self._build_native_model()
 
@@ -125,6 +126,7 @@ class FastConformerLayers:
         m.eps, m.mask_floor = self.eps, MASK_FLOOR
         m.layers = ctypes.cast(arr, ctypes.POINTER(_lib.FastConformerLayer))
         m.quant_kind = self.qkind
+        m.rel_window = ptr(self._rel_window)
         self._native_layers, self._native_model = arr, m      # keep both alive
 
     def _layers_native(self, rows: torch.Tensor, g) -> torch.Tensor:
@@ -137,9 +139,14 @@ class FastConformerLayers:
 
         M, C = rows.shape
         res = rows
-        table = self._position_table(g["T"])
+        if self._windowed(g["T"]):         # no position table: the model's own windowed rows serve every batch
+            self._window_table()
+            table, table_rows = None, (2 * g["T"] - 1 + 7) // 8 * 8
+        else:
+            table = self._position_table(g["T"])
+            table_rows = table.size(0)
         lib = _lib.load()
-        need = lib.oasr_b200_fastconformer_workspace_bytes(ctypes.byref(self._native_model), M, table.size(0), g["bias_numel"])
+        need = lib.oasr_b200_fastconformer_workspace_bytes(ctypes.byref(self._native_model), M, table_rows, g["bias_numel"])
         if self._workspace is None or self._workspace.numel() < need + 256:
             self._workspace = torch.empty(int(need * 1.25) + 256, dtype=torch.uint8, device=res.device)
         ws = self._workspace
@@ -147,7 +154,7 @@ class FastConformerLayers:
         out = torch.empty(M, C, device=res.device, dtype=torch.float32)
         _lib.call("oasr_b200_fastconformer_layers_packed", ctypes.byref(self._native_model), _p(rows),
                   1 if rows.dtype == torch.float32 else 0, _p(out), _p(table),
-                  table.size(0), _p(g["cu"]), _p(g["offsets"]), g["bias_numel"], g["cu"].numel() - 1, M, g["T"],
+                  table_rows, _p(g["cu"]), _p(g["offsets"]), g["bias_numel"], g["cu"].numel() - 1, M, g["T"],
                   ctypes.c_void_p(ws.data_ptr() + off), ws.numel() - off, _stream(res))
         return out
 
@@ -177,10 +184,7 @@ class FastConformerLayers:
         hit = self._tables.get(T)
         if hit is not None:
             return hit
-        inv_freq = 1.0 / (10000.0 ** (torch.arange(0, self.C, 2, dtype=torch.float32) / self.C))
-        positions = torch.arange(T - 1, -T, -1, dtype=torch.float32)
-        freqs = torch.outer(positions, inv_freq)
-        table = torch.stack([freqs.sin(), freqs.cos()], dim=-1).reshape(freqs.size(0), self.C)
+        table = self._sinusoid(torch.arange(T - 1, -T, -1, dtype=torch.float32))
         P = table.size(0)
         table = torch.nn.functional.pad(table, (0, 0, 0, (P + 7) // 8 * 8 - P))
         out = table.to(self.dtype).to(self.device)             # (roundup8(2T-1), C)
@@ -189,10 +193,46 @@ class FastConformerLayers:
         self._tables[T] = out
         return out
 
+    # ---- windowed attention: long packed segments and streams (csrc/fmha_window.cu) ----
+    WINDOW_FRAMES = 128     # segments up to this length attend through the general kernels (as csrc/fastconformer.cu)
+
+    def _window_geometry(self):
+        chunk = self.right + 1
+        return chunk, self.left // chunk
+
+    def _window_fits(self) -> bool:
+        return self.left >= 0 and fused.fmha_window_supported(self.D, *self._window_geometry())
+
+    def _windowed(self, T: int) -> bool:
+        return T > self.WINDOW_FRAMES and self._window_fits()
+
+    def _window_table(self) -> torch.Tensor:
+        """``relative_k_proj`` of the 64 distances a window can hold, every layer: row ``y`` = distance ``off - y`` with
+        ``off = left_chunks * chunk + chunk - 1``.  Depends on the model only; built once."""
+        if self._rel_window is None:
+            chunk, left_chunks = self._window_geometry()
+            off = left_chunks * chunk + chunk - 1
+            table = self._sinusoid(off - torch.arange(64, dtype=torch.float32)).to(self.dtype).to(self.device)
+            self._rel_window = torch.stack([OF.gemm(table, lw["rel"]) for lw in self.layers]).contiguous()
+            self._native_model.rel_window = self._rel_window.data_ptr()
+        return self._rel_window
+
+    def _sinusoid(self, positions: torch.Tensor) -> torch.Tensor:
+        inv_freq = 1.0 / (10000.0 ** (torch.arange(0, self.C, 2, dtype=torch.float32) / self.C))
+        freqs = torch.outer(positions, inv_freq)
+        return torch.stack([freqs.sin(), freqs.cos()], dim=-1).reshape(freqs.size(0), self.C)
+
     # ---- one layer; ``g`` is the geometry of the rows: padded (B, T, lens) or packed (cu, offsets) ----
-    def _attention(self, lw, h: torch.Tensor, rel_table: torch.Tensor, g) -> torch.Tensor:
+    def _attention(self, i: int, h: torch.Tensor, g) -> torch.Tensor:
         C, H, D = self.C, self.H, self.D
         M = h.size(0)
+        lw = self.layers[i]
+        if g["packed"] and self._windowed(g["T"]):
+            chunk, left_chunks = self._window_geometry()
+            out = fused.fmha_window_packed(self._linear(h, *lw["qkv4"]), self._window_table()[i], left_chunks * chunk + chunk - 1, g["cu"],
+                                           g["T"], H, chunk, left_chunks, D ** -0.5)
+            return self._linear(out, *lw["o"])
+        rel_table = self._position_table(g["T"])
         qkv4 = self._linear(h, *lw["qkv4"]).view(M, 4, H, D)                          # q+u | q+v | k | v of every row
         # projected positions; the table carries zero rows up to a multiple of 8 (the GEMM's column granule)
         Pp = rel_table.size(0)
@@ -237,7 +277,6 @@ class FastConformerLayers:
         """The stack operator by operator from Python: padded batches, and the check of the native executor (same
         kernels, same order, so bit-identical results, with 16-bit and with 8-bit Linear GEMMs)."""
         M, C = res.shape
-        rel_table = self._position_table(g["T"])
         h = torch.empty(M, C, device=res.device, dtype=self.dtype)
         first = self.layers[0]["norm_feed_forward1"]
         fused.add_norm_f32(h, None, res, None, 0.0, fused.ADD_NORM_LN, *first, eps=self.eps)          # LN(x)
@@ -246,7 +285,7 @@ class FastConformerLayers:
             w1, b1, w2, b2 = lw["feed_forward1"]
             y = self._linear(self._linear(h, w1, b1, _SWISH), w2, b2)
             fused.add_norm_f32(h, res, res, y, 0.5, fused.ADD_NORM_LN, *lw["norm_self_att"], eps=self.eps)
-            y = self._attention(lw, h, rel_table, g)
+            y = self._attention(i, h, g)
             fused.add_norm_f32(h, res, res, y, 1.0, fused.ADD_NORM_LN, *lw["norm_conv"], eps=self.eps)
             y = self._conv(lw, h, g)
             fused.add_norm_f32(h, res, res, y, 1.0, fused.ADD_NORM_LN, *lw["norm_feed_forward2"], eps=self.eps)
@@ -303,8 +342,12 @@ class FastConformerLayers:
         slots = list(slots)
         if Tq != cache.chunk or len(slots) != B:
             raise RuntimeError(f"expected {len(slots)} streams x {cache.chunk} frames, got {B} x {Tq}")
-        H, D, SL = self.H, self.D, self.K - 1
         table, cached, total, pos_start, slot_ids = cache.prepare(slots)
+        if self.native and not self.qkind and self._window_fits() and hidden.dtype in (torch.float32, self.dtype):
+            out = self._chunk_native(hidden.reshape(B * Tq, C).contiguous(), B, Tq, cache, table, cached, pos_start, slot_ids)
+            cache.commit(slots)
+            return out.view(B, Tq, C)
+        H, D, SL = self.H, self.D, self.K - 1
         offsets = pos_start + cached                                   # encoder frames emitted before this chunk
         lmax = cache.max_past + Tq
         tk = table.size(1) * cache.block_size
@@ -352,6 +395,29 @@ class FastConformerLayers:
                 fused.add_norm_f32(h, out, res, y, 0.5, fused.ADD_NORM_LN_LN, *lw["norm_out"], *lw["norm_out"], eps=self.eps)
         cache.commit(slots)
         return out.view(B, Tq, C)
+
+    def _chunk_native(self, rows: torch.Tensor, B: int, Tq: int, cache, table, cached, pos_start, slot_ids) -> torch.Tensor:
+        """The streaming step in ONE call into the native executor (oasr_b200_fastconformer_chunk_paged): 18 launches per
+        layer where the composition below makes 24 from Python."""
+        import ctypes
+
+        from . import _lib
+        from .functional import _p, _stream
+
+        self._window_table()
+        lib = _lib.load()
+        need = lib.oasr_b200_fastconformer_chunk_workspace_bytes(ctypes.byref(self._native_model), B, Tq)
+        if self._workspace is None or self._workspace.numel() < need + 256:
+            self._workspace = torch.empty(int(need * 1.25) + 256, dtype=torch.uint8, device=rows.device)
+        ws = self._workspace
+        off = (-ws.data_ptr()) % 256
+        out = torch.empty(B * Tq, self.C, device=rows.device, dtype=torch.float32)
+        kp, vp = cache.pool_pointers()
+        _lib.call("oasr_b200_fastconformer_chunk_paged", ctypes.byref(self._native_model), _p(rows),
+                  1 if rows.dtype == torch.float32 else 0, _p(out), B, Tq, kp, vp, _p(table), _p(cached), _p(pos_start), table.size(1),
+                  cache.block_size, cache.num_blocks, _p(cache.cnn_state), cache.max_streams, _p(slot_ids),
+                  ctypes.c_void_p(ws.data_ptr() + off), ws.numel() - off, _stream(rows))
+        return out
 
     def forward(self, hidden: torch.Tensor, lengths: List[int], packed: bool = True) -> torch.Tensor:
         """``hidden (B, T, C)`` post-subsampling states, host ``lengths`` -> ``(B, T, C)`` fp32: the output of the

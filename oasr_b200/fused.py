@@ -309,6 +309,27 @@ def fmha_varlen_strided(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_se
     return out
 
 
+def fmha_window_supported(head_dim: int, chunk: int, left_chunks: int) -> bool:
+    """Does a chunked-limited window fit :func:`fmha_window_packed` / the streaming executor?"""
+    return bool(_lib.load().oasr_b200_fmha_window_supported(head_dim, chunk, left_chunks))
+
+
+def fmha_window_packed(qkv4: torch.Tensor, rel_k: torch.Tensor, center: int, cu_seqlens: torch.Tensor, max_seg_len: int, heads: int,
+                       chunk: int, left_chunks: int, scale: float) -> torch.Tensor:
+    """Windowed relative-position attention over packed rows (oasr/models/nemotron/encoder.py:82-149, 300-359):
+    ``qkv4 (total, 4*C)`` = ``[q+u | q+v | k | v]``, ``rel_k (rows, C)`` with the projection of distance ``d`` at row
+    ``center - d``; returns ``(total, C)``.  The work is linear in the frames."""
+    _need_cuda(qkv4, rel_k, cu_seqlens)
+    total, C = qkv4.size(0), qkv4.size(1) // 4
+    if not qkv4.is_contiguous() or not rel_k.is_contiguous() or rel_k.size(1) != C or rel_k.dtype != qkv4.dtype:
+        raise ValueError("qkv4 (total, 4*C) and rel_k (rows, C) must be contiguous and share a dtype")
+    out = torch.empty(total, C, device=qkv4.device, dtype=qkv4.dtype)
+    _lib.call("oasr_b200_fmha_window_packed", _p(out), _p(qkv4), _p(rel_k), rel_k.size(0), int(center), _p(cu_seqlens),
+              cu_seqlens.numel() - 1, int(max_seg_len), total, heads, C // heads, int(chunk), int(left_chunks), float(scale),
+              _DTYPE_ID[qkv4.dtype], _stream(qkv4))
+    return out
+
+
 def bmm_strided(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     """``out[i] = a[i] @ b[i]^T`` for views ``a (batch, M, K)``, ``b (batch, N, K)`` with unit stride along ``K`` and row /
     batch strides that are multiples of 8 elements: the operands are read in place (``oasr.bmm``,

@@ -10,6 +10,7 @@ logic; nothing here synchronises with the device.
 """
 from __future__ import annotations
 
+import ctypes
 from typing import List, Optional, Sequence
 
 import numpy as np
@@ -42,6 +43,7 @@ class StreamingCache:
         self.k_pool = torch.zeros(num_layers, self.num_blocks, block_size, heads, head_dim, device=self.device, dtype=dtype_pool)
         self.v_pool = torch.zeros_like(self.k_pool)
         self.cnn_state = torch.zeros(num_layers, max_streams, conv_kernel - 1, d_model, device=self.device, dtype=dtype)
+        self._pool_pointers = None
         # further per-stream buffers a front end keeps (leading dimension = slot); zeroed with the stream
         self.extra_state: List[torch.Tensor] = []
         # physical pages are handed out in a random order (a seeded permutation)
@@ -59,6 +61,14 @@ class StreamingCache:
         self._frames = np.zeros(max_streams, dtype=np.int64)
         self._offset = np.zeros(max_streams, dtype=np.int64)
         self._cols = np.arange(self.max_blocks, dtype=np.int64)[None, :]
+
+    def pool_pointers(self):
+        """Per-layer device pointers of the K and V pools as the host arrays the native executors take; built once."""
+        if self._pool_pointers is None:
+            step = self.k_pool.stride(0) * self.k_pool.element_size()
+            self._pool_pointers = tuple((ctypes.c_void_p * self.L)(*[pool.data_ptr() + i * step for i in range(self.L)])
+                                        for pool in (self.k_pool, self.v_pool))
+        return self._pool_pointers
 
     # ---- host bookkeeping -------------------------------------------------------------------
     @property
