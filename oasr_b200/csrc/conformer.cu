@@ -234,7 +234,7 @@ int oasr_b200_conformer_encode_packed(const oasr_b200_conformer_model* model, co
                     oasr_b200_gemm_add_norm_supported(d, m.ffn) != 0 && oasr_b200_gemm_add_norm_supported(d, m.embed_in) != 0;
   // Few rows: the Linear adds into the fp32 residual stream itself (its few output bytes cost nothing there) and the norm
   // reads the sum, which is then never rounded to 16 bits.
-  const bool resid = !fuse && qk == 0 && M <= gsm::kMaxRows;
+  const bool resid = !fuse && qk == 0;
   // add + norm; with an 8-bit kind (and an unsplit h) the kernel also leaves the quantised row of h in w.q8 / w.qs for
   // the Linear that reads h next, which then skips its own quantisation launch (OB_LINEAR_H)
 #define OB_ADD_NORM(hout, rout, rin, y_, alpha, mode, wa, ba, wb, bb, eps_, split)                                      \
@@ -250,7 +250,7 @@ int oasr_b200_conformer_encode_packed(const oasr_b200_conformer_model* model, co
     if (fuse) {                                                                                                     \
       OB_STEP("gemm_addnorm " label, fl, oasr_b200_gemm_add_norm_f32(hout, w.res, rin, in, wt, bs, M, d, K, alpha, mode, wa, ba, \
                                                                     wb, bb, eps_, split, dt, stream));              \
-    } else if (resid) {                                                                                             \
+    } else if (resid && gsm::takes(gsm::kResid, M, d, K)) {                                                                                             \
       OB_STEP("gemm " label, fl, gemm_residual_f32_op(w.res, rin, in, wt, bs, M, d, K, alpha, dt, stream, kInner));   \
       OB_ADD_NORM(hout, (mode) == 2 ? w.res : nullptr, w.res, nullptr, 0.0, mode, wa, ba, wb, bb, eps_, split);       \
     } else {                                                                                                        \
@@ -440,10 +440,9 @@ int oasr_b200_conformer_chunk_paged(const oasr_b200_conformer_model* model, cons
     else OB_STEP("gemm_q8 " label, fl, oasr_b200_gemm_q8(out, w.q8, w.qs, (lay).q_w[qi], (lay).q_s[qi], bs, M, N, d, act, 0, qk, dt, stream)); \
   } while (0)
   // last Linear of a sub-layer, residual step and norm; few rows: see the offline executor
-  const bool resid = qk == 0 && M <= gsm::kMaxRows;
 #define OB_CHUNK_LINEAR_ADDNORM(label, fl, hout, in, wt, bs, lay, qi, K, alpha, mode, wa, ba, wb, bb, split)          \
   do {                                                                                                                \
-    if (resid) {                                                                                                      \
+    if (qk == 0 && gsm::takes(gsm::kResid, M, d, K)) {                                                                \
       OB_STEP("gemm " label, fl, gemm_residual_f32_op(w.res, w.res, in, wt, bs, M, d, K, alpha, dt, stream, kInner));   \
       OB_ADD_NORM(hout, (mode) == 2 ? w.res : nullptr, w.res, nullptr, 0.0, mode, wa, ba, wb, bb, m.eps, split);        \
     } else {                                                                                                          \

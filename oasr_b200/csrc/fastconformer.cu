@@ -277,7 +277,7 @@ int oasr_b200_fastconformer_chunk_paged(const oasr_b200_fastconformer_model* mod
   // the fp32 stream itself
 #define FC_CHUNK_LINEAR_ADDNORM(in, wt, bs, K, alpha, mode, res_to, wa, ba, wb, bb)                                     \
   do {                                                                                                                \
-    if (M <= gsm::kMaxRows) {                                                                                         \
+    if (gsm::takes(gsm::kResid, M, C, K)) {                                                                           \
       FC_STEP(gemm_residual_f32_op(w.res, w.res, in, wt, bs, M, C, K, alpha, dt, stream, inner));                     \
       FC_STEP(oasr_b200_add_norm_f32(w.h, (mode) == 2 ? res_to : nullptr, w.res, nullptr, 0.0, mode, wa, ba, wb, bb, M, C, eps, 0, dt, stream)); \
     } else {                                                                                                          \

@@ -1248,7 +1248,9 @@ namespace ob {
 
 namespace gemm {
 // Dense 16-bit problems of few rows go to gemm_small.cu; a forced tile width names a kernel of this file.
-static bool small_rows(int64_t M, int64_t N, int64_t K) { return g_force_bn == 0 && gsm::takes(M, N, K); }
+static bool small_rows(int epi, int64_t M, int64_t N, int64_t K, int64_t dup_cols = 0) {
+  return g_force_bn == 0 && gsm::takes(epi, M, N, K, dup_cols);
+}
 }  // namespace gemm
 
 int gemm_op(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int activation, int dtype, void* stream, Chain chain) {
@@ -1259,7 +1261,7 @@ int gemm_op(void* D, const void* A, const void* B, const void* bias, int64_t M, 
   if (M == 0) return OASR_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (use_simt(M, N, K)) return gemm_simt_reference(D, A, B, bias, M, N, K, activation, dtype, s);
-  if (small_rows(M, N, K)) {
+  if (small_rows(gsm::kStore, M, N, K)) {
     gsm::Args a;
     a.D = D; a.A = A; a.B = B; a.bias = bias; a.M = M; a.N = N; a.K = K; a.act = activation;
     a.b_static = chain.b_static; a.late_launch = chain.late_launch;
@@ -1282,7 +1284,7 @@ int gemm_dup_first_op(void* D, const void* A, const void* B, const void* bias, i
              (long long)N, (long long)dup_cols);
   if (M == 0) return OASR_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (small_rows(M, N, K)) {
+  if (small_rows(gsm::kDup, M, N, K, dup_cols)) {
     gsm::Args a;
     a.D = D; a.A = A; a.B = B; a.bias = bias; a.M = M; a.N = N; a.K = K; a.dup_cols = dup_cols;
     a.b_static = chain.b_static; a.late_launch = chain.late_launch;
@@ -1330,7 +1332,7 @@ int gemm_residual_f32_op(float* R_out, const float* R_in, const void* A, const v
   if (int rc = validate_common("gemm_residual_f32", R_out, A, B, bias, M, N, K)) return rc;
   OB_REQUIRE(M == 0 || !R_in || is_aligned(R_in, 16), OASR_ERR_ALIGN, "gemm_residual_f32: residual pointer unaligned");
   if (M == 0) return OASR_OK;
-  if (small_rows(M, N, K)) {
+  if (small_rows(gsm::kResid, M, N, K)) {
     gsm::Args a;
     a.D = R_out; a.R_in = R_in; a.A = A; a.B = B; a.bias = bias; a.M = M; a.N = N; a.K = K; a.alpha = static_cast<float>(alpha);
     a.b_static = chain.b_static; a.late_launch = chain.late_launch;
@@ -1349,7 +1351,7 @@ int gemm_glu_op(void* D, const void* A, const void* B, const void* bias, int64_t
   using namespace ob::gemm;
   if (int rc = validate_common("gemm_glu", D, A, B, bias, M, N, K)) return rc;
   if (M == 0) return OASR_OK;
-  if (g_force_bn == 0 && gsm::takes_glu(M, N, K)) {
+  if (small_rows(gsm::kGlu, M, N, K)) {
     gsm::Args a;
     a.D = D; a.A = A; a.B = B; a.bias = bias; a.M = M; a.N = N; a.K = K;
     a.b_static = chain.b_static; a.late_launch = chain.late_launch;
@@ -1380,7 +1382,7 @@ int gemm_log_softmax_op(void* out, const void* A, const void* B, const void* bia
   const bool split_ok = out_dtype == OASR_DT_F32 && !use_simt(M, N, K) && !tokens_only;
   const bool split = split_ok && (g_lsm_path == 2 || (g_lsm_path == 0 && lsm_split_wins(M, N, K)));
   if (split) {
-    if (small_rows(M, N, K)) {
+    if (small_rows(gsm::kResid, M, N, K)) {
       gsm::Args a;
       a.D = out; a.A = A; a.B = B; a.bias = bias; a.M = M; a.N = N; a.K = K;
       a.b_static = chain.b_static; a.late_launch = chain.late_launch;

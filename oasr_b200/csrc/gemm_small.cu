@@ -22,8 +22,9 @@
 //     refill a round trip through MMA, commit, producer and L2: 8 single-block stages took 2.3 us for 16 rows.
 //   * the exchange is pushed (st.async credited to the owner's mbarrier), so that an owner waits for its data and not for
 //     a cluster-wide barrier.
-// The number of splits depends on K only, and a tile's K order never depends on M, so a row's result does not depend on
-// the rows that share its batch (as long as the batch stays on this kernel).
+// The number of splits depends on N and K only, and a tile's K order never depends on M; unsplit products give the bits of
+// gemm.cu.  So up to kMaxRows a row's result does not depend on the rows that share its batch, for all outputs of up to 512
+// columns and all unsplit ones.
 //
 // Roles: warp 0 TMA producer, warp 1 MMA issuer and tensor-memory owner, the other 4 (128-wide tiles: 8) epilogue, a
 // thread per row (and column half); output goes through padded shared memory so that global accesses are coalesced.
@@ -69,7 +70,7 @@ struct Geo {
   static constexpr int kBBlk = BN * BK * 2;                       // one K block of B
   static constexpr int kW = BN / S;                               // columns of the tile this CTA owns after the exchange
   static constexpr int kHead = 2048;                              // 2 * BN floats of bias, 2 * kMaxStages + 2 barriers, flags
-  static constexpr int kRecv = S == 1 ? 0 : BM * BN * 4;          // [source rank][4-column group][row] float4
+  static constexpr int kRecv = (S - 1) * kW * BM * 4;            // [other rank][4-column group][row] float4
   static constexpr int kEpiWarps = BN == 128 ? 8 : 4;
   static constexpr int kThreads = 64 + 32 * kEpiWarps;
   static constexpr int kHalves = kEpiWarps / 4;                   // epilogue warps that share a row
@@ -95,6 +96,14 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
     __half2 v = __floats2half2_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&v);
   }
+}
+
+template <int kCols>
+__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t* r) {
+  static_assert(kCols == 8 || kCols == 16 || kCols == 32, "columns of one tensor-memory load");
+  if constexpr (kCols == 32) ptx::tmem_ld_32x32(taddr, *reinterpret_cast<uint32_t(*)[32]>(r));
+  else if constexpr (kCols == 16) ptx::tmem_ld_32x16(taddr, *reinterpret_cast<uint32_t(*)[16]>(r));
+  else ptx::tmem_ld_32x8(taddr, *reinterpret_cast<uint32_t(*)[8]>(r));
 }
 
 // S = CTAs of a cluster that share one tile's K range.
@@ -322,38 +331,45 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     const int shift = kEpi == kDup && !twice ? p.dup_cols : 0;
 
     if constexpr (S > 1) {
-      uint32_t acc[BN];
-      if constexpr (BN == 64) ptx::tmem_ld_32x64(t_acc, acc);
-      else ptx::tmem_ld_32x32(t_acc, acc);
-      ptx::tmem_ld_wait();
-      // column (relative to the tile) of the i-th value that CTA j owns
-      auto owned = [](int j, int i) -> int {
-        if constexpr (kEpi == kGlu) return i < kOutAll ? j * kOutAll + i : BN / 2 + j * kOutAll + (i - kOutAll);
-        else return j * W + i;
+      // A thread exchanges the columns it will finish: of every CTA's W columns the WH from `half` on (GLU: half of the value
+      // and the gate columns behind them).  i-th of them, owner j, relative to the tile:
+      auto owned = [&](int j, int i) -> int {
+        if constexpr (kEpi == kGlu) return (i < kOutW ? 0 : BN / 2 - kOutW) + j * kOutAll + hc + i;
+        else return j * W + hc + i;
       };
-      cluster_wait();
-      float own[W];
+      constexpr int kLd = kEpi == kGlu ? kOutW : WH;      // contiguous columns per tensor-memory load
+      float4* mine = recv + (half * (WH / 4)) * BM + row;
+      auto slot_of = [](int from, int to) { return from < to ? from : from - 1; };   // of `from`'s partial sums in `to`'s buffer
+      uint32_t all[S * WH];
 #pragma unroll
       for (int j = 0; j < S; ++j) {
+#pragma unroll
+        for (int c = 0; c < WH; c += kLd) tmem_ld_cols<kLd>(t_acc + owned(j, c), all + j * WH + c);
+      }
+      ptx::tmem_ld_wait();
+      cluster_wait();
+      float own[WH];
+#pragma unroll
+      for (int j = 0; j < S; ++j) {
+        const uint32_t* acc = all + j * WH;
         if (j == rank) {
 #pragma unroll
-          for (int i = 0; i < W; ++i) own[i] = __uint_as_float(acc[owned(j, i)]);
+          for (int i = 0; i < WH; ++i) own[i] = __uint_as_float(acc[i]);
         } else {
-          const uint32_t dst = ptx::map_to_cta(recv + rank * (W / 4) * BM + row, j), bar = ptx::map_to_cta(recv_bar, j);
+          const uint32_t dst = ptx::map_to_cta(mine + slot_of(rank, j) * (W / 4) * BM, j), bar = ptx::map_to_cta(recv_bar, j);
 #pragma unroll
-          for (int i = 0; i < W; i += 4)
-            st_async_v4(dst + (i / 4) * BM * 16, bar, acc[owned(j, i)], acc[owned(j, i + 1)], acc[owned(j, i + 2)], acc[owned(j, i + 3)]);
+          for (int i = 0; i < WH; i += 4) st_async_v4(dst + (i / 4) * BM * 16, bar, acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
         }
       }
       ok = ptx::mbar_wait(recv_bar, 0, abort_flag) && ok;
       // sum in rank order, so that the result does not depend on which CTA adds
-      float sum[W];
+      float sum[WH];
 #pragma unroll
       for (int j = 0; j < S; ++j) {
 #pragma unroll
-        for (int i = 0; i < W; i += 4) {
+        for (int i = 0; i < WH; i += 4) {
           float4 v = make_float4(own[i], own[i + 1], own[i + 2], own[i + 3]);
-          if (j != rank) v = recv[(j * (W / 4) + i / 4) * BM + row];
+          if (j != rank) v = mine[(slot_of(j, rank) * (W / 4) + i / 4) * BM];
           if (j == 0) { sum[i] = v.x; sum[i + 1] = v.y; sum[i + 2] = v.z; sum[i + 3] = v.w; }
           else { sum[i] += v.x; sum[i + 1] += v.y; sum[i + 2] += v.z; sum[i + 3] += v.w; }
         }
@@ -366,18 +382,18 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           for (int i = 0; i < 8; ++i) { v[i] = sum[c + i]; g[i] = sum[kOutW + c + i]; }
           finish_glu8(v, g, c);
         }
-        flush(col0);
+        flush(col0 + hc);
       } else {
 #pragma unroll 1
         for (int pass = 0; pass < (twice ? 2 : 1); ++pass) {
 #pragma unroll
-          for (int c = 0; c < W; c += 8) {
+          for (int c = 0; c < WH; c += 8) {
             float v[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = sum[c + i];
             finish8(v, c, pass);
           }
-          flush(col0 + shift + pass * p.dup_cols);
+          flush(col0 + hc + shift + pass * p.dup_cols);
         }
       }
     } else if constexpr (kEpi == kGlu) {
@@ -432,18 +448,55 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
-// CTAs per cluster: about 512 elements of K each.  A function of K only: see the header comment.
-int splits_for(int64_t K) {
-  if (K < 1024) return 1;
-  if (K < 2048) return 2;
-  if (K < 4096) return 4;
-  return 8;
+// CTAs per cluster: about 512 elements of K each while N / 64 tiles times the splits stay within 64 CTAs per 128 rows; a
+// wide product has enough tiles of its own, and an unsplit one gives the bits of gemm.cu.  A function of N and K only: see
+// the header comment.
+int splits_for(int64_t n_acc, int64_t K) {
+  int s = K < 1024 ? 1 : (K < 2048 ? 2 : (K < 4096 ? 4 : 8));
+  while (s > 1 && (n_acc + 63) / 64 * s > 64) s >>= 1;
+  return s;
 }
 
-// Where the kernel wins: the operand bytes per SM grow with M as in gemm.cu, but each CTA runs its phases (operands,
-// exchange, output) once and in series, so past a few waves the persistent kernel with its overlapped epilogue is ahead.
-bool takes(int64_t M, int64_t N, int64_t K) {
-  return M > 0 && M <= kMaxRows && N >= 32 && K >= 64;
+// Tile width: the one that leaves the fewest operand bytes on the busiest SM (a column tile costs its own rows of B and the
+// rows of A that exist, and about 24 rows' worth of fixed time); ties go to the wider tile, which moves fewer bytes in all.
+int pick_bn(int epi, int64_t M, int64_t n_acc, int S, int64_t dup_cols, int64_t* ctas_out) {
+  const int64_t m_tiles = (M + BM - 1) / BM;
+  const int rows = static_cast<int>(M < BM ? M : BM);
+  int bn = 64;
+  double best = 1e30;
+  for (int cand = ((S == 1 && epi == kResid) || S == 8 ? 64 : 128); cand >= 32; cand >>= 1) {
+    if (cand == 32 && (epi == kGlu || S == 8)) continue;   // at least 8 output columns per CTA
+    if (epi == kDup && dup_cols % cand) continue;
+    const int64_t ctas = m_tiles * ((n_acc + cand - 1) / cand) * S;
+    const int64_t per_sm = (ctas + sm_count() - 1) / sm_count();
+    const double cost = static_cast<double>(per_sm) * (rows + cand + 24);
+    if (cost < best * 0.999) {
+      best = cost;
+      bn = cand;
+      if (ctas_out) *ctas_out = ctas;
+    }
+  }
+  return bn;
+}
+
+// Where the kernel is ahead of the persistent one (B200, weights from HBM, us here / there):
+//   N 512, K 2048:  592 rows 5.4 / 17.1, 2048 rows 16.6 / 17.8, 4096 rows 32.7 / 23.8
+//   N 2048, K 512:  512 rows 4.5 / 6.3, 2560 rows 11.6 / 18.2, 4096 rows 13.8 / 12.7
+//   N 4096, K 1024: 512 rows 7.7 / 9.8, 1536 rows 17.9 / 21.0, 2048 rows 19.9 / 18.3
+//   N 1024, K 4096: 512 rows 11.0 / 27.2, 1024 rows 25.0 / 27.5, 1536 rows 35.5 / 33.3
+// Each CTA runs its phases (operands, exchange, output) once and in series, so what counts is the number of CTAs: an SM
+// hides them with two or three.  Narrow outputs (N up to 512) keep the kernel over its whole range: their K split changes
+// the bits, and a row's result is not to depend on its batch.
+bool takes(int epi, int64_t M, int64_t N, int64_t K, int64_t dup_cols) {
+  if (M <= 0 || M > kMaxRows || N < 32 || K < 64) return false;
+  const int64_t n_acc = epi == kGlu ? 2 * N : N;
+  const int S = splits_for(n_acc, K);
+  if (epi == kGlu && (N % 32 || S > 4)) return false;
+  if (S > 1 && n_acc <= 512) return true;
+  if (S == 1 && epi == kResid) return true;        // gemm.cu stores fp32 rows a thread each
+  int64_t ctas = 0;
+  pick_bn(epi, M, n_acc, S, dup_cols, &ctas);
+  return S > 1 ? ctas * 5 <= 9 * sm_count() : ctas * 5 <= 13 * sm_count();
 }
 
 template <typename T, int BN, int S, int kEpi>
@@ -456,8 +509,8 @@ int launch(const Args& a, Params& p, int m_tiles, int dtype, cudaStream_t s) {
   const int rows = static_cast<int>(a.M < BM ? (a.M + 7) / 8 * 8 : BM);
   p.a_blk = rows * BK * 2;
   const int fixed = 1024 + G::kHead + G::kRecv + (rows < BM ? 16384 - p.a_blk : 0), blk = p.a_blk + G::kBBlk;
-  const bool alone = static_cast<int64_t>(m_tiles) * n_tiles * S <= sm_count();
-  const int fit = ((alone ? 227 : 113) * 1024 - fixed) / blk;
+  int fit = (113 * 1024 - fixed) / blk;
+  if (fit < 3 || static_cast<int64_t>(m_tiles) * n_tiles * S <= sm_count()) fit = (227 * 1024 - fixed) / blk;
   const int whole = fit < p.kb_per ? fit : p.kb_per;              // K blocks held at a time
   p.kg = !p.k_whole || whole < 4 ? 1 : (whole > 2 * kMaxStages ? 4 : 2);
   p.stages = whole / p.kg < kMaxStages ? whole / p.kg : kMaxStages;
@@ -509,21 +562,9 @@ template <typename T, int kEpi>
 int run_typed(const Args& a, Params& p, int dtype, cudaStream_t s) {
   constexpr bool kGluE = kEpi == kGlu;
   const int64_t n_acc = kGluE ? 2 * a.N : a.N;
-  const int S = splits_for(a.K);
+  const int S = splits_for(n_acc, a.K);
   const int m_tiles = static_cast<int>((a.M + BM - 1) / BM);
-  // Tile width: the one that leaves the fewest operand bytes on the busiest SM (a column tile costs its own rows of B and
-  // the rows of A that exist); ties go to the wider tile, which moves fewer bytes in all.
-  const int rows = static_cast<int>(a.M < BM ? a.M : BM);
-  int bn = 64;
-  double best = 1e30;
-  for (int cand = (S == 1 && kEpi != kResid ? 128 : 64); cand >= 32; cand >>= 1) {
-    if (cand == 32 && (kGluE || S == 8)) continue;   // at least 8 output columns per CTA
-    if (kEpi == kDup && a.dup_cols % cand) continue;
-    const int64_t ctas = static_cast<int64_t>(m_tiles) * ((n_acc + cand - 1) / cand) * S;
-    const int64_t per_sm = (ctas + sm_count() - 1) / sm_count();
-    const double cost = static_cast<double>(per_sm) * (rows + cand + 24);     // 24 rows' worth of fixed cost per tile
-    if (cost < best * 0.999) { best = cost; bn = cand; }
-  }
+  const int bn = pick_bn(kEpi, a.M, n_acc, S, a.dup_cols, nullptr);
   p.kb_total = static_cast<int>((a.K + BK - 1) / BK);
   p.kb_per = (p.kb_total + S - 1) / S;
   p.k_whole = a.K % BK == 0;
@@ -538,12 +579,14 @@ int run_typed(const Args& a, Params& p, int dtype, cudaStream_t s) {
     GSM_CASE(64, 1);
   }
   if (S == 2) {
+    if (bn == 128) GSM_CASE(128, 2);
     if constexpr (!kGluE) {
       if (bn == 32) GSM_CASE(32, 2);
     }
     GSM_CASE(64, 2);
   }
   if (S == 4) {
+    if (bn == 128) GSM_CASE(128, 4);
     if constexpr (!kGluE) {
       if (bn == 32) GSM_CASE(32, 4);
     }
@@ -553,8 +596,6 @@ int run_typed(const Args& a, Params& p, int dtype, cudaStream_t s) {
   return set_error(OASR_ERR_UNSUPPORTED, "gemm_small: no kernel for this shape");
 #undef GSM_CASE
 }
-
-bool takes_glu(int64_t M, int64_t N, int64_t K) { return takes(M, N, K) && N % 32 == 0 && splits_for(K) <= 4; }
 
 int run(int epi, const Args& a, int dtype, cudaStream_t s) {
   Params p{};

@@ -24,11 +24,10 @@ struct Args {
   int late_launch = 0;
 };
 
-// Rows up to which the kernel is used.
+// Rows up to which the kernel is used (takes() says where).
 constexpr int64_t kMaxRows = 2560;
 
-bool takes(int64_t M, int64_t N, int64_t K);
-bool takes_glu(int64_t M, int64_t N, int64_t K);
+bool takes(int epi, int64_t M, int64_t N, int64_t K, int64_t dup_cols = 0);
 int run(int epi, const Args& a, int dtype, cudaStream_t s);
 
 }  // namespace gsm
