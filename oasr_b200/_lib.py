@@ -239,9 +239,17 @@ def check(code: int) -> None:
     raise OasrB200Error(code, msg)
 
 
+_entry = {}    # name -> bound entry point
+
+
 def call(name: str, *args) -> None:
     if _call_hook is None:
-        check(getattr(load(), name)(*args))
+        fn = _entry.get(name)
+        if fn is None:
+            fn = _entry[name] = getattr(load(), name)
+        code = fn(*args)
+        if code:
+            check(code)
         return
     _call_hook(name, "begin", args)
     try:

@@ -10,6 +10,7 @@ from . import _lib
 from .functional import _DTYPE_ID, _need_cuda, _p, _stream
 
 _HALF = (torch.float16, torch.bfloat16)
+_Strides = ctypes.c_int64 * 3
 
 
 def _strides3(t: torch.Tensor):
@@ -21,8 +22,7 @@ def _strides3(t: torch.Tensor):
     for extent, s in zip(t.shape[:3], st):
         if extent > 1 and (s <= 0 or s % 8):
             return None
-    st = [s if e > 1 else 8 for e, s in zip(t.shape[:3], st)]
-    return (ctypes.c_int64 * 3)(*st)
+    return _Strides(*[s if e > 1 else 8 for e, s in zip(t.shape[:3], st)])
 
 
 def _canon(t: torch.Tensor):
@@ -200,8 +200,9 @@ def fmha_varlen(q, k, v, *, softmax_scale: float, cu_seqlens_q: torch.Tensor, cu
         bias_offsets = bias_offsets.contiguous()
         attn_bias = attn_bias.contiguous()
     S = cu_seqlens_q.numel() - 1
+    cu_seqlens_q, cu_seqlens_k = cu_seqlens_q.contiguous(), cu_seqlens_k.contiguous()
     _lib.call("oasr_b200_fmha_varlen", _p(out), _p(q), _p(k), _p(v), _p(attn_bias), _p(bias_offsets), off_i64,
-              _p(cu_seqlens_q.contiguous()), _p(cu_seqlens_k.contiguous()), S, q.size(0), k.size(0),
+              _p(cu_seqlens_q), _p(cu_seqlens_k), S, q.size(0), k.size(0),
               int(max_seqlen_q), q.size(1), k.size(1), q.size(2), float(softmax_scale), _DTYPE_ID[q.dtype],
               _stream(q))
     return out

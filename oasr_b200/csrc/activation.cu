@@ -2,6 +2,7 @@
 // grid sized as a multiple of the SM count.  Algorithmic bytes (16-bit type):
 // GLU 6C per output row of width C, swish 4 per element.
 #include "common.cuh"
+#include "sm100_ptx.cuh"
 
 namespace ob {
 namespace {
@@ -9,6 +10,8 @@ namespace {
 template <typename T>
 __global__ void __launch_bounds__(256) glu_vec_kernel(T* __restrict__ out, const T* __restrict__ in,
                                                       int64_t rows, int channels) {
+  ptx::grid_dep_launch();   // no-ops unless launched with programmatic stream serialisation
+  ptx::grid_dep_wait();
   constexpr int V = Elem<T>::kVec;
   const int ppr = channels / V;
   const int64_t total = rows * ppr;
@@ -43,6 +46,8 @@ __global__ void __launch_bounds__(256) glu_scalar_kernel(T* __restrict__ out, co
 template <typename T>
 __global__ void __launch_bounds__(256) swish_vec_kernel(T* __restrict__ out, const T* __restrict__ in,
                                                         int64_t packs) {
+  ptx::grid_dep_launch();   // no-ops unless launched with programmatic stream serialisation
+  ptx::grid_dep_wait();
   constexpr int V = Elem<T>::kVec;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; p < packs; p += stride) {
@@ -273,7 +278,7 @@ int oasr_b200_glu(void* out, const void* in, int64_t rows, int64_t channels, int
   return OB_DISPATCH_FLOAT(dtype, T, [&]() -> int {
     constexpr int V = Elem<T>::kVec;
     if (channels % V == 0 && is_aligned(in, 16) && is_aligned(out, 16)) {
-      glu_vec_kernel<T><<<grid_for(rows * (channels / V), 256), 256, 0, s>>>(
+      launch_pdl(glu_vec_kernel<T>, dim3(grid_for(rows * (channels / V), 256)), dim3(256), 0, s,
           static_cast<T*>(out), static_cast<const T*>(in), rows, (int)channels);
     } else {
       glu_scalar_kernel<T><<<grid_for(rows * channels, 256), 256, 0, s>>>(
@@ -296,7 +301,7 @@ int oasr_b200_swish(void* out, const void* in, int64_t numel, int dtype, void* s
       const int64_t packs = numel / V;
       vec_elems = packs * V;
       if (packs > 0) {
-        swish_vec_kernel<T><<<grid_for(packs, 256), 256, 0, s>>>(static_cast<T*>(out),
+        launch_pdl(swish_vec_kernel<T>, dim3(grid_for(packs, 256)), dim3(256), 0, s, static_cast<T*>(out),
                                                                   static_cast<const T*>(in), packs);
       }
     }

@@ -419,12 +419,14 @@ __global__ void __launch_bounds__(256, 2) dwconv_stream_kernel(DwArgs a) {
 // and an output costs its K two-channel FMAs, one load, the unpack / pack, the activation and the store.
 constexpr int kRollRuns = 4;   // 2 and 4 measure the same (0.253-0.256 ms for the 12 launches of a step), 8 is slower (0.349)
 
-template <typename T, int K, bool kAffine, int kAct>
+// kRuns: runs of K frames per thread, 4, or 1 where 4 would leave SMs without a block (a thread's frames are a serial chain:
+// 78 frames of one utterance 5.8 us with 4, 4.2 us with 1).  kMask: the operator's bool time mask and its add_input.
+template <typename T, int K, bool kAffine, int kAct, int kRuns, bool kMask>
 __global__ void __launch_bounds__(128, 4) dwconv_roll_kernel(DwArgs a) {
   static_assert(sizeof(T) == 2, "16-bit element types only");
   ptx::grid_dep_launch();   // no-ops unless launched with programmatic stream serialisation
   ptx::grid_dep_wait();
-  constexpr int kRun = kRollRuns * K;
+  constexpr int kRun = kRuns * K;
   const int C = a.channels;
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 2;
   if (c >= C) return;
@@ -447,10 +449,14 @@ __global__ void __launch_bounds__(128, 4) dwconv_roll_kernel(DwArgs a) {
   }
   const uint32_t* __restrict__ in = reinterpret_cast<const uint32_t*>(static_cast<const T*>(a.in) + in_row0 * C + c);
   const int64_t row_u32 = C / 2;
+  const uint8_t* mask = kMask && a.mask ? static_cast<const uint8_t*>(a.mask) + b * a.seq_len : nullptr;
   auto fetch = [&](int ti) -> uint32_t {    // input frame ti of the segment: data, the fill value past its end, else zero
     uint32_t v = 0;
-    if (ti >= 0 && ti < TL) v = __ldg(in + ti * row_u32);
-    else if (ti >= TL && ti < fill_end) v = fill;
+    if (ti >= 0 && ti < TL) {
+      if (!kMask || !mask || mask[ti]) v = __ldg(in + ti * row_u32);
+    } else if (ti >= TL && ti < fill_end) {
+      v = fill;
+    }
     return v;
   };
   float2 w[K];
@@ -489,6 +495,15 @@ __global__ void __launch_bounds__(128, 4) dwconv_roll_kernel(DwArgs a) {
       float2 acc = bias;
 #pragma unroll
       for (int k = 0; k < K; ++k) acc = __ffma2_rn(x[(s + k) % K], w[k], acc);
+      if constexpr (kMask) {
+        const int t = base + s;
+        if (a.add_input && t < t_end) {
+          const float2 xc = unpack_pair<T>(fetch(t));
+          acc.x += xc.x;
+          acc.y += xc.y;
+        }
+        if (mask && t < t_end && !mask[t]) acc = make_float2(0.f, 0.f);
+      }
       if constexpr (kAct == 1) {
         const float2 h = __fmul2_rn(acc, make_float2(0.5f, 0.5f));
         acc = __ffma2_rn(h, make_float2(tanh_approx(h.x), tanh_approx(h.y)), h);
@@ -508,20 +523,26 @@ int launch_roll(const DwArgs& a, int max_out_len, cudaStream_t s) {
   } else {
     const int pairs = a.channels / 2;
     const int threads = pairs >= 128 ? 128 : ((pairs + 31) / 32) * 32;
-    constexpr int kRun = kRollRuns * K;
-    dim3 block(threads);
-    dim3 grid((max_out_len + kRun - 1) / kRun, (pairs + threads - 1) / threads, static_cast<unsigned>(a.batch));
+    const int64_t per_run = static_cast<int64_t>((pairs + threads - 1) / threads) * a.batch;     // blocks of one run of frames
+    const bool masked = a.mask != nullptr || a.add_input;
+    const bool few = !masked && (max_out_len + kRollRuns * K - 1) / (kRollRuns * K) * per_run < 2 * sm_count();
+    const int run = (few ? 1 : kRollRuns) * K;
+    const dim3 block(threads), grid((max_out_len + run - 1) / run, (pairs + threads - 1) / threads, static_cast<unsigned>(a.batch));
     const bool affine = a.post_scale != nullptr;
     const int act = a.act == OASR_ACT_NONE ? 0 : (a.act == OASR_ACT_SWISH ? 1 : 2);
-    if (affine) {
-      if (act == 1) launch_pdl(dwconv_roll_kernel<T, K, true, 1>, grid, block, 0, s, a);
-      else if (act == 0) launch_pdl(dwconv_roll_kernel<T, K, true, 0>, grid, block, 0, s, a);
-      else launch_pdl(dwconv_roll_kernel<T, K, true, 2>, grid, block, 0, s, a);
-    } else {
-      if (act == 1) launch_pdl(dwconv_roll_kernel<T, K, false, 1>, grid, block, 0, s, a);
-      else if (act == 0) launch_pdl(dwconv_roll_kernel<T, K, false, 0>, grid, block, 0, s, a);
-      else launch_pdl(dwconv_roll_kernel<T, K, false, 2>, grid, block, 0, s, a);
-    }
+#define OB_ROLL(AFFINE, ACT)                                                                                    \
+  do {                                                                                                          \
+    if (few) launch_pdl(dwconv_roll_kernel<T, K, AFFINE, ACT, 1, false>, grid, block, 0, s, a);                 \
+    else launch_pdl(dwconv_roll_kernel<T, K, AFFINE, ACT, kRollRuns, false>, grid, block, 0, s, a);             \
+  } while (0)
+    if (masked) launch_pdl(dwconv_roll_kernel<T, K, false, 2, kRollRuns, true>, grid, block, 0, s, a);
+    else if (affine && act == 1) OB_ROLL(true, 1);
+    else if (affine && act == 0) OB_ROLL(true, 0);
+    else if (affine) OB_ROLL(true, 2);
+    else if (act == 1) OB_ROLL(false, 1);
+    else if (act == 0) OB_ROLL(false, 0);
+    else OB_ROLL(false, 2);
+#undef OB_ROLL
     return check_launch("depthwise_conv1d (rolling) kernel launch");
   }
 }
@@ -603,17 +624,22 @@ int launch_window(const DwArgs& a, int max_out_len, cudaStream_t s) {
 template <typename T>
 int launch_dw(const DwArgs& a, int max_out_len, cudaStream_t s) {
   const bool plain = a.mask == nullptr && !a.add_input;
-  const bool fast = plain && a.channels % 2 == 0 && is_aligned(a.in, 2 * sizeof(T)) &&
+  const bool even = a.channels % 2 == 0 && is_aligned(a.in, 2 * sizeof(T)) &&
                     is_aligned(a.out, 2 * sizeof(T)) && is_aligned(a.weight, 2 * sizeof(T)) &&
                     (!a.bias || is_aligned(a.bias, 2 * sizeof(T))) && a.batch <= 65535 &&
                     (max_out_len + kTile - 1) / kTile <= 65535;
+  const bool fast = plain && even;
   const bool tiled = fast && (a.channels * sizeof(T)) % 16 == 0 && (a.channels % kCB == 0 || a.channels < kCB) &&
                      is_aligned(a.in, 16) && (max_out_len + kTT - 1) / kTT <= 65535 &&
                      (a.channels + kCB - 1) / kCB <= 65535;
-  const bool stream = fast && sizeof(T) == 2 && is_aligned(a.in, 4) && is_aligned(a.out, 4) && is_aligned(a.weight, 4) &&
+  const bool words = even && sizeof(T) == 2 && is_aligned(a.in, 4) && is_aligned(a.out, 4) && is_aligned(a.weight, 4) &&
                       (!a.bias || is_aligned(a.bias, 4)) && (!a.post_scale || (is_aligned(a.post_scale, 8) && is_aligned(a.post_shift, 8))) &&
                       (max_out_len + kST - 1) / kST <= 65535 && a.kernel_size <= 15 && g_dw_path != 1;
-  if (stream && g_dw_path == 2) {
+  const bool stream = words && plain;
+  // the rolling kernel also takes a bool mask and add_input (operators without an affine step; an element-typed mask scales
+  // and stays with the general kernel)
+  const bool rolled = words && (plain || ((!a.mask || a.mask_is_bool) && !a.post_scale && !a.cu_seqlens));
+  if (rolled && g_dw_path == 2) {
     switch (a.kernel_size) {
       case 9: return launch_roll<T, 9>(a, max_out_len, s);
       case 15: return launch_roll<T, 15>(a, max_out_len, s);

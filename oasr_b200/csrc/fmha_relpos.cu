@@ -574,6 +574,8 @@ int run(void* out, const void* qkv4, const void* pos, int64_t pos_rows, int64_t 
 // ranks before it.  plan = [int32 n_items, pad to 16 bytes][int2 items...].
 constexpr int kPlanMaxSegs = 1024;
 __global__ void __launch_bounds__(kPlanMaxSegs) plan_kernel(int32_t* plan, const int32_t* __restrict__ cu, int S, int H) {
+  ptx::grid_dep_launch();   // no-ops unless launched with programmatic stream serialisation
+  ptx::grid_dep_wait();
   __shared__ int len[kPlanMaxSegs];
   __shared__ int seg_of_rank[kPlanMaxSegs];
   __shared__ int start[kPlanMaxSegs + 1];
@@ -616,7 +618,7 @@ __global__ void __launch_bounds__(kPlanMaxSegs) plan_kernel(int32_t* plan, const
 int64_t plan_bytes(int64_t num_segs, int64_t H, int64_t total) { return 16 + 8 * H * (total / BQ + num_segs); }
 
 int plan(void* plan_buf, const int32_t* cu_seqlens, int64_t num_segs, int64_t H, cudaStream_t stream) {
-  plan_kernel<<<1, kPlanMaxSegs, 0, stream>>>(static_cast<int32_t*>(plan_buf), cu_seqlens, static_cast<int>(num_segs),
+  launch_pdl(plan_kernel, dim3(1), dim3(kPlanMaxSegs), 0, stream, static_cast<int32_t*>(plan_buf), cu_seqlens, static_cast<int>(num_segs),
                                               static_cast<int>(H));
   return check_launch("fmha_relpos_plan launch");
 }

@@ -989,6 +989,8 @@ int pick_bn(int64_t m_tiles_total, int64_t N, int64_t K = 512) {
 // (up to 8192 columns; longer rows are re-read), max and sum reduced across the block.
 __global__ void __launch_bounds__(256) log_softmax_rows_f32_kernel(float* __restrict__ x, int32_t* __restrict__ argmax,
                                                                    int M, int N) {
+  ptx::grid_dep_launch();   // no-ops unless launched with programmatic stream serialisation
+  ptx::grid_dep_wait();
   constexpr int kCache = 8;
   __shared__ float s_val[8];
   __shared__ int s_idx[8];
@@ -1396,7 +1398,7 @@ int gemm_log_softmax_op(void* out, const void* A, const void* B, const void* bia
     if (int rc = run<kSchedDense, kEpiResid>(pg, dtype, static_cast<cudaStream_t>(stream))) return rc;
     }
     int64_t g = M < static_cast<int64_t>(sm_count()) * 8 ? M : static_cast<int64_t>(sm_count()) * 8;
-    log_softmax_rows_f32_kernel<<<static_cast<unsigned>(g), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    launch_pdl(log_softmax_rows_f32_kernel, dim3(static_cast<unsigned>(g)), dim3(256), 0, static_cast<cudaStream_t>(stream),
         static_cast<float*>(out), argmax, (int)M, (int)N);
     return check_launch("log_softmax_rows launch");
   }

@@ -73,6 +73,8 @@ struct NormArgs {
 // TIn: type of in/residual; TOut: type of out/res_out; TW: type of weight/bias.
 template <typename TIn, typename TOut, typename TW, int kChunks, bool kRms, bool kAdd, bool kAct>
 __global__ void __launch_bounds__(128) norm_warp_rows_kernel(NormArgs a) {
+  ptx::grid_dep_launch();   // no-ops unless launched with programmatic stream serialisation
+  ptx::grid_dep_wait();
   const int lane = threadIdx.x & 31;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= a.rows) return;
@@ -211,7 +213,7 @@ int launch_norm(const NormArgs& a, cudaStream_t stream) {
     const int warps = 4;
     const unsigned grid = static_cast<unsigned>((a.rows + warps - 1) / warps);
 #define OB_NORM_CASE(C)                                                                          \
-  norm_warp_rows_kernel<TIn, TOut, TW, C, kRms, kAdd, kAct><<<grid, warps * 32, 0, stream>>>(a)
+  launch_pdl(norm_warp_rows_kernel<TIn, TOut, TW, C, kRms, kAdd, kAct>, dim3(grid), dim3(warps * 32), 0, stream, a)
     if (chunks <= 1) OB_NORM_CASE(1);
     else if (chunks <= 2) OB_NORM_CASE(2);
     else if (chunks <= 4) OB_NORM_CASE(4);
@@ -271,6 +273,8 @@ struct BnArgs {
 // per-channel scale/shift are computed once per thread.
 template <typename T, bool kAct>
 __global__ void __launch_bounds__(256) batch_norm_vec_kernel(BnArgs a) {
+  ptx::grid_dep_launch();   // no-ops unless launched with programmatic stream serialisation
+  ptx::grid_dep_wait();
   const int ppr = a.channels / kGran;  // packs per row
   const int64_t total = a.rows * ppr;
   const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -337,7 +341,7 @@ int launch_bn(const BnArgs& a, cudaStream_t s) {
     const int64_t cap = static_cast<int64_t>(sm_count()) * 8;
     if (want > cap) want = cap;
     int64_t grid = ((want + unit - 1) / unit) * unit;
-    batch_norm_vec_kernel<T, kAct><<<static_cast<unsigned>(grid), block, 0, s>>>(a);
+    launch_pdl(batch_norm_vec_kernel<T, kAct>, dim3(static_cast<unsigned>(grid)), dim3(block), 0, s, a);
   } else {
     int64_t grid = (a.rows * a.channels + block - 1) / block;
     const int64_t cap = static_cast<int64_t>(sm_count()) * 8;

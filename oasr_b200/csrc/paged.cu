@@ -8,6 +8,7 @@
 #include <cuda_fp8.h>
 
 #include "common.cuh"
+#include "sm100_ptx.cuh"
 
 namespace ob {
 namespace {
@@ -26,6 +27,8 @@ struct PagedWriteArgs {
 // One thread moves one 16-byte (or narrower, `VB`-byte) piece of one (b, t, h) row for K and V.
 template <int VB>
 __global__ void __launch_bounds__(256) paged_kv_write_kernel(PagedWriteArgs a) {
+  ptx::grid_dep_launch();   // no-ops unless launched with programmatic stream serialisation
+  ptx::grid_dep_wait();
   const int64_t row_bytes = a.D * a.elem_bytes;
   const int64_t pieces = row_bytes / VB;
   const int64_t total = a.B * a.T * a.Hkv * pieces;
@@ -105,6 +108,8 @@ template <bool kScatter>
 __global__ void __launch_bounds__(256) move_rows_kernel(uint8_t* __restrict__ out, const uint8_t* __restrict__ in,
                                                         const int64_t* __restrict__ index, int64_t n,
                                                         int64_t row_bytes, int64_t table_rows) {
+  ptx::grid_dep_launch();   // no-ops unless launched with programmatic stream serialisation
+  ptx::grid_dep_wait();
   const int64_t pieces = row_bytes / 16;
   const int64_t total = n * pieces;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -152,6 +157,8 @@ __device__ __forceinline__ uint2 to_e4m3x8(const Pack<T>& v, float inv) {
 
 template <typename T>
 __global__ void __launch_bounds__(256) paged_kv_write_fp8_kernel(PagedWriteFp8Args a) {
+  ptx::grid_dep_launch();   // no-ops unless launched with programmatic stream serialisation
+  ptx::grid_dep_wait();
   const int64_t pieces = a.D / 8;
   const int64_t total = a.B * a.T * a.Hkv * pieces;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -211,13 +218,13 @@ int oasr_b200_paged_kv_write(void* k_pool, void* v_pool, const void* k_new, cons
                    (stride_t * elem_bytes) % 16 == 0 && is_aligned(k_pool, 16) && is_aligned(v_pool, 16) &&
                    is_aligned(k_new, 16) && is_aligned(v_new, 16);
   if (vec) {
-    paged_kv_write_kernel<16><<<grid_for(B * T * Hkv * (row_bytes / 16)), 256, 0, s>>>(a);
+    launch_pdl(paged_kv_write_kernel<16>, dim3(grid_for(B * T * Hkv * (row_bytes / 16))), dim3(256), 0, s, a);
   } else {
     a.elem_bytes = elem_bytes;
     // piece = one element
-    if (elem_bytes == 1) paged_kv_write_kernel<1><<<grid_for(B * T * Hkv * D), 256, 0, s>>>(a);
-    else if (elem_bytes == 2) paged_kv_write_kernel<2><<<grid_for(B * T * Hkv * D), 256, 0, s>>>(a);
-    else paged_kv_write_kernel<4><<<grid_for(B * T * Hkv * D), 256, 0, s>>>(a);
+    if (elem_bytes == 1) launch_pdl(paged_kv_write_kernel<1>, dim3(grid_for(B * T * Hkv * D)), dim3(256), 0, s, a);
+    else if (elem_bytes == 2) launch_pdl(paged_kv_write_kernel<2>, dim3(grid_for(B * T * Hkv * D)), dim3(256), 0, s, a);
+    else launch_pdl(paged_kv_write_kernel<4>, dim3(grid_for(B * T * Hkv * D)), dim3(256), 0, s, a);
   }
   return check_launch("paged_kv_write launch");
 }
@@ -240,7 +247,7 @@ int oasr_b200_paged_kv_write_fp8(void* k_pool, void* v_pool, const void* k_new, 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const unsigned grid = grid_for(B * T * Hkv * (D / 8));
   return OB_DISPATCH_HALF(dtype, T_, [&]() -> int {
-    paged_kv_write_fp8_kernel<T_><<<grid, 256, 0, s>>>(a);
+    launch_pdl(paged_kv_write_fp8_kernel<T_>, dim3(grid), dim3(256), 0, s, a);
     return check_launch("paged_kv_write_fp8 launch");
   });
 }
@@ -280,8 +287,8 @@ int oasr_b200_gather_rows(void* out, const void* in, const int64_t* index, int64
              "gather_rows: row size must be a positive multiple of 16 bytes (got %lld)", (long long)row_bytes);
   OB_REQUIRE(is_aligned(out, 16) && is_aligned(in, 16), OASR_ERR_ALIGN, "gather_rows: pointers must be 16-byte aligned");
   if (n_out == 0) return OASR_OK;
-  move_rows_kernel<false><<<grid_for(n_out * (row_bytes / 16)), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<uint8_t*>(out), static_cast<const uint8_t*>(in), index, n_out, row_bytes, in_rows);
+  launch_pdl(move_rows_kernel<false>, dim3(grid_for(n_out * (row_bytes / 16))), dim3(256), 0, static_cast<cudaStream_t>(stream),
+             static_cast<uint8_t*>(out), static_cast<const uint8_t*>(in), index, n_out, row_bytes, in_rows);
   return check_launch("gather_rows launch");
 }
 
@@ -294,8 +301,8 @@ int oasr_b200_scatter_rows(void* out, const void* in, const int64_t* index, int6
              "scatter_rows: row size must be a positive multiple of 16 bytes (got %lld)", (long long)row_bytes);
   OB_REQUIRE(is_aligned(out, 16) && is_aligned(in, 16), OASR_ERR_ALIGN, "scatter_rows: pointers must be 16-byte aligned");
   if (n_in == 0) return OASR_OK;
-  move_rows_kernel<true><<<grid_for(n_in * (row_bytes / 16)), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<uint8_t*>(out), static_cast<const uint8_t*>(in), index, n_in, row_bytes, out_rows);
+  launch_pdl(move_rows_kernel<true>, dim3(grid_for(n_in * (row_bytes / 16))), dim3(256), 0, static_cast<cudaStream_t>(stream),
+             static_cast<uint8_t*>(out), static_cast<const uint8_t*>(in), index, n_in, row_bytes, out_rows);
   return check_launch("scatter_rows launch");
 }
 

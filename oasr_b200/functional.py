@@ -23,24 +23,32 @@ _DTYPE_ID = {torch.float32: DT_F32, torch.float16: DT_F16, torch.bfloat16: DT_BF
 ACTIVATION_IDS = {"relu": 0, "gelu": 1, "gelu_tanh": 1, "swish": 2, "silu": 2, "gelu_erf": 4}
 
 
-def _dt(t: torch.Tensor, allowed=(torch.float32, torch.float16, torch.bfloat16)) -> int:
-    if t.dtype not in allowed:
-        raise RuntimeError(f"unsupported dtype {t.dtype}; expected one of {allowed}")
-    return _DTYPE_ID[t.dtype]
+def _dt(t: torch.Tensor) -> int:
+    dt = _DTYPE_ID.get(t.dtype)
+    if dt is None:
+        raise RuntimeError(f"unsupported dtype {t.dtype}; expected one of {tuple(_DTYPE_ID)}")
+    return dt
 
 
 def _p(t: Optional[torch.Tensor]):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    """Device address as ctypes' ``c_void_p`` arguments take it (a plain int: no wrapper object per argument)."""
+    return None if t is None else t.data_ptr()
+
+
+_current_device = torch._C._cuda_getDevice if hasattr(torch._C, "_cuda_getDevice") else torch.cuda.current_device
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda index: torch.cuda.current_stream(index).cuda_stream)
 
 
 def _stream(t: torch.Tensor):
     """The caller's current stream on the tensor's device.  The library launches on the CURRENT device (its SM count,
     status word and tensor maps are per current device), so a tensor that lives on another GPU is refused here rather
-    than launched against the wrong context."""
-    if t.device.index is not None and t.device.index != torch.cuda.current_device():
+    than launched against the wrong context.  (The raw handle: building a ``torch.cuda.Stream`` costs more than the
+    launch of a small kernel.)"""
+    index = t.get_device()
+    if index != _current_device():
         raise RuntimeError(f"tensor on {t.device} but the current CUDA device is cuda:{torch.cuda.current_device()}: "
                            f"wrap the call in `with torch.cuda.device({t.device.index}):`")
-    return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+    return _raw_stream(index)
 
 
 def _need_cuda(*tensors) -> None:
@@ -70,13 +78,14 @@ def _is_row_dense(x: torch.Tensor) -> bool:
 
 
 def _check_rows(x: torch.Tensor, *same_layout: Optional[torch.Tensor]) -> None:
-    if not _is_row_dense(x):
+    dense = x.is_contiguous()
+    if not dense and not _is_row_dense(x):
         raise RuntimeError(
             "Tensor rows must tile memory exactly (trailing dim contiguous, no padded row stride); "
             "a row-wise kernel walks `base + row * row_len`"
         )
     for o in same_layout:
-        if o is None:
+        if o is None or (dense and o.is_contiguous() and o.shape == x.shape):
             continue
         if o.shape != x.shape or (o.stride() != x.stride() and not (o.is_contiguous() and x.is_contiguous())):
             raise RuntimeError("Tensors must have identical shape and strides")
@@ -470,8 +479,8 @@ def group_gemm(A, B, offset, out=None):
     B = B if B.is_contiguous() else B.contiguous()
     if out is None:
         out = torch.empty(L, N, device=A.device, dtype=A.dtype)
-    _lib.call("oasr_b200_group_gemm", _p(out), _p(A), _p(B), _p(offset.contiguous()), L, G, N, K, _dt(A),
-              _stream(A))
+    offset = offset.contiguous()
+    _lib.call("oasr_b200_group_gemm", _p(out), _p(A), _p(B), _p(offset), L, G, N, K, _dt(A), _stream(A))
     return out
 
 
