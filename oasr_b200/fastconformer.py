@@ -76,8 +76,8 @@ class FastConformerLayers:
                 lw[n] = (w(params[p + n + ".weight"]), w(params[p + n + ".bias"]))
             self.layers.append(lw)
         self._workspace = None
-        self._rel_window = None           # (L, 64, C): see _window_table
         self.native = True                # packed batches run through the one-call native executor
+        self._rel_window = self._window_table() if self.device.type == "cuda" and self._window_fits() else None
         self._build_native_model()
 
     def set_quant(self, quant) -> None:
@@ -140,7 +140,6 @@ class FastConformerLayers:
         M, C = rows.shape
         res = rows
         if self._windowed(g["T"]):         # no position table: the model's own windowed rows serve every batch
-            self._window_table()
             table, table_rows = None, (2 * g["T"] - 1 + 7) // 8 * 8
         else:
             table = self._position_table(g["T"])
@@ -208,14 +207,15 @@ class FastConformerLayers:
 
     def _window_table(self) -> torch.Tensor:
         """``relative_k_proj`` of the 64 distances a window can hold, every layer: row ``y`` = distance ``off - y`` with
-        ``off = left_chunks * chunk + chunk - 1``.  Depends on the model only; built once."""
-        if self._rel_window is None:
-            chunk, left_chunks = self._window_geometry()
-            off = left_chunks * chunk + chunk - 1
+        ``off = left_chunks * chunk + chunk - 1``.  Depends on the model only, so it is built with it, complete before any
+        stream can use it."""
+        chunk, left_chunks = self._window_geometry()
+        off = left_chunks * chunk + chunk - 1
+        with torch.cuda.device(self.device):
             table = self._sinusoid(off - torch.arange(64, dtype=torch.float32)).to(self.dtype).to(self.device)
-            self._rel_window = torch.stack([OF.gemm(table, lw["rel"]) for lw in self.layers]).contiguous()
-            self._native_model.rel_window = self._rel_window.data_ptr()
-        return self._rel_window
+            rows = torch.stack([OF.gemm(table, lw["rel"]) for lw in self.layers]).contiguous()
+            torch.cuda.current_stream().synchronize()
+        return rows
 
     def _sinusoid(self, positions: torch.Tensor) -> torch.Tensor:
         inv_freq = 1.0 / (10000.0 ** (torch.arange(0, self.C, 2, dtype=torch.float32) / self.C))
@@ -229,7 +229,7 @@ class FastConformerLayers:
         lw = self.layers[i]
         if g["packed"] and self._windowed(g["T"]):
             chunk, left_chunks = self._window_geometry()
-            out = fused.fmha_window_packed(self._linear(h, *lw["qkv4"]), self._window_table()[i], left_chunks * chunk + chunk - 1, g["cu"],
+            out = fused.fmha_window_packed(self._linear(h, *lw["qkv4"]), self._rel_window[i], left_chunks * chunk + chunk - 1, g["cu"],
                                            g["T"], H, chunk, left_chunks, D ** -0.5)
             return self._linear(out, *lw["o"])
         rel_table = self._position_table(g["T"])
@@ -404,7 +404,6 @@ class FastConformerLayers:
         from . import _lib
         from .functional import _p, _stream
 
-        self._window_table()
         lib = _lib.load()
         need = lib.oasr_b200_fastconformer_chunk_workspace_bytes(ctypes.byref(self._native_model), B, Tq)
         if self._workspace is None or self._workspace.numel() < need + 256:

@@ -63,12 +63,13 @@ class StreamingCache:
         self._cols = np.arange(self.max_blocks, dtype=np.int64)[None, :]
 
     def pool_pointers(self):
-        """Per-layer device pointers of the K and V pools as the host arrays the native executors take; built once."""
-        if self._pool_pointers is None:
+        """Per-layer device pointers of the K and V pools as the host arrays the native executors take; rebuilt when a
+        pool has been replaced."""
+        base = (self.k_pool.data_ptr(), self.v_pool.data_ptr())
+        if self._pool_pointers is None or self._pool_pointers[0] != base:
             step = self.k_pool.stride(0) * self.k_pool.element_size()
-            self._pool_pointers = tuple((ctypes.c_void_p * self.L)(*[pool.data_ptr() + i * step for i in range(self.L)])
-                                        for pool in (self.k_pool, self.v_pool))
-        return self._pool_pointers
+            self._pool_pointers = (base, tuple((ctypes.c_void_p * self.L)(*[b + i * step for i in range(self.L)]) for b in base))
+        return self._pool_pointers[1]
 
     # ---- host bookkeeping -------------------------------------------------------------------
     @property
