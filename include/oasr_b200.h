@@ -104,8 +104,8 @@ OASR_API int oasr_b200_selftest_bounded_wait(int64_t poll_limit, uint32_t* repor
  * (host-side counter, one per launch; no reference counterpart). */
 OASR_API unsigned long long oasr_b200_launch_count(void);
 /* Process-wide integer tunables.  "gemm_bn": 0 = heuristic tile width, or 64 /
- * 128 / 256 to force it; "gemm_pairs": 1 lets large dense GEMMs run
- * on CTA pairs (tcgen05 cta_group::2), 0 (default) keeps single-CTA tiles;
+ * 128 / 256 to force it; "gemm_pairs": dense GEMMs on CTA pairs
+ * (tcgen05 cta_group::2) where they are ahead (2, default), wherever they can run (1), never (0);
  * "dwconv_path": 0 (default) = register-streaming depthwise conv where it
  * applies, 1 = the shared-memory tiled kernel; "fmha_chunk_path": 1 (default)
  * = paged rel-pos attention with <= 16 query frames runs the warp-per-(stream,

@@ -86,7 +86,7 @@ int oasr_b200_set_tunable(const char* name, int value) {
     return OASR_OK;
   }
   if (name && std::strcmp(name, "gemm_pairs") == 0) {
-    ob::gemm::g_use_pairs = value != 0;
+    ob::gemm::g_use_pairs = value == 0 || value == 2 ? value : 1;
     return OASR_OK;
   }
   if (name && std::strcmp(name, "fmha_chunk_path") == 0) {

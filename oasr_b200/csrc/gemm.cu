@@ -898,8 +898,16 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(T* __restrict__ D, const
 // ---------------------------------------------------------------------------
 int g_force_bn = 0;  // 0 = heuristic; otherwise 64 / 128 / 256 (set through oasr_b200_set_tunable)
 int g_lsm_path = 0;   // CTC head: 0 = by size, 1 = one fused two-sweep kernel, 2 = fp32 logits GEMM + in-place row kernel
-int g_use_pairs = 0; // 1 = large dense problems run on CTA pairs (cta_group::2); 0 (default) = single-CTA tiles.
-                     // Measured on B200 (M 17.5k, K 512..2048): pairs are 5-20 % slower than single-CTA tiles here.
+int g_use_pairs = 2; // CTA pairs (cta_group::2) for dense problems: 0 never, 1 wherever they can run, 2 (default) by size.
+// Where pairs are ahead.  A pair halves the operand bytes of B, which is what bounds the main loop, but starts and drains two
+// CTAs together: a long K and a tile for every pair of SMs are needed.  B200, us single / pair, the bits are the same:
+//   28000 rows: N 4096, K 1024 166.0 / 153.6;  N 1024, K 4096 155.6 / 145.4;  N 1024, K 1024 53.2 / 51.2;  GLU 1024, K 1024 82.0 / 75.8
+//    8000 rows: N 4096, K 1024 59.4 / 57.3;    N 1024, K 4096 61.4 / 57.3;    GLU 34.8 / 32.9
+//    4000 rows: N 1024, K 1024 (64 pair tiles) 18.4 / 20.5;   16722 rows: N 2048, K 512 43.0 / 47.1, N 1536, K 512 36.9 / 38.9
+bool pairs_ahead(int64_t M, int64_t n_acc, int64_t K) {
+  const int64_t tiles = (M + 2 * BM - 1) / (2 * BM) * ((n_acc + 255) / 256);
+  return K >= 1024 && tiles >= sm_count() / 2;
+}
 
 template <typename T, int BN, int kStages, int kSched, int kEpi>
 int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const Params& p, int64_t work_items,
@@ -954,7 +962,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
   int64_t clusters = sm_count() / 2;
   if (work_items < clusters) clusters = work_items;
   if (clusters < 1) clusters = 1;
-  kern<<<static_cast<unsigned>(2 * clusters), threads_for<kSchedDense, kEpi>(), S::kDynamic, s>>>(ta, tb, td, p);
+  launch_pdl(kern, dim3(static_cast<unsigned>(2 * clusters)), dim3(threads_for<kSchedDense, kEpi>()), S::kDynamic, s, ta, tb, td, p);
   return check_launch("tcgen05 pair gemm launch");
 }
 
@@ -1119,7 +1127,8 @@ int run_typed(Problem& pr, int dtype, cudaStream_t s) {
   int bn = kEpi == kEpiLsm ? (g_force_bn ? g_force_bn : 256) : pick_bn(m_tiles_total, n_eff, pr.K);
   if (kEpi == kEpiGlu && bn < 128) bn = 128;  // half tiles of >= 64 columns
   constexpr bool kPairCapable = kSched == kSchedDense && (kEpi == kEpiStore || kEpi == kEpiGlu);
-  const bool pair = kPairCapable && g_use_pairs && g_force_bn == 0 && pr.M >= 1024 && n_eff >= 256 && pr.K >= 128;
+  const bool pair = kPairCapable && g_use_pairs && g_force_bn == 0 && pr.M >= 1024 && n_eff >= 256 && pr.K >= 128 &&
+                    (g_use_pairs == 1 || (pr.batch == 1 && bn == 256 && pairs_ahead(pr.M, n_eff, pr.K)));
   if (pair) bn = 256;
   p.num_m_tiles = static_cast<int>((pr.M + BM - 1) / BM);
   if (pair) p.num_m_tiles = static_cast<int>((pr.M + 2 * BM - 1) / (2 * BM));

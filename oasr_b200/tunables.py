@@ -3,7 +3,8 @@
 ``gemm_bn``: 0 lets the heuristic choose the GEMM tile width, 64 / 128 / 256 force it.
 ``lsm_path``: the CTC head - 0 (default) chooses by size, 1 the fused two-sweep kernel, 2 an fp32 logits GEMM followed by
 an in-place row log-softmax kernel (fp32 output only).
-``gemm_pairs``: 1 runs large dense GEMMs on CTA pairs (tcgen05 cta_group::2), 0 (default) on single-CTA tiles.
+``gemm_pairs``: dense GEMMs on CTA pairs (tcgen05 cta_group::2) where they are ahead (2, default), wherever they can run
+(1) or never (0).
 ``dwconv_path``: 2 (default) runs the depthwise conv of kernel size 9 / 15 on the rolling register-window kernel (other sizes
 up to 15 on the run-at-once register-streaming kernel), 0 all of them on the run-at-once kernel, 1 on the shared-memory tiled one.
 ``fmha_chunk_path``: 1 (default) runs paged rel-pos attention with <= 16 query frames on the warp-per-(stream, head)

@@ -290,3 +290,20 @@ def test_gemm_dup_first_equals_the_gemm_with_the_repeated_weight_block(M):
     assert got.shape == (M, 4 * d) and torch.equal(got, want) and torch.equal(got_view, want)
     with pytest.raises(Exception, match="multiples of 256"):
         fused.gemm_dup_first(A, W3[:3 * d - 8], bias4, d)
+
+
+@pytest.mark.parametrize("M,N,K", [(9473, 512, 1024), (4737, 1024, 1032), (2561, 1024, 1024), (1024, 4864, 1024), (18689, 272, 1024)])
+def test_gemm_rule_for_cta_pairs(M, N, K):
+    """Both sides of the rule's tile count (74 pair tiles on 148 SMs) and ragged rows, columns and K: whichever kernel a
+    product runs on, the bits are those of single-CTA tiles."""
+    from oasr_b200 import tunables
+
+    A, B, C = (t.cuda() for t in (_rand((M, K), torch.bfloat16, 41), _rand((N, K), torch.bfloat16, 42, K ** -0.5), _rand((N,), torch.bfloat16, 43)))
+    try:
+        tunables.set("gemm_pairs", 2)
+        by_size, by_size_glu = ob.gemm_activation(A, B, C, 2), ob.gemm_glu(A, B, C)
+        tunables.set("gemm_pairs", 0)
+        assert torch.equal(by_size, ob.gemm_activation(A, B, C, 2))
+        assert torch.equal(by_size_glu, ob.gemm_glu(A, B, C))
+    finally:
+        tunables.set("gemm_pairs", 2)
