@@ -17,9 +17,11 @@
 // distance column x - r.  All 80 scores of a row are in registers, so the softmax is one pass.
 //
 // Two forms share the arithmetic: packed segments (64 frames per block; K, V and the 64 table rows shared through shared
-// memory by its 4 warps; two blocks per SM), and paged streams (a warp per (stream, head, 16 frames); K and table rows
-// straight from memory into fragments, the chunk's own keys from the projection, and the warp that reads them also writes
-// them to their pages, so that no separate page-write launch is needed).
+// memory by its 4 warps; two blocks per SM), and paged streams (a block per (stream, head, 16 frames); the chunk's own keys
+// from the projection, and the block that reads them also writes them to their pages, so that no separate page-write launch
+// is needed).  A streaming step has few items and a chain of launches behind it, so what counts there is one item's latency:
+// four warps fetch its keys, values and table rows into shared memory, share the position scores and P.V, and repeat the
+// content scores (24 streams x 8 heads: 10.1 us; 36.4 us as a warp per item with keys straight from memory into fragments).
 #include <type_traits>
 
 #include "common.cuh"
@@ -84,18 +86,21 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 template <int D>
 struct QFrag { uint4 lo[D / 32], hi[D / 32]; };
 
-// One warp's 16 frames: `key16(n, blk)` / `rel16(n, blk)` give this lane's 16 bytes of key (distance) row 8 n + g, block blk;
-// `v_tile` = the warp's 80 value rows in shared memory (D * 2 bytes each, 16-byte chunk c of row r at c ^ (r & 7));
-// `escore` = the warp's buffer, >= 16 * kPitch floats and >= 16 rows of output; `v_ready()` waits for the value tile.
-template <typename T, int D, typename KeyFn, typename RelFn, typename VReady>
+// 16 frames by kSplit warps (this one is number `part`): `key16(n, blk)` / `rel16(n, blk)` give this lane's 16 bytes of key
+// (distance) row 8 n + g, block blk; `v_tile` = the 80 value rows in shared memory (D * 2 bytes each, 16-byte chunk c of row r
+// at c ^ (r & 7)); `escore` = the item's buffer, >= 16 * kPitch floats and >= 16 rows of output; `v_ready()` waits for the value
+// tile, and with several warps for all of them, as `sync()` does.
+template <typename T, int D, int kSplit, typename KeyFn, typename RelFn, typename VReady, typename Sync>
 __device__ __forceinline__ void warp_attention(const QFrag<D>& qu, const QFrag<D>& qv, KeyFn key16, RelFn rel16, VReady v_ready,
                                                const uint8_t* v_tile, float* escore, T* out, int64_t out_ld, int rows_live,
-                                               int j0, const int (&klo)[2], const int (&khi)[2], float scale_log2) {
+                                               int j0, const int (&klo)[2], const int (&khi)[2], float scale_log2, int part,
+                                               Sync sync) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   constexpr int kBlk = D / 32;
   // position scores of the 16 frames against the 64 distances
 #pragma unroll 4
-  for (int n = 0; n < kDist / 8; ++n) {
+  for (int nn = 0; nn < kDist / 8 / kSplit; ++nn) {
+    const int n = part * (kDist / 8 / kSplit) + nn;
     float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int b = 0; b < kBlk; ++b) {
@@ -106,7 +111,7 @@ __device__ __forceinline__ void warp_attention(const QFrag<D>& qu, const QFrag<D
     *reinterpret_cast<float2*>(escore + g * kPitch + n * 8 + 2 * t) = make_float2(c[0], c[1]);
     *reinterpret_cast<float2*>(escore + (g + 8) * kPitch + n * 8 + 2 * t) = make_float2(c[2], c[3]);
   }
-  __syncwarp();
+  sync();
   // content scores, shifted position scores, mask
   float s[kKeys / 8][4];
   float mx[2] = {-INFINITY, -INFINITY};
@@ -163,7 +168,8 @@ __device__ __forceinline__ void warp_attention(const QFrag<D>& qu, const QFrag<D
   uint8_t* obuf = reinterpret_cast<uint8_t*>(escore);
   const int vr = (lane & 7) + ((lane >> 3) & 1) * 8, vc = lane >> 4;   // ldmatrix row of this lane, second 8 columns
 #pragma unroll 2
-  for (int d = 0; d < D / 16; ++d) {
+  for (int dd = 0; dd < D / 16 / kSplit; ++dd) {
+    const int d = part * (D / 16 / kSplit) + dd;
     float o[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
     for (int k = 0; k < kKeys / 16; ++k) {
@@ -180,10 +186,10 @@ __device__ __forceinline__ void warp_attention(const QFrag<D>& qu, const QFrag<D
       *reinterpret_cast<uint32_t*>(obuf + (g + 8) * (D * 2) + ((c ^ (g & 7)) << 4) + 4 * t) = pack2<T>(o[e][2] * sum[1], o[e][3] * sum[1]);
     }
   }
-  __syncwarp();
+  sync();
   constexpr int kC = D / 8;
 #pragma unroll
-  for (int i = lane; i < kRows * kC; i += 32) {
+  for (int i = part * 32 + lane; i < kRows * kC; i += 32 * kSplit) {
     const int r = i / kC, c = i - r * kC;
     if (r < rows_live) *reinterpret_cast<uint4*>(out + r * out_ld + c * 8) = *reinterpret_cast<const uint4*>(obuf + r * (D * 2) + ((c ^ (r & 7)) << 4));
   }
@@ -260,35 +266,35 @@ __global__ void __launch_bounds__(kWarps * 32, 2) window_packed_kernel(const Par
     cp_async_wait<0>();
     __syncthreads();
   };
-  warp_attention<T, D>(qu, qv, key16, rel16, v_ready, smem + S::kV + warp * kRows * S::kRow,
-                       reinterpret_cast<float*>(smem + S::kE) + warp * kRows * kPitch,
-                       static_cast<T*>(p.out) + (row0 + i0) * C + h * D, C, rows_live, i0 - off, klo, khi, p.scale_log2);
+  warp_attention<T, D, 1>(qu, qv, key16, rel16, v_ready, smem + S::kV + warp * kRows * S::kRow,
+                          reinterpret_cast<float*>(smem + S::kE) + warp * kRows * kPitch,
+                          static_cast<T*>(p.out) + (row0 + i0) * C + h * D, C, rows_live, i0 - off, klo, khi, p.scale_log2, 0,
+                          [] { __syncwarp(); });
 }
 
 template <int D>
 struct SmemPaged {
-  static constexpr int kRow = D * 2, kWarpBytes = kKeys * kRow + kRows * kPitch * 4, kBytes = kWarps * kWarpBytes;
+  static constexpr int kRow = D * 2, kK = 0, kV = kK + kKeys * kRow, kR = kV + kKeys * kRow, kE = kR + kDist * kRow,
+                       kBytes = kE + kRows * kPitch * 4;
 };
 
-// Paged streams: a warp per (stream, block of 16 new frames, head), heads of a stream side by side.
+// Paged streams: a block per (stream, block of 16 new frames, head), heads of a stream side by side.
 template <typename T, int D>
-__global__ void __launch_bounds__(kWarps * 32, 2) window_paged_kernel(const Params p) {
+__global__ void __launch_bounds__(kWarps * 32, 3) window_paged_kernel(const Params p) {
   using S = SmemPaged<D>;
   ptx::grid_dep_launch();
   ptx::grid_dep_wait();
   extern __shared__ __align__(128) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int qblocks = (p.Tq + kRows - 1) / kRows;
-  const int item = blockIdx.x * kWarps + warp;
-  if (item >= p.B * qblocks * p.H) return;
-  const int h = item % p.H, rest = item / p.H, qb = rest % qblocks, b = rest / qblocks;
+  const int item = blockIdx.x, h = item % p.H, rest = item / p.H, qb = rest % qblocks, b = rest / qblocks;
   const int64_t C = static_cast<int64_t>(p.H) * D, ld = 4 * C;
   const T* rows = static_cast<const T*>(p.qkv4) + static_cast<int64_t>(b) * p.Tq * ld + h * D;   // new frame t: row t
   T* kp = static_cast<T*>(p.k_pool);
   T* vp = static_cast<T*>(p.v_pool);
   const int cached = p.cached[b], total = cached + p.Tq, f0 = p.pos_start[b];   // key j of the stream is frame f0 + j
   const int off = p.left_chunks * p.chunk + p.chunk - 1;
-  const int i0 = qb * kRows, rows_live = p.Tq - i0, j0 = cached + i0 - off;     // first key of the warp (may be negative)
+  const int i0 = qb * kRows, rows_live = p.Tq - i0, j0 = cached + i0 - off;     // first key of the block (may be negative)
   const int32_t* table = p.block_table + static_cast<int64_t>(b) * p.blocks_per_seq;
   // element offset of key j in the pools, or -1
   auto page_at = [&](int j) -> int64_t {
@@ -298,36 +304,52 @@ __global__ void __launch_bounds__(kWarps * 32, 2) window_paged_kernel(const Para
     if (page < 0 || page >= p.num_blocks) return -1;
     return ((static_cast<int64_t>(page) * p.block_size + (j - col * p.block_size)) * p.H + h) * D;
   };
-  uint8_t* v_tile = smem + warp * S::kWarpBytes;
-  constexpr int kC = D / 8;
-  // values: the cached ones from their pages, the chunk's own from the projection
-  for (int i = lane; i < kKeys * kC; i += 32) {
-    const int r = i / kC, c = i - r * kC, j = j0 + r;
-    const T* src = rows;
-    bool live = false;
+  constexpr int kC = D / 8, kStep = kWarps * 32 / kC;      // 16-byte chunks of a row, rows of one pass of the block
+  const int lr = threadIdx.x / kC, lc = threadIdx.x - lr * kC;
+  // keys, then values: the cached ones from their pages, the chunk's own from the projection
+  auto source = [&](int r, const T* pool, int64_t part, bool& live) -> const T* {
+    const int j = j0 + r;
+    live = false;
     if (j >= cached && j < total) {
-      src = rows + (j - cached) * ld + 3 * C + c * 8;
       live = true;
-    } else if (j >= 0 && j < cached) {
-      const int64_t at = page_at(j);
-      if (at >= 0) { src = vp + at + c * 8; live = true; }
+      return rows + (j - cached) * ld + part * C + lc * 8;
     }
-    cp_async16(v_tile + r * S::kRow + ((c ^ (r & 7)) << 4), src, live);
+    if (j >= 0 && j < cached) {
+      const int64_t at = page_at(j);
+      if (at >= 0) {
+        live = true;
+        return pool + at + lc * 8;
+      }
+    }
+    return rows;
+  };
+  for (int r = lr; r < kKeys; r += kStep) {
+    bool live;
+    const T* src = source(r, kp, 2, live);
+    cp_async16(smem + S::kK + r * S::kRow + ((lc ^ ((r & 1) << 2)) << 4), src, live);
+  }
+  for (int r = lr; r < kDist; r += kStep) {
+    int64_t at = static_cast<int64_t>(p.center) - off + r;
+    at = at < 0 ? 0 : (at >= p.table_rows ? p.table_rows - 1 : at);
+    cp_async16(smem + S::kR + r * S::kRow + ((lc ^ ((r & 1) << 2)) << 4), static_cast<const T*>(p.rel_k) + at * C + h * D + lc * 8, true);
+  }
+  cp_async_commit();
+  for (int r = lr; r < kKeys; r += kStep) {
+    bool live;
+    const T* src = source(r, vp, 3, live);
+    cp_async16(smem + S::kV + r * S::kRow + ((lc ^ (r & 7)) << 4), src, live);
   }
   cp_async_commit();
   QFrag<D> qu, qv;
   load_q<T, D>(qu, rows + i0 * ld, ld, rows_live);
   load_q<T, D>(qv, rows + i0 * ld + C, ld, rows_live);
-  // this warp's new keys and values to their pages (the index rule of paged_kv_write: positions outside the table are dropped)
-  for (int i = lane; i < kRows * kC; i += 32) {
-    const int r = i / kC, c = i - r * kC;
-    if (r < rows_live) {
-      const int64_t at = page_at(cached + i0 + r);
-      if (at >= 0) {
-        const T* src = rows + (i0 + r) * ld + 2 * C + c * 8;
-        *reinterpret_cast<uint4*>(kp + at + c * 8) = *reinterpret_cast<const uint4*>(src);
-        *reinterpret_cast<uint4*>(vp + at + c * 8) = *reinterpret_cast<const uint4*>(src + C);
-      }
+  // the new keys and values to their pages (the index rule of paged_kv_write: positions outside the table are dropped)
+  for (int r = lr; r < kRows && r < rows_live; r += kStep) {
+    const int64_t at = page_at(cached + i0 + r);
+    if (at >= 0) {
+      const T* src = rows + (i0 + r) * ld + 2 * C + lc * 8;
+      *reinterpret_cast<uint4*>(kp + at + lc * 8) = *reinterpret_cast<const uint4*>(src);
+      *reinterpret_cast<uint4*>(vp + at + lc * 8) = *reinterpret_cast<const uint4*>(src + C);
     }
   }
   int klo[2], khi[2];
@@ -337,28 +359,17 @@ __global__ void __launch_bounds__(kWarps * 32, 2) window_paged_kernel(const Para
     klo[hh] = max(0, (qc - p.left_chunks) * p.chunk - f0);
     khi[hh] = r < p.Tq ? min((qc + 1) * p.chunk - f0, total) : 0;
   }
-  auto key16 = [&](int n, int blk) {
-    const int j = j0 + n * 8 + g;
-    const T* src = nullptr;
-    if (j >= cached && j < total) src = rows + (j - cached) * ld + 2 * C;
-    else if (j >= 0 && j < cached) {
-      const int64_t at = page_at(j);
-      if (at >= 0) src = kp + at;
-    }
-    return src ? *reinterpret_cast<const uint4*>(src + blk * 32 + t * 8) : make_uint4(0, 0, 0, 0);
-  };
-  auto rel16 = [&](int n, int blk) {
-    int64_t at = static_cast<int64_t>(p.center) - off + n * 8 + g;
-    at = at < 0 ? 0 : (at >= p.table_rows ? p.table_rows - 1 : at);
-    return __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.rel_k) + at * C + h * D + blk * 32 + t * 8));
-  };
+  cp_async_wait<1>();
+  __syncthreads();
+  auto key16 = [&](int n, int blk) { return *reinterpret_cast<const uint4*>(smem + S::kK + (n * 8 + g) * S::kRow + (((blk * 4 + t) ^ ((g & 1) << 2)) << 4)); };
+  auto rel16 = [&](int n, int blk) { return *reinterpret_cast<const uint4*>(smem + S::kR + (n * 8 + g) * S::kRow + (((blk * 4 + t) ^ ((g & 1) << 2)) << 4)); };
   auto v_ready = [&]() {
     cp_async_wait<0>();
-    __syncwarp();
+    __syncthreads();
   };
-  warp_attention<T, D>(qu, qv, key16, rel16, v_ready, v_tile, reinterpret_cast<float*>(v_tile + kKeys * S::kRow),
-                       static_cast<T*>(p.out) + (static_cast<int64_t>(b) * p.Tq + i0) * C + h * D, C, rows_live, j0, klo, khi,
-                       p.scale_log2);
+  warp_attention<T, D, kWarps>(qu, qv, key16, rel16, v_ready, smem + S::kV, reinterpret_cast<float*>(smem + S::kE),
+                               static_cast<T*>(p.out) + (static_cast<int64_t>(b) * p.Tq + i0) * C + h * D, C, rows_live, j0, klo, khi,
+                               p.scale_log2, warp, [] { __syncthreads(); });
 }
 
 template <typename K>
@@ -427,8 +438,7 @@ int oasr_b200_fmha_window_paged(void* out, const void* qkv4, void* k_pool, void*
   p.chunk = (int)chunk; p.left_chunks = (int)left_chunks; p.scale_log2 = static_cast<float>(scale * 1.4426950408889634);
   p.k_pool = k_pool; p.v_pool = v_pool; p.block_table = block_table; p.cached = cached; p.pos_start = pos_start;
   p.B = (int)B; p.Tq = (int)Tq; p.blocks_per_seq = (int)blocks_per_seq; p.block_size = (int)block_size; p.num_blocks = (int)num_blocks;
-  const int64_t items = B * ((Tq + kRows - 1) / kRows) * heads;
-  const dim3 grid(static_cast<unsigned>((items + kWarps - 1) / kWarps));
+  const dim3 grid(static_cast<unsigned>(B * ((Tq + kRows - 1) / kRows) * heads));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   return OB_DISPATCH_HALF(dtype, T, [&]() -> int {
     if (head_dim == 128) return launch(window_paged_kernel<T, 128>, SmemPaged<128>::kBytes, grid, p, s, "fmha_window_paged launch");
