@@ -84,18 +84,29 @@ __global__ void __launch_bounds__(128) norm_warp_rows_kernel(NormArgs a) {
   TOut* out = static_cast<TOut*>(a.out) + row * H;
   TOut* res_out = (kAdd && a.res_out) ? static_cast<TOut*>(a.res_out) + row * H : nullptr;
 
-  float x[kChunks][kGran];
+  // with a residual: the whole row is requested before the first store, behind which a load would wait (res_out may be in)
+  constexpr bool kAhead = kAdd && kChunks <= 4;
+  float x[kChunks][kGran], r[kAhead ? kChunks : 1][kGran];
+  if constexpr (kAhead) {
+#pragma unroll
+    for (int c = 0; c < kChunks; ++c) {
+      const int e = (c * 32 + lane) * kGran;
+      if (e < H) {
+        load8(in + e, x[c]);
+        load8(res + e, r[c]);
+      }
+    }
+  }
   float sum = 0.f;
 #pragma unroll
   for (int c = 0; c < kChunks; ++c) {
     const int e = (c * 32 + lane) * kGran;
     if (e < H) {
-      load8(in + e, x[c]);
+      if constexpr (!kAhead) load8(in + e, x[c]);
       if constexpr (kAdd) {
-        float r[kGran];
-        load8(res + e, r);
+        if constexpr (!kAhead) load8(res + e, r[0]);
 #pragma unroll
-        for (int i = 0; i < kGran; ++i) x[c][i] = fmaf(a.alpha, x[c][i], r[i]);
+        for (int i = 0; i < kGran; ++i) x[c][i] = fmaf(a.alpha, x[c][i], r[kAhead ? c : 0][i]);
         if (res_out) store8(res_out + e, x[c]);
       }
 #pragma unroll
@@ -486,27 +497,27 @@ __global__ void __launch_bounds__(128) add_norm_f32_kernel(AddNormArgs a) {
   const int H = a.hidden;
   const float* res = a.res_in ? a.res_in + row * H : nullptr;
   const T* y = a.y ? static_cast<const T*>(a.y) + row * H : nullptr;
+  // The whole row is requested before the first store: res_out may be res_in, so a load behind a store waits for the loads
+  // before it, one trip to memory per chunk (384 rows of 1024: 4.8 -> 4.2 us; 592 rows of 512: 3.1 -> 2.9 us).
   float x[kChunks][kGran];
+  Pack<T> yy[kChunks];
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c) {
+    const int e = (c * 32 + lane) * kGran;
+#pragma unroll
+    for (int i = 0; i < kGran; ++i) x[c][i] = 0.f;
+    if (e < H && res) load8(res + e, x[c]);
+    if (e < H && y) yy[c] = ld128(y + e);
+  }
 #pragma unroll
   for (int c = 0; c < kChunks; ++c) {
     const int e = (c * 32 + lane) * kGran;
     if (e < H) {
-      if (res) {
-        load8(res + e, x[c]);
-      } else {
-#pragma unroll
-        for (int i = 0; i < kGran; ++i) x[c][i] = 0.f;
-      }
       if (y) {
-        float yy[kGran];
-        load8(y + e, yy);
 #pragma unroll
-        for (int i = 0; i < kGran; ++i) x[c][i] = fmaf(a.alpha, yy[i], x[c][i]);
+        for (int i = 0; i < kGran; ++i) x[c][i] = fmaf(a.alpha, Elem<T>::to_f(yy[c].v[i]), x[c][i]);
       }
       if (kMode != 2 && a.res_out) store8(a.res_out + row * H + e, x[c]);
-    } else {
-#pragma unroll
-      for (int i = 0; i < kGran; ++i) x[c][i] = 0.f;
     }
   }
   const bool split = a.split_out != 0;
