@@ -293,6 +293,21 @@ OASR_API int oasr_b200_depthwise_conv1d_packed_causal(void* out, const void* in,
                                                       const void* bias /*nullable*/, const int32_t* cu_seqlens,
                                                       int64_t num_segs, int64_t max_seg_len, int64_t channels,
                                                       int64_t kernel_size, int activation, int dtype, void* stream);
+/* Causal depthwise conv + LayerNorm over the channels + SiLU in one kernel (the middle of the FastConformer conv module,
+ * oasr/models/nemotron/encoder.py:183-214): weight (kernel_size, channels), norm_w / norm_b (channels); the conv
+ * values are rounded to 16 bits as by the conv alone.  _packed: segments cu_seqlens of `total` rows, zeros before each; _stream:
+ * B segments of T rows, each continuing from state[slot_ids[b]] (slots, kernel_size - 1, channels), which is set to its last
+ * rows (a slot outside the buffer: zeros, nothing kept).  16-bit types; _supported: 9 taps, channels a multiple of 128 up to
+ * 1024. */
+OASR_API int oasr_b200_dwconv_norm_swish_supported(int64_t channels, int64_t kernel_size);
+OASR_API int oasr_b200_dwconv_norm_swish_packed(void* out, const void* in, const void* weight, const void* bias /*nullable*/,
+                                                const void* norm_w, const void* norm_b /*nullable*/, const int32_t* cu_seqlens,
+                                                int64_t num_segs, int64_t max_seg, int64_t total, int64_t channels,
+                                                int64_t kernel_size, double eps, int dtype, void* stream);
+OASR_API int oasr_b200_dwconv_norm_swish_stream(void* out, const void* in, const void* weight, const void* bias /*nullable*/,
+                                                const void* norm_w, const void* norm_b /*nullable*/, void* state, int64_t num_slots,
+                                                const int64_t* slot_ids, int64_t B, int64_t T, int64_t channels, int64_t kernel_size,
+                                                double eps, int dtype, void* stream);
 /* oasr_b200_depthwise_conv1d with a per-channel affine (fp32 post_scale /
  * post_shift, a folded inference BatchNorm) applied after the bias and before
  * the activation: depthwise_conv followed by BatchNormActivation of the conv

@@ -89,6 +89,9 @@ _SIGNATURES = {
     "oasr_b200_fmha_window_supported": [I, I, I],
     "oasr_b200_fmha_window_packed": [P, P, P, I, I, P, I, I, I, I, I, I, I, c_double, c_int, P],
     "oasr_b200_fmha_window_paged": [P, P, P, P, P, I, I, P, P, P, I, I, I, I, I, I, I, I, I, c_double, c_int, P],
+    "oasr_b200_dwconv_norm_swish_supported": [I, I],
+    "oasr_b200_dwconv_norm_swish_packed": [P, P, P, P, P, P, P, I, I, I, I, I, c_double, c_int, P],
+    "oasr_b200_dwconv_norm_swish_stream": [P, P, P, P, P, P, P, I, P, I, I, I, I, c_double, c_int, P],
     "oasr_b200_bmm_strided": [P, P, P, I, I, I, I, I, I, I, I, c_int, P],
     "oasr_b200_fmha_bthd": [P, P, P, P, P, P, P, P, I, I, I, P, P, P, I, I, I, I, I, I, I, I, I, c_double, c_int, c_int, P],
     "oasr_b200_fmha_varlen": [P, P, P, P, P, P, c_int, P, P, I, I, I, I, I, I, I, c_double, c_int, P],

@@ -1,6 +1,7 @@
 // Native executor of the packed FastConformer / Nemotron layer stack: one host call enqueues the whole fixed
 // kernel sequence of NemotronEncoder.forward's layer loop (oasr/models/nemotron/encoder.py:217-267, 542-583) on the
-// caller's stream -- per layer 17 launches (21 with an 8-bit kind: the add + norm kernels also write the quantised
+// caller's stream -- per layer 14 launches, 17 where segments of up to 128 frames keep the
+// general attention (4 more with an 8-bit kind: the add + norm kernels also write the quantised
 // row for the Linear behind them) of this library's own C-ABI kernels: macaron FFN, Transformer-XL
 // relative-position attention (q projected once per global bias, position scores as one batched GEMM over heads,
 // one kernel for the relative shift + scale + chunked-limited window, head_dim 128 attention with that bias),
@@ -154,6 +155,7 @@ int oasr_b200_fastconformer_layers_packed(const oasr_b200_fastconformer_model* m
   const double scale = 1.0 / std::sqrt(static_cast<double>(D));
   const int64_t chunk = m.right_context + 1;
   const int64_t left_chunks = fc_left_chunks(m, max_seg);
+  const bool conv_norm = oasr_b200_dwconv_norm_swish_supported(C, m.kernel) != 0 && num_segs < 65536;
   const oasr_b200_fastconformer_layer* ly = m.layers;
   const double eps = m.eps;
 
@@ -222,10 +224,15 @@ int oasr_b200_fastconformer_layers_packed(const oasr_b200_fastconformer_model* m
     FC_ADD_NORM(res, w.y, 1.0, 0, l.norm_conv_w, l.norm_conv_b, nullptr, nullptr);
     // conv module: pointwise + GLU, causal depthwise conv per segment, LayerNorm + SiLU, pointwise
     FC_LINEAR_H(w.g, l.pw1_w, l.pw1_b, l, 4, C, C, OASR_ACT_NONE, 1);
-    FC_STEP(oasr_b200_depthwise_conv1d_packed_causal(w.cv, w.g, l.dw_w, l.dw_b, cu_seqlens, num_segs, max_seg, C, m.kernel, -1, dt,
-                                                     stream));
-    FC_STEP(oasr_b200_layer_norm_activation(w.g, w.cv, l.conv_norm_w, l.conv_norm_b, M, C, 1e-5, OASR_ACT_SWISH, dt, stream));
-    FC_LINEAR(w.y, w.g, l.pw2_w, l.pw2_b, l, 5, C, C, OASR_ACT_NONE, 0);
+    if (conv_norm) {
+      FC_STEP(oasr_b200_dwconv_norm_swish_packed(w.cv, w.g, l.dw_w, l.dw_b, l.conv_norm_w, l.conv_norm_b, cu_seqlens, num_segs, max_seg, M, C,
+                                                 m.kernel, 1e-5, dt, stream));
+    } else {
+      FC_STEP(oasr_b200_depthwise_conv1d_packed_causal(w.att, w.g, l.dw_w, l.dw_b, cu_seqlens, num_segs, max_seg, C, m.kernel, -1, dt,
+                                                       stream));
+      FC_STEP(oasr_b200_layer_norm_activation(w.cv, w.att, l.conv_norm_w, l.conv_norm_b, M, C, 1e-5, OASR_ACT_SWISH, dt, stream));
+    }
+    FC_LINEAR(w.y, w.cv, l.pw2_w, l.pw2_b, l, 5, C, C, OASR_ACT_NONE, 0);
     FC_ADD_NORM(res, w.y, 1.0, 0, l.norm_ff2_w, l.norm_ff2_b, nullptr, nullptr);
     // second feed-forward, norm_out, then the next layer's first pre-norm in the same kernel
     FC_LINEAR_H(w.a_ffn, l.ff2_w1, l.ff2_b1, l, 6, F, C, OASR_ACT_SWISH, 0);
@@ -272,6 +279,7 @@ int oasr_b200_fastconformer_chunk_paged(const oasr_b200_fastconformer_model* mod
   const int dt = m.dtype;
   const double scale = 1.0 / std::sqrt(static_cast<double>(D)), eps = m.eps;
   const oasr_b200_fastconformer_layer* ly = m.layers;
+  const bool conv_norm = oasr_b200_dwconv_norm_swish_supported(C, m.kernel) != 0 && B < 65536;
   const Chain inner{1, 0};       // weights settled: see gemm_small.cuh
   // last Linear of a sub-layer + residual + norm (mode 2: norm_out and the next pre-norm); few rows: the Linear adds into
   // the fp32 stream itself
@@ -304,11 +312,16 @@ int oasr_b200_fastconformer_chunk_paged(const oasr_b200_fastconformer_model* mod
     FC_CHUNK_LINEAR_ADDNORM(w.att, l.o_w, l.o_b, C, 1.0, 0, w.res, l.norm_conv_w, l.norm_conv_b, nullptr, nullptr);
     // conv module continuing from the stream's post-GLU tail
     FC_STEP(gemm_glu_op(w.g, w.h, l.pw1_w, l.pw1_b, M, C, C, dt, stream, inner));
-    FC_STEP(oasr_b200_conv_state_concat(w.xcat, static_cast<uint8_t*>(cnn_state) + i * num_slots * SL * C * 2, num_slots, slot_ids, w.g, B,
-                                        SL, Tq, C, dt, stream));
-    FC_STEP(oasr_b200_depthwise_conv1d(w.cv, w.xcat, l.dw_w, l.dw_b, B, SL + Tq, C, m.kernel, 0, 0, nullptr, 0, 0, OASR_ACT_NONE, dt, stream));
-    FC_STEP(oasr_b200_layer_norm_activation(w.g, w.cv, l.conv_norm_w, l.conv_norm_b, M, C, 1e-5, OASR_ACT_SWISH, dt, stream));
-    FC_CHUNK_LINEAR_ADDNORM(w.g, l.pw2_w, l.pw2_b, C, 1.0, 0, w.res, l.norm_ff2_w, l.norm_ff2_b, nullptr, nullptr);
+    uint8_t* state = static_cast<uint8_t*>(cnn_state) + i * num_slots * SL * C * 2;
+    if (conv_norm) {
+      FC_STEP(oasr_b200_dwconv_norm_swish_stream(w.cv, w.g, l.dw_w, l.dw_b, l.conv_norm_w, l.conv_norm_b, state, num_slots, slot_ids, B, Tq, C,
+                                                 m.kernel, 1e-5, dt, stream));
+    } else {
+      FC_STEP(oasr_b200_conv_state_concat(w.xcat, state, num_slots, slot_ids, w.g, B, SL, Tq, C, dt, stream));
+      FC_STEP(oasr_b200_depthwise_conv1d(w.att, w.xcat, l.dw_w, l.dw_b, B, SL + Tq, C, m.kernel, 0, 0, nullptr, 0, 0, OASR_ACT_NONE, dt, stream));
+      FC_STEP(oasr_b200_layer_norm_activation(w.cv, w.att, l.conv_norm_w, l.conv_norm_b, M, C, 1e-5, OASR_ACT_SWISH, dt, stream));
+    }
+    FC_CHUNK_LINEAR_ADDNORM(w.cv, l.pw2_w, l.pw2_b, C, 1.0, 0, w.res, l.norm_ff2_w, l.norm_ff2_b, nullptr, nullptr);
     FC_STEP(gemm_op(w.a_ffn, w.h, l.ff2_w1, l.ff2_b1, M, F, C, OASR_ACT_SWISH, dt, stream, inner));
     if (i + 1 < L) {
       FC_CHUNK_LINEAR_ADDNORM(w.a_ffn, l.ff2_w2, l.ff2_b2, F, 0.5, 2, w.res, l.norm_out_w, l.norm_out_b, ly[i + 1].norm_ff1_w, ly[i + 1].norm_ff1_b);

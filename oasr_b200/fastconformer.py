@@ -260,6 +260,8 @@ class FastConformerLayers:
 
     def _conv(self, lw, h: torch.Tensor, g) -> torch.Tensor:
         x = self._linear(h, *lw["pw1"], glu=True)                                     # pointwise_conv1 + GLU
+        if g["packed"] and fused.dwconv_norm_swish_supported(self.C, self.K):
+            return self._linear(fused.dwconv_norm_swish_packed(x, *lw["dw"], *lw["conv_norm"], g["cu"], g["T"]), *lw["pw2"])
         if g["packed"]:
             x = fused.depthwise_conv1d_packed_causal(x, lw["dw"][0], lw["dw"][1], g["cu"], g["T"])
         else:
@@ -397,7 +399,7 @@ class FastConformerLayers:
         return out.view(B, Tq, C)
 
     def _chunk_native(self, rows: torch.Tensor, B: int, Tq: int, cache, table, cached, pos_start, slot_ids) -> torch.Tensor:
-        """The streaming step in ONE call into the native executor (oasr_b200_fastconformer_chunk_paged): 18 launches per
+        """The streaming step in ONE call into the native executor (oasr_b200_fastconformer_chunk_paged): 14 launches per
         layer where the composition below makes 24 from Python."""
         import ctypes
 

@@ -123,6 +123,36 @@ def depthwise_conv1d_packed_causal(x: torch.Tensor, weight: torch.Tensor, bias: 
     return out
 
 
+def dwconv_norm_swish_supported(channels: int, kernel_size: int) -> bool:
+    """Does a conv module's depthwise conv + LayerNorm + SiLU run as one kernel (csrc/dwconv_norm.cu)?"""
+    return bool(_lib.load().oasr_b200_dwconv_norm_swish_supported(channels, kernel_size))
+
+
+def dwconv_norm_swish_packed(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], norm_w: torch.Tensor,
+                             norm_b: Optional[torch.Tensor], cu_seqlens: torch.Tensor, max_seg_len: int, eps: float = 1e-5) -> torch.Tensor:
+    """``silu(layer_norm(causal depthwise conv(x)))`` over packed ``(total, C)`` rows, ``weight (K, C)``, in one kernel."""
+    _need_cuda(x, weight, bias, norm_w, norm_b, cu_seqlens)
+    x = x.contiguous()
+    out = torch.empty_like(x)
+    _lib.call("oasr_b200_dwconv_norm_swish_packed", _p(out), _p(x), _p(weight), _p(bias), _p(norm_w), _p(norm_b), _p(cu_seqlens),
+              cu_seqlens.numel() - 1, int(max_seg_len), x.size(0), x.size(1), weight.size(0), float(eps), _DTYPE_ID[x.dtype], _stream(x))
+    return out
+
+
+def dwconv_norm_swish_stream(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], norm_w: torch.Tensor,
+                             norm_b: Optional[torch.Tensor], state: torch.Tensor, slot_ids: torch.Tensor, eps: float = 1e-5) -> torch.Tensor:
+    """The same for streams: ``x (B, T, C)`` continues from ``state[slot] (K - 1, C)``, which is set to the stream's last rows."""
+    _need_cuda(x, weight, bias, norm_w, norm_b, state, slot_ids)
+    x = x.contiguous()
+    if not state.is_contiguous() or state.dtype != x.dtype or state.shape[1:] != (weight.size(0) - 1, x.size(2)):
+        raise ValueError("state must be contiguous (slots, K - 1, C) of the rows' type")
+    B, T, C = x.shape
+    out = torch.empty_like(x)
+    _lib.call("oasr_b200_dwconv_norm_swish_stream", _p(out), _p(x), _p(weight), _p(bias), _p(norm_w), _p(norm_b), _p(state), state.size(0),
+              _p(slot_ids), B, T, C, weight.size(0), float(eps), _DTYPE_ID[x.dtype], _stream(x))
+    return out
+
+
 def fmha_relpos_plan(cu_seqlens: torch.Tensor, heads: int, total: int) -> torch.Tensor:
     """Work list for :func:`fmha_varlen_relpos` (``plan=``): the (segment, head, query tile) items of a packed batch,
     longest segments first, built on the device from ``cu_seqlens``; at most 1024 segments.  Build once per batch."""

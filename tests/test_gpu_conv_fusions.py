@@ -1,0 +1,64 @@
+"""GPU: the FastConformer's fused conv steps against their separate operators and fp64."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+from oasr_b200 import fused
+
+pytestmark = pytest.mark.gpu
+
+# relative error of a rounding to 16 bits (8 and 11 significant bits)
+TOL = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}
+
+
+def _conv_norm(x, w, b, nw, nb, dtype, eps=1e-5):
+    """fp64: rows (8 + T, C) whose first 8 are the history -> (T, C), and what the conv's rounding may add to the error."""
+    x, w, b, nw, nb = (t.double().cpu() for t in (x, w, b, nw, nb))
+    y = F.conv1d(x.t()[None], w.t()[:, None], b, groups=x.size(1))[0].t()
+    # what the rounding of a conv value (TOL, relative) can move its output by: SiLU's slope is at most 1.1
+    slack = 1.1 * TOL[dtype] * y.abs() / (y.var(1, unbiased=False, keepdim=True) + eps).sqrt() * nw.abs()
+    return F.silu(F.layer_norm(y, (x.size(1),), nw, nb, eps)), slack
+
+
+def _params(C, dtype, seed):
+    g = torch.Generator().manual_seed(seed)
+    r = lambda *s: torch.randn(*s, generator=g)
+    return [t.to(dtype).cuda() for t in (r(9, C) * 0.3, r(C) * 0.1, 1 + 0.1 * r(C), 0.1 * r(C))], g
+
+
+def _check(got, want, dtype):
+    # beside the two roundings: what those of the other channels move the mean and the variance by (a tenth of the conv's own
+    # rounding and 0.05 of a unit), and fp32 sums
+    want, slack = want
+    err = (got.double().cpu() - want).abs()
+    assert bool((err <= TOL[dtype] * (want.abs() + 0.05) + 1.1 * slack).all()), err.max().item()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("C,lens", [(1024, [1, 7, 8, 9, 31, 32, 33, 100]), (128, [40, 3]), (384, [17]), (512, [150] * 70), (1024, [40] * 150)])
+def test_packed_depthwise_conv_norm_swish(dtype, C, lens):
+    (w, b, nw, nb), g = _params(C, dtype, C)
+    x = torch.randn(sum(lens), C, generator=g).to(dtype).cuda()
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32).cuda()
+    got = fused.dwconv_norm_swish_packed(x, w, b, nw, nb, cu, max(lens))
+    at = 0
+    for n in lens[:8]:
+        _check(got[at:at + n], _conv_norm(torch.cat([x.new_zeros(8, C), x[at:at + n]]), w, b, nw, nb, dtype), dtype)
+        at += n
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T", [1, 4, 8, 9, 16, 17])
+def test_streaming_depthwise_conv_norm_swish(dtype, T):
+    C, slots = 256, [5, 0, 3, 99]                     # 99: outside the buffer, an empty left context that is not kept
+    (w, b, nw, nb), g = _params(C, dtype, T)
+    state = torch.randn(6, 8, C, generator=g).to(dtype).cuda()
+    x = torch.randn(len(slots), T, C, generator=g).to(dtype).cuda()
+    before = state.clone()
+    got = fused.dwconv_norm_swish_stream(x, w, b, nw, nb, state, torch.tensor(slots, dtype=torch.int64).cuda())
+    for i, slot in enumerate(slots):
+        rows = torch.cat([before[slot] if slot < 6 else x.new_zeros(8, C), x[i]])
+        _check(got[i], _conv_norm(rows, w, b, nw, nb, dtype), dtype)
+        if slot < 6:
+            before[slot] = rows[-8:]
+    assert torch.equal(state, before)
