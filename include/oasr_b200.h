@@ -308,6 +308,14 @@ OASR_API int oasr_b200_dwconv_norm_swish_stream(void* out, const void* in, const
                                                 const void* norm_w, const void* norm_b /*nullable*/, void* state, int64_t num_slots,
                                                 const int64_t* slot_ids, int64_t B, int64_t T, int64_t channels, int64_t kernel_size,
                                                 double eps, int dtype, void* stream);
+/* The FastConformer subsampling stem (oasr_b200_subsample_conv1, 3x3 / stride 2, of the features padded (2, 1) on both axes)
+ * and the depthwise conv behind it (oasr_b200_depthwise_conv2d_k3s2, same padding) in one kernel, with the same bits:
+ * in (B, T, F) fp32 unpadded, out (B, To, Fo, C) 16-bit with To = (T / 2 + 1) / 2 + 1; mid_len / out_len (nullable) the valid
+ * frames behind each conv.  _supported: channels / 4 divides 256 and the block's features fit shared memory. */
+OASR_API int oasr_b200_subsample_stem_dw_supported(int64_t F, int64_t C);
+OASR_API int oasr_b200_subsample_stem_dw(void* out, const float* in, const float* stem_w, const float* stem_b, const void* dw_w,
+                                         const void* dw_b /*nullable*/, const int32_t* mid_len, const int32_t* out_len, int64_t B,
+                                         int64_t T, int64_t F, int64_t C, int dtype, void* stream);
 /* oasr_b200_depthwise_conv1d with a per-channel affine (fp32 post_scale /
  * post_shift, a folded inference BatchNorm) applied after the bias and before
  * the activation: depthwise_conv followed by BatchNormActivation of the conv

@@ -92,6 +92,8 @@ _SIGNATURES = {
     "oasr_b200_dwconv_norm_swish_supported": [I, I],
     "oasr_b200_dwconv_norm_swish_packed": [P, P, P, P, P, P, P, I, I, I, I, I, c_double, c_int, P],
     "oasr_b200_dwconv_norm_swish_stream": [P, P, P, P, P, P, P, I, P, I, I, I, I, c_double, c_int, P],
+    "oasr_b200_subsample_stem_dw_supported": [I, I],
+    "oasr_b200_subsample_stem_dw": [P, P, P, P, P, P, P, P, I, I, I, I, c_int, P],
     "oasr_b200_bmm_strided": [P, P, P, I, I, I, I, I, I, I, I, c_int, P],
     "oasr_b200_fmha_bthd": [P, P, P, P, P, P, P, P, I, I, I, P, P, P, I, I, I, I, I, I, I, I, I, c_double, c_int, c_int, P],
     "oasr_b200_fmha_varlen": [P, P, P, P, P, P, c_int, P, P, I, I, I, I, I, I, I, c_double, c_int, P],

@@ -517,11 +517,16 @@ class FastConformerEncoder:
         # stem: one input channel, pad (2, 1) on time and frequency, 3x3 / stride 2, + bias + ReLU (fp32 in, 16-bit NHWC out)
         # (frames past a stream's length are not computed: the next stage reads them as zeros through its ``in_len``)
         lengths = nxt(lengths)
-        x = fused.subsample_conv1(torch.nn.functional.pad(feats.float(), (2, 1, 2, 1)), *self.conv_in, self.dtype,
-                                  t1_limit=dev_i32(lengths))
-        for dw_w, dw_b, pw_w, pw_b in self.sub_stages:
-            in_len, lengths = lengths, nxt(lengths)
-            x = fused.depthwise_conv2d_k3s2(x, dw_w, dw_b, 2, 1, out_len=dev_i32(lengths), in_len=dev_i32(in_len))
+        # the stem with the first depthwise conv
+        stem = self.sub_stages and feats.numel() and fused.subsample_stem_dw_supported(feats.size(2), self.Cs)
+        x = feats.float() if stem else fused.subsample_conv1(torch.nn.functional.pad(feats.float(), (2, 1, 2, 1)), *self.conv_in,
+                                                             self.dtype, t1_limit=dev_i32(lengths))
+        for i, (dw_w, dw_b, pw_w, pw_b) in enumerate(self.sub_stages):
+            in_len, lengths = dev_i32(lengths), nxt(lengths)
+            if stem and i == 0:
+                x = fused.subsample_stem_dw(x, *self.conv_in, dw_w, dw_b, in_len, dev_i32(lengths))
+            else:
+                x = fused.depthwise_conv2d_k3s2(x, dw_w, dw_b, 2, 1, out_len=dev_i32(lengths), in_len=in_len)
             _, T, Fd, C = x.shape
             x = OF.gemm_activation(x.view(B * T * Fd, C), pw_w, pw_b, 0).view(B, T, Fd, C)   # pointwise conv + ReLU
         B, T, Fd, C = x.shape

@@ -307,6 +307,28 @@ def depthwise_conv2d_k3s2(x: torch.Tensor, weight: torch.Tensor, bias: Optional[
     return out
 
 
+def subsample_stem_dw_supported(bins: int, channels: int) -> bool:
+    """Do the subsampling stem and the depthwise conv behind it run as one kernel (csrc/stem_dw.cu)?"""
+    return bool(_lib.load().oasr_b200_subsample_stem_dw_supported(bins, channels))
+
+
+def subsample_stem_dw(feats: torch.Tensor, stem_w: torch.Tensor, stem_b: torch.Tensor, dw_w: torch.Tensor, dw_b: Optional[torch.Tensor],
+                      mid_len: Optional[torch.Tensor], out_len: Optional[torch.Tensor]) -> torch.Tensor:
+    """:func:`subsample_conv1` of the features padded ``(2, 1)`` on both axes, then :func:`depthwise_conv2d_k3s2` with the same
+    padding, in one kernel and with the same bits: ``feats (B, T, F)`` fp32 unpadded, ``mid_len`` / ``out_len`` the valid frames
+    behind each."""
+    _need_cuda(feats, stem_w, stem_b, dw_w, dw_b, mid_len, out_len)
+    if feats.dtype != torch.float32 or stem_w.dtype != torch.float32 or stem_b.dtype != torch.float32:
+        raise RuntimeError("subsample_stem_dw takes fp32 features, stem weight and bias")
+    feats = feats.contiguous()
+    B, T, Fb = feats.shape
+    C = stem_w.size(0)
+    out = torch.empty(B, (T // 2 + 1) // 2 + 1, (Fb // 2 + 1) // 2 + 1, C, device=feats.device, dtype=dw_w.dtype)
+    _lib.call("oasr_b200_subsample_stem_dw", _p(out), _p(feats), _p(stem_w), _p(stem_b), _p(dw_w), _p(dw_b), _p(mid_len), _p(out_len),
+              B, T, Fb, C, _DTYPE_ID[dw_w.dtype], _stream(feats))
+    return out
+
+
 def relshift_bias_packed(bd: torch.Tensor, cu_seqlens: torch.Tensor, bias_offsets: torch.Tensor, bias_numel: int, T: int,
                          scale: float, chunk: int, left_chunks: int, floor_value: float = -1.0e4) -> torch.Tensor:
     """Packed ``relshift_bias``: ``bd (H, total, ld >= 2T-1)`` scores of packed rows -> flat block-diagonal bias, segment

@@ -62,3 +62,20 @@ def test_streaming_depthwise_conv_norm_swish(dtype, T):
         if slot < 6:
             before[slot] = rows[-8:]
     assert torch.equal(state, before)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,T,Fb,C,lens", [(1, 3, 128, 256, [3]), (3, 41, 80, 256, [41, 17, 1]), (2, 64, 7, 128, [64, 9]),
+                                           (40, 130, 128, 256, list(range(91, 131))), (2, 30, 1, 512, [30, 5])])
+def test_stem_and_depthwise_conv_in_one(dtype, B, T, Fb, C, lens):
+    assert fused.subsample_stem_dw_supported(Fb, C)
+    g = torch.Generator().manual_seed(T + C)
+    feats = torch.randn(B, T, Fb, generator=g).cuda()
+    w1, b1 = torch.randn(C, 3, 3, generator=g).cuda() * 0.5, torch.randn(C, generator=g).cuda() * 0.1
+    w2, b2 = (torch.randn(C, 3, 3, generator=g) * 0.5).to(dtype).cuda(), (torch.randn(C, generator=g) * 0.1).to(dtype).cuda()
+    mid = torch.tensor([n // 2 + 1 for n in lens], dtype=torch.int32).cuda()
+    out = mid // 2 + 1
+    x = fused.subsample_conv1(F.pad(feats, (2, 1, 2, 1)), w1, b1, dtype, t1_limit=mid)
+    want = fused.depthwise_conv2d_k3s2(x, w2, b2, 2, 1, out_len=out, in_len=mid)
+    got = fused.subsample_stem_dw(feats, w1, b1, w2, b2, mid, out)
+    assert got.shape == want.shape and torch.equal(got, want)
