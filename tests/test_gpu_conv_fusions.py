@@ -79,3 +79,25 @@ def test_stem_and_depthwise_conv_in_one(dtype, B, T, Fb, C, lens):
     want = fused.depthwise_conv2d_k3s2(x, w2, b2, 2, 1, out_len=out, in_len=mid)
     got = fused.subsample_stem_dw(feats, w1, b1, w2, b2, mid, out)
     assert got.shape == want.shape and torch.equal(got, want)
+
+
+def test_other_kernel_sizes_keep_the_separate_steps():
+    """A conv of 5 taps: packed batches native and composed agree bit for bit, streams continue their cached tail (chunks
+    against the offline pass, tolerance of the streaming tests: the two attend through different kernels in bf16)."""
+    from oasr_b200.fastconformer import FastConformerLayers
+    from oracle import fastconformer as OFC
+
+    cfg = OFC.FastConformerConfig(hidden=256, heads=2, ffn=512, layers=2, kernel=5, sliding_window=25, lookahead=3, bias=True)
+    model = FastConformerLayers(cfg.hidden, cfg.heads, cfg.ffn, cfg.layers, cfg.kernel, cfg.sliding_window, cfg.lookahead,
+                                OFC.init_params(cfg, 21))
+    assert not fused.dwconv_norm_swish_supported(cfg.hidden, cfg.kernel)
+    lengths, hidden = [64, 17, 1], torch.randn(3, 64, 256, generator=torch.Generator().manual_seed(4)).cuda()
+    native, _ = model.forward_rows(hidden, lengths)
+    model.native = False
+    composed, _ = model.forward_rows(hidden, lengths)
+    model.native = True
+    assert torch.equal(native, composed)
+    cache = model.new_streaming_cache(max_streams=3, chunk_frames=16)
+    chunks = torch.cat([model.forward_chunk(hidden[:1, 16 * c:16 * (c + 1)], [2], cache) for c in range(4)], 1)
+    d = (chunks[0] - model.forward(hidden[:1], [64])[0]).abs()
+    assert d.max().item() < 6e-2 and d.mean().item() < 6e-3
