@@ -131,9 +131,8 @@ fmha_tcgen05_kernel(const __grid_constant__ Maps maps, const Params p) {
   constexpr uint32_t kColS = 0, kColO = 256;
   constexpr float kNegInf = -INFINITY;
 
-  // no-ops unless launched with programmatic stream serialisation; cu_seqlens / seqlens below are already
+  // no-op unless launched with programmatic stream serialisation; cu_seqlens / seqlens below are already
   // global reads, so the wait comes first
-  ptx::grid_dep_launch();
   ptx::grid_dep_wait();
   // ---- which rows / keys does this CTA own ---------------------------------
   const int q0 = blockIdx.x * BQ;
@@ -227,6 +226,9 @@ fmha_tcgen05_kernel(const __grid_constant__ Maps maps, const Params p) {
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  // Only now: the 146 KB of head dimension 64 leave room for a small GEMM's block, and one that held tensor memory before
+  // this block has its 512 columns would wait for this grid while this block waited for it.
+  ptx::grid_dep_launch();
 
   if (warp == 4) {
     // =================== TMA producer + MMA issuer (whole warp, one elected lane issues: see gemm.cu) ===================

@@ -118,8 +118,7 @@ fmha_relpos64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   constexpr uint32_t kIdescPV = ptx::umma_idesc_f16(kBf16, BQ, D + 16, false, true);  // V is MN-major
   constexpr float kNegInf = -INFINITY;
 
-  ptx::grid_dep_launch();   // no-ops unless launched with programmatic stream serialisation
-  ptx::grid_dep_wait();
+  ptx::grid_dep_wait();     // no-op unless launched with programmatic stream serialisation
   if (threadIdx.x == 0) stamp(p, 0);
   if (p.trace != nullptr && threadIdx.x == 0) p.trace[64 + blockIdx.x * 4] = static_cast<unsigned long long>(clock64());
   // Persistent CTA: the items of the list (or of the natural enumeration) are dealt to the CTAs in rounds of gridDim.x,
@@ -205,6 +204,7 @@ fmha_relpos64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  ptx::grid_dep_launch();
   if (threadIdx.x == 0) stamp(p, 1);
 
   // Every barrier that completes once per key tile is indexed by the CTA's running tile count g (stage g & 1, phase

@@ -96,6 +96,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 // is still draining: everything before grid_dep_wait() (barrier set-up, TMEM allocation, descriptor
 // prefetch) overlaps that tail; after it the previous grid has completed and its writes are visible.  Without
 // the launch attribute both are no-ops.
+// A kernel that allocates tensor memory calls grid_dep_launch() only once it has its columns.  The next kernel's blocks may
+// allocate theirs before their own grid_dep_wait(), on the same SM: with the trigger first they could take the columns this
+// kernel still waits for (an allocation has no time limit) and hold them until this kernel has ended.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
