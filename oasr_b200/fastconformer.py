@@ -406,11 +406,10 @@ class FastConformerLayers:
         from . import _lib
         from .functional import _p, _stream
 
-        lib = _lib.load()
-        need = lib.oasr_b200_fastconformer_chunk_workspace_bytes(ctypes.byref(self._native_model), B, Tq)
-        if self._workspace is None or self._workspace.numel() < need + 256:
-            self._workspace = torch.empty(int(need * 1.25) + 256, dtype=torch.uint8, device=rows.device)
-        ws = self._workspace
+        # scratch of this call alone, from the allocator of the caller's stream: several streams or threads, each with a cache
+        # of its own, may be in flight at once, and beside a packed batch
+        need = _lib.load().oasr_b200_fastconformer_chunk_workspace_bytes(ctypes.byref(self._native_model), B, Tq)
+        ws = torch.empty(need + 256, dtype=torch.uint8, device=rows.device)
         off = (-ws.data_ptr()) % 256
         out = torch.empty(B * Tq, self.C, device=rows.device, dtype=torch.float32)
         kp, vp = cache.pool_pointers()

@@ -357,3 +357,34 @@ def test_native_executor_equals_the_operator_by_operator_stack():
                   ctypes.c_void_p(offs.data_ptr()), cfg.heads * 64, 1, 8, 128, ctypes.c_void_p(ws.data_ptr() + (-ws.data_ptr()) % 256),
                   2048, None)
     assert _lib.launch_count() == before
+
+
+def test_streaming_steps_and_packed_batches_run_on_streams_of_their_own():
+    """One model, live streams on two CUDA streams and packed batches on a third, enqueued without waiting for one another:
+    every result is the one of the same calls made alone."""
+    cfg = OFC.FastConformerConfig(hidden=1024, heads=8, ffn=4096, layers=4, kernel=9, sliding_window=57, lookahead=3, bias=False)
+    model = FastConformerLayers(cfg.hidden, cfg.heads, cfg.ffn, cfg.layers, cfg.kernel, cfg.sliding_window, cfg.lookahead,
+                                OFC.init_params(cfg, 3, w_std=0.02))
+    g = torch.Generator().manual_seed(5)
+    chunks = [torch.randn(6, n, 16, cfg.hidden, generator=g).cuda() for n in (24, 9)]
+    hidden, lengths = torch.randn(12, 200, cfg.hidden, generator=g).cuda(), [200, 160, 129, 7] * 3
+    caches = lambda: [model.new_streaming_cache(x.size(1)) for x in chunks]
+    step = lambda k, c, cache: model.forward_chunk(chunks[k][c], list(range(chunks[k].size(1))), cache)
+    alone = [[step(k, c, cache) for c in range(6)] for k, cache in enumerate(caches())]
+    rows_alone = model.forward_rows(hidden, lengths)[0]
+    torch.cuda.synchronize()
+    for _ in range(5):
+        fresh, streams = caches(), [torch.cuda.Stream() for _ in range(3)]
+        got, rows = [[], []], []
+        torch.cuda.synchronize()
+        for c in range(6):
+            for k in (0, 1):
+                with torch.cuda.stream(streams[k]):
+                    got[k].append(step(k, c, fresh[k]))
+            with torch.cuda.stream(streams[2]):
+                rows.append(model.forward_rows(hidden, lengths)[0])
+        torch.cuda.synchronize()
+        assert ob.device_status() == 0
+        for k in (0, 1):
+            assert all(torch.equal(a, b) for a, b in zip(got[k], alone[k]))
+        assert all(torch.equal(r, rows_alone) for r in rows)
