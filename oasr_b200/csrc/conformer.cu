@@ -33,8 +33,7 @@ struct Workspace {
 
 int64_t align256(int64_t x) { return (x + 255) / 256 * 256; }
 
-constexpr Chain kFirst{0, 1};   // the executor's first GEMM, and the ones behind it (gemm_small.cuh)
-constexpr Chain kInner{1, 0};
+constexpr Chain kFirst{0, 1};   // the executor's first GEMM; the ones behind it: inner_chain() (gemm_small.cuh)
 
 struct ChunkWorkspace {
   float* res;
@@ -212,8 +211,8 @@ int oasr_b200_conformer_encode_packed(const oasr_b200_conformer_model* model, co
 #define OB_LINEAR(label, fl, out, in, wt, bs, lay, qi, N, K, act, glu)                                              \
   do {                                                                                                              \
     if (qk == 0) {                                                                                                  \
-      if (glu) OB_STEP("gemm_glu " label, fl, gemm_glu_op(out, in, wt, bs, M, N, K, dt, stream, kInner));             \
-      else OB_STEP("gemm " label, fl, gemm_op(out, in, wt, bs, M, N, K, act, dt, stream, kInner));                   \
+      if (glu) OB_STEP("gemm_glu " label, fl, gemm_glu_op(out, in, wt, bs, M, N, K, dt, stream, inner));             \
+      else OB_STEP("gemm " label, fl, gemm_op(out, in, wt, bs, M, N, K, act, dt, stream, inner));                   \
     } else {                                                                                                        \
       OB_STEP("quantize_rows", 0, oasr_b200_quantize_rows(w.q8, w.qs, in, M, K, qk, dt, stream));                     \
       OB_STEP("gemm_q8 " label, fl, oasr_b200_gemm_q8(out, w.q8, w.qs, (lay).q_w[qi], (lay).q_s[qi], bs, M, N, K, act, glu, qk, dt, stream)); \
@@ -235,6 +234,7 @@ int oasr_b200_conformer_encode_packed(const oasr_b200_conformer_model* model, co
   // Few rows: the Linear adds into the fp32 residual stream itself (its few output bytes cost nothing there) and the norm
   // reads the sum, which is then never rounded to 16 bits.
   const bool resid = !fuse && qk == 0;
+  const Chain inner = inner_chain(!fuse && starts_late(gsm::kResid, M, d, m.embed_in));
   // add + norm; with an 8-bit kind (and an unsplit h) the kernel also leaves the quantised row of h in w.q8 / w.qs for
   // the Linear that reads h next, which then skips its own quantisation launch (OB_LINEAR_H)
 #define OB_ADD_NORM(hout, rout, rin, y_, alpha, mode, wa, ba, wb, bb, eps_, split)                                      \
@@ -251,7 +251,7 @@ int oasr_b200_conformer_encode_packed(const oasr_b200_conformer_model* model, co
       OB_STEP("gemm_addnorm " label, fl, oasr_b200_gemm_add_norm_f32(hout, w.res, rin, in, wt, bs, M, d, K, alpha, mode, wa, ba, \
                                                                     wb, bb, eps_, split, dt, stream));              \
     } else if (resid && gsm::takes(gsm::kResid, M, d, K)) {                                                                                             \
-      OB_STEP("gemm " label, fl, gemm_residual_f32_op(w.res, rin, in, wt, bs, M, d, K, alpha, dt, stream, kInner));   \
+      OB_STEP("gemm " label, fl, gemm_residual_f32_op(w.res, rin, in, wt, bs, M, d, K, alpha, dt, stream, inner));   \
       OB_ADD_NORM(hout, (mode) == 2 ? w.res : nullptr, w.res, nullptr, 0.0, mode, wa, ba, wb, bb, eps_, split);       \
     } else {                                                                                                        \
       OB_LINEAR(label, fl, w.y, in, wt, bs, lay, qi, d, K, OASR_ACT_NONE, 0);                                        \
@@ -283,7 +283,7 @@ int oasr_b200_conformer_encode_packed(const oasr_b200_conformer_model* model, co
     att_plan = w.att_plan;
   }
   // linear_pos of every layer in one GEMM: (max_seg, d) x (L*d, d)^T
-  OB_STEP("gemm linear_pos", 2.0 * max_seg * L * d * d, gemm_op(w.pos, m.pe, m.pos_w_all, nullptr, max_seg, L * d, d, OASR_ACT_NONE, dt, stream, kInner));
+  OB_STEP("gemm linear_pos", 2.0 * max_seg * L * d * d, gemm_op(w.pos, m.pe, m.pos_w_all, nullptr, max_seg, L * d, d, OASR_ACT_NONE, dt, stream, inner));
 
   for (int64_t i = 0; i < L; ++i) {
     const oasr_b200_conformer_layer& l = ly[i];
@@ -293,7 +293,7 @@ int oasr_b200_conformer_encode_packed(const oasr_b200_conformer_model* model, co
                       l.norm_mha_b, nullptr, nullptr, m.eps, 0);
     // relative-position self-attention
     if (qkv_dup) {   // [Wq;Wk;Wv] are rows d.. of [Wq;Wq;Wk;Wv]: the query block once, stored as q+u and q+v
-      OB_STEP("gemm qkv4", 2.0 * M * 3 * d * d, gemm_dup_first_op(w.qkv4, w.h, static_cast<const uint8_t*>(l.qkv4_w) + d * d * 2, l.qkv4_b, M, 3 * d, d, d, dt, stream, kInner));
+      OB_STEP("gemm qkv4", 2.0 * M * 3 * d * d, gemm_dup_first_op(w.qkv4, w.h, static_cast<const uint8_t*>(l.qkv4_w) + d * d * 2, l.qkv4_b, M, 3 * d, d, d, dt, stream, inner));
     } else {
       OB_LINEAR_H("qkv4", 2.0 * M * 3 * d * d /* algorithmic: the query block is issued twice */, w.qkv4, l.qkv4_w, l.qkv4_b, l, 2, 4 * d, OASR_ACT_NONE, 0);
     }
@@ -320,7 +320,7 @@ int oasr_b200_conformer_encode_packed(const oasr_b200_conformer_model* model, co
   }
   if (log_probs || argmax) {   // log_probs == NULL: token-only head, one vocabulary sweep, no log-prob write
     OB_STEP("gemm_log_softmax", 2.0 * M * m.vocab_padded * d /* algorithmic; issued with the input split in two 16-bit terms (K = 2d) */, gemm_log_softmax_op(log_probs, w.h3, m.ctc_w, m.ctc_b, M, m.vocab_padded, 2 * d, dt, OASR_DT_F32,
-                                       argmax, stream, kInner));
+                                       argmax, stream, inner));
   }
   return OASR_OK;
 }
@@ -419,14 +419,15 @@ int oasr_b200_conformer_chunk_paged(const oasr_b200_conformer_model* model, cons
   const double scale = 1.0 / std::sqrt(64.0);
   const oasr_b200_conformer_layer* ly = m.layers;
 
+  const Chain inner = inner_chain(starts_late(gsm::kResid, M, d, m.embed_in));
   const bool qkv_dup = qk == 0 && g_qkv_dup != 0 && B * T >= 128 && oasr_b200_gemm_dup_first_supported(3 * m.d_model, m.d_model, m.d_model) != 0;
   // One Linear over `R` rows: 16-bit GEMM, or per-token quantisation of the input followed by the 8-bit GEMM on the
   // layer's pre-quantised weight `qi` (order of oasr_b200_conformer_layer::q_w), as in the offline executor.
 #define OB_CHUNK_LINEAR(label, fl, out, in, wt, bs, lay, qi, R, N, K, act, glu)                                       \
   do {                                                                                                                \
     if (qk == 0) {                                                                                                    \
-      if (glu) OB_STEP("gemm_glu " label, fl, gemm_glu_op(out, in, wt, bs, R, N, K, dt, stream, kInner));               \
-      else OB_STEP("gemm " label, fl, gemm_op(out, in, wt, bs, R, N, K, act, dt, stream, kInner));                     \
+      if (glu) OB_STEP("gemm_glu " label, fl, gemm_glu_op(out, in, wt, bs, R, N, K, dt, stream, inner));               \
+      else OB_STEP("gemm " label, fl, gemm_op(out, in, wt, bs, R, N, K, act, dt, stream, inner));                     \
     } else {                                                                                                          \
       OB_STEP("quantize_rows", 0, oasr_b200_quantize_rows(w.q8, w.qs, in, R, K, qk, dt, stream));                       \
       OB_STEP("gemm_q8 " label, fl, oasr_b200_gemm_q8(out, w.q8, w.qs, (lay).q_w[qi], (lay).q_s[qi], bs, R, N, K, act, glu, qk, dt, stream)); \
@@ -443,7 +444,7 @@ int oasr_b200_conformer_chunk_paged(const oasr_b200_conformer_model* model, cons
 #define OB_CHUNK_LINEAR_ADDNORM(label, fl, hout, in, wt, bs, lay, qi, K, alpha, mode, wa, ba, wb, bb, split)          \
   do {                                                                                                                \
     if (qk == 0 && gsm::takes(gsm::kResid, M, d, K)) {                                                                \
-      OB_STEP("gemm " label, fl, gemm_residual_f32_op(w.res, w.res, in, wt, bs, M, d, K, alpha, dt, stream, kInner));   \
+      OB_STEP("gemm " label, fl, gemm_residual_f32_op(w.res, w.res, in, wt, bs, M, d, K, alpha, dt, stream, inner));   \
       OB_ADD_NORM(hout, (mode) == 2 ? w.res : nullptr, w.res, nullptr, 0.0, mode, wa, ba, wb, bb, m.eps, split);        \
     } else {                                                                                                          \
       OB_CHUNK_LINEAR(label, fl, w.y, in, wt, bs, lay, qi, M, d, K, OASR_ACT_NONE, 0);                                 \
@@ -463,7 +464,7 @@ int oasr_b200_conformer_chunk_paged(const oasr_b200_conformer_model* model, cons
     OB_CHUNK_LINEAR_ADDNORM("ffn_w2", 2.0 * M * m.ffn * d, w.h, w.a_ffn, l.ffm_w2, l.ffm_b2, l, 1, m.ffn, 0.5, 0, l.norm_mha_w, l.norm_mha_b, nullptr, nullptr, 0);
     // attention: project, append the chunk's keys/values to the pages, attend over cache + chunk
     if (qkv_dup) {
-      OB_STEP("gemm qkv4", 2.0 * M * 3 * d * d, gemm_dup_first_op(w.qkv4, w.h, static_cast<const uint8_t*>(l.qkv4_w) + d * d * 2, l.qkv4_b, M, 3 * d, d, d, dt, stream, kInner));
+      OB_STEP("gemm qkv4", 2.0 * M * 3 * d * d, gemm_dup_first_op(w.qkv4, w.h, static_cast<const uint8_t*>(l.qkv4_w) + d * d * 2, l.qkv4_b, M, 3 * d, d, d, dt, stream, inner));
     } else {
       OB_CHUNK_LINEAR_H("qkv4", 2.0 * M * 3 * d * d, w.qkv4, l.qkv4_w, l.qkv4_b, l, 2, 4 * d, OASR_ACT_NONE);
     }
@@ -505,7 +506,7 @@ int oasr_b200_conformer_chunk_paged(const oasr_b200_conformer_model* model, cons
   }
   if (log_probs || argmax) {   // log_probs == NULL: token-only head, one vocabulary sweep, no log-prob write
     OB_STEP("gemm_log_softmax", 2.0 * M * m.vocab_padded * d /* algorithmic; issued with the input split in two 16-bit terms (K = 2d) */, gemm_log_softmax_op(log_probs, w.h3, m.ctc_w, m.ctc_b, M, m.vocab_padded, 2 * d, dt, OASR_DT_F32,
-                                       argmax, stream, kInner));
+                                       argmax, stream, inner));
   }
   return OASR_OK;
 }

@@ -280,7 +280,7 @@ int oasr_b200_fastconformer_chunk_paged(const oasr_b200_fastconformer_model* mod
   const double scale = 1.0 / std::sqrt(static_cast<double>(D)), eps = m.eps;
   const oasr_b200_fastconformer_layer* ly = m.layers;
   const bool conv_norm = oasr_b200_dwconv_norm_swish_supported(C, m.kernel) != 0 && B < 65536;
-  const Chain inner{1, 0};       // weights settled: see gemm_small.cuh
+  const Chain inner = inner_chain(starts_late(gsm::kStore, M, F, C));   // see gemm_small.cuh
   // last Linear of a sub-layer + residual + norm (mode 2: norm_out and the next pre-norm); few rows: the Linear adds into
   // the fp32 stream itself
 #define FC_CHUNK_LINEAR_ADDNORM(in, wt, bs, K, alpha, mode, res_to, wa, ba, wb, bb)                                     \

@@ -1264,6 +1264,8 @@ static bool small_rows(int epi, int64_t M, int64_t N, int64_t K, int64_t dup_col
 }
 }  // namespace gemm
 
+bool starts_late(int epi, int64_t M, int64_t N, int64_t K) { return gemm::small_rows(epi, M, N, K) && !gemm::use_simt(M, N, K); }
+
 int gemm_op(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int activation, int dtype, void* stream, Chain chain) {
   using namespace ob;
   using namespace ob::gemm;

@@ -19,7 +19,8 @@ struct Args {
   float alpha = 1.f;
   // How an executor's chain of launches uses programmatic dependent launch.  late_launch: the chain's first GEMM lets its
   // successor start only once everything before the chain is complete and visible; b_static: a later GEMM of the chain,
-  // whose weights (B, bias) are therefore settled, fetches them before it waits for its predecessor.
+  // whose weights (B, bias) are therefore settled, fetches them before it waits for its predecessor.  Only behind a first
+  // GEMM that starts_late(): the other kernels let their successor start before their own wait.
   int b_static = 0;
   int late_launch = 0;
 };
@@ -36,6 +37,9 @@ int run(int epi, const Args& a, int dtype, cudaStream_t s);
 struct Chain {
   int b_static = 0, late_launch = 0;
 };
+// Does the operator with this epilogue run a kernel that honours late_launch?  The chain behind it may then be inner_chain().
+bool starts_late(int epi, int64_t M, int64_t N, int64_t K);
+inline Chain inner_chain(bool first_starts_late) { return Chain{first_starts_late ? 1 : 0, 0}; }
 int gemm_op(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int activation, int dtype,
             void* stream, Chain chain);
 int gemm_glu_op(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int dtype, void* stream,
