@@ -344,8 +344,12 @@ class FastConformerLayers:
         slots = list(slots)
         if Tq != cache.chunk or len(slots) != B:
             raise RuntimeError(f"expected {len(slots)} streams x {cache.chunk} frames, got {B} x {Tq}")
+        if C != self.C:
+            raise RuntimeError(f"expected states of width {self.C}, got {C}")
+        native = (self.native and not self.qkind and self._window_fits() and hidden.dtype in (torch.float32, self.dtype) and
+                  self._native_cache(cache))
         table, cached, total, pos_start, slot_ids = cache.prepare(slots)
-        if self.native and not self.qkind and self._window_fits() and hidden.dtype in (torch.float32, self.dtype):
+        if native:
             out = self._chunk_native(hidden.reshape(B * Tq, C).contiguous(), B, Tq, cache, table, cached, pos_start, slot_ids)
             cache.commit(slots)
             return out.view(B, Tq, C)
@@ -397,6 +401,17 @@ class FastConformerLayers:
                 fused.add_norm_f32(h, out, res, y, 0.5, fused.ADD_NORM_LN_LN, *lw["norm_out"], *lw["norm_out"], eps=self.eps)
         cache.commit(slots)
         return out.view(B, Tq, C)
+
+    def _native_cache(self, cache) -> bool:
+        """Is ``cache`` laid out as the native step takes it by address (this model's type and geometry, dense layers)?  Any
+        other goes to the composition, whose operators accept or refuse it."""
+        k, v, state = cache.k_pool, cache.v_pool, cache.cnn_state
+        if not all(isinstance(t, torch.Tensor) and t.dtype == self.dtype and t.device == k.device for t in (k, v, state)):
+            return False
+        pages = (cache.num_blocks, cache.block_size, self.H, self.D)
+        return (k.shape[1:] == pages and k.size(0) >= self.L and v.shape == k.shape and v.stride() == k.stride() and
+                k[0].is_contiguous() and state.is_contiguous() and state.size(0) >= self.L and
+                state.shape[1:] == (cache.max_streams, self.K - 1, self.C))
 
     def _chunk_native(self, rows: torch.Tensor, B: int, Tq: int, cache, table, cached, pos_start, slot_ids) -> torch.Tensor:
         """The streaming step in ONE call into the native executor (oasr_b200_fastconformer_chunk_paged): 14 launches per

@@ -388,3 +388,19 @@ def test_streaming_steps_and_packed_batches_run_on_streams_of_their_own():
         for k in (0, 1):
             assert all(torch.equal(a, b) for a, b in zip(got[k], alone[k]))
         assert all(torch.equal(r, rows_alone) for r in rows)
+
+
+def test_streaming_step_refuses_what_its_operators_refuse():
+    """A cache of fp8 pages or of another 16-bit type, and states of another width, are errors and not read as the model's own."""
+    from oasr_b200.streaming import StreamingCache
+
+    cfg = OFC.TINY
+    model = FastConformerLayers(cfg.hidden, cfg.heads, cfg.ffn, cfg.layers, cfg.kernel, cfg.sliding_window, cfg.lookahead, OFC.init_params(cfg, 3))
+    geometry = (cfg.layers, cfg.heads, cfg.hidden // cfg.heads, cfg.hidden, cfg.kernel, 2, 16)
+    hidden = torch.randn(1, 16, cfg.hidden, device="cuda")
+    for kw in ({"kv_scales": torch.ones(cfg.layers, 2, cfg.heads)}, {"dtype": torch.float16}):
+        with pytest.raises(ValueError, match="dtypes must match"):
+            model.forward_chunk(hidden, [0], StreamingCache(*geometry, **kw))
+    with pytest.raises(RuntimeError, match="width"):
+        model.forward_chunk(hidden[..., :128], [0], model.new_streaming_cache(2))
+    assert ob.device_status() == 0
