@@ -234,9 +234,9 @@ fmha_relpos64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   };
   constexpr uint32_t kIdleLimit = 1u << 24;   // polls without progress before the role gives up (a sleep between polls
                                               // measured slower: 45.4 / 46.0 / 46.3 / 46.7 us per launch for 0 / 20 / 40 / 100 ns)
-  // Both run as whole warps with one elected lane issuing (see gemm.cu); a barrier counts as complete as soon as one lane
-  // has seen it, so that all lanes take the same way.
-  auto done = [&](uint64_t* bar, uint32_t parity) -> bool { return __any_sync(0xffffffffu, ptx::mbar_test(bar, parity)) != 0; };
+  // Both run as whole warps with one elected lane issuing (see gemm.cu); a barrier counts as complete once every lane has
+  // seen it, so that all lanes take the same way and the one that issues has acquired what the barrier orders.
+  auto done = [&](uint64_t* bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, ptx::mbar_test(bar, parity)) != 0; };
   if (warp == 5) {
     // =================== TMA producer ===================
     {

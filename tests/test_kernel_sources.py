@@ -24,3 +24,10 @@ def test_tensor_memory_is_allocated_before_dependents_may_start(name):
         trigger = body.find("grid_dep_launch()")
         assert trigger < 0 or trigger > body.rfind("tmem_alloc"), f"{name}: grid_dep_launch() before the allocation"
     assert kernel_allocs
+
+
+@pytest.mark.parametrize("name", sorted(p.name for p in CSRC.glob("*.cu*") if "mbar_test(" in _code(p)))
+def test_a_warp_counts_a_barrier_as_complete_only_if_every_lane_has_seen_it(name):
+    """mbarrier tests acquire for the lane that sees the phase complete; a vote carries no ordering to the others, and the lane
+    that issues the copy or the MMA behind it may be any of them."""
+    assert not re.search(r"__(any|ballot)_sync\b", _code(CSRC / name))
