@@ -453,7 +453,11 @@ __global__ void __launch_bounds__(128, 4) dwconv_roll_kernel(DwArgs a) {
   auto fetch = [&](int ti) -> uint32_t {    // input frame ti of the segment: data, the fill value past its end, else zero
     uint32_t v = 0;
     if (ti >= 0 && ti < TL) {
-      if (!kMask || !mask || mask[ti]) v = __ldg(in + ti * row_u32);
+      v = __ldg(in + ti * row_u32);
+      if (kMask && mask && !mask[ti]) {       // a product with zero and not a choice: what is no number stays none
+        const float2 x = unpack_pair<T>(v);
+        v = pack_pair<T>(x.x * 0.f, x.y * 0.f);
+      }
     } else if (ti >= TL && ti < fill_end) {
       v = fill;
     }
@@ -502,7 +506,7 @@ __global__ void __launch_bounds__(128, 4) dwconv_roll_kernel(DwArgs a) {
           acc.x += xc.x;
           acc.y += xc.y;
         }
-        if (mask && t < t_end && !mask[t]) acc = make_float2(0.f, 0.f);
+        if (mask && t < t_end && !mask[t]) acc = make_float2(acc.x * 0.f, acc.y * 0.f);
       }
       if constexpr (kAct == 1) {
         const float2 h = __fmul2_rn(acc, make_float2(0.5f, 0.5f));

@@ -155,6 +155,22 @@ def test_depthwise_conv1d_fsmn_mask(dtype, bool_mask):
     _close(got, O.depthwise_conv1d(x, w, None, (K - 1) // 2, mask=mask, add_input=True), dtype, scale=2.0)
 
 
+# 16-bit types at kernel sizes 9 and 15: the rolling kernel takes the bool mask; T around its runs of 4 K frames
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("K,T,C", [(9, 36, 64), (9, 73, 10), (15, 60, 256), (15, 7, 24), (15, 121, 514)])
+@pytest.mark.parametrize("masked,add_input", [(True, False), (True, True), (False, True)])
+def test_depthwise_conv1d_mask_of_the_rolling_kernel(dtype, K, T, C, masked, add_input):
+    x, w, b = _rand((3, T, C), dtype, 33), _rand((K, C), dtype, 34, 0.3), _rand((C,), dtype, 35)
+    mask = (torch.arange(T)[None, :] < torch.tensor([T, (T + 1) // 2, 1])[:, None]).unsqueeze(-1) if masked else None
+    if masked:          # padding that is no number: the input is multiplied by the mask, here as everywhere
+        x[1, -1, :2], x[2, -1, 2:4] = float("inf"), float("nan")
+        x[1, -2, 4:6] = -torch.finfo(dtype).max
+    got = ob.depthwise_conv1d(x.cuda(), w.cuda(), b.cuda(), (K - 1) // 2, mask=mask.cuda() if masked else None, add_input=add_input)
+    want = O.depthwise_conv1d(x, w, b, (K - 1) // 2, mask=mask, add_input=add_input)
+    # one rounding (half an ulp, 2^-9 / 2^-12 of the value) and K + 1 fp32 additions of values of a few units
+    torch.testing.assert_close(got.float().cpu(), want, rtol=2.0 ** (-8 if dtype == torch.bfloat16 else -11), atol=1e-5, equal_nan=True)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("T", [16, 3, 1])
 def test_causal_conv1d_state(dtype, T):
