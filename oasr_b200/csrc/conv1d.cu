@@ -511,6 +511,9 @@ __global__ void __launch_bounds__(128, 4) dwconv_roll_kernel(DwArgs a) {
       if constexpr (kAct == 1) {
         const float2 h = __fmul2_rn(acc, make_float2(0.5f, 0.5f));
         acc = __ffma2_rn(h, make_float2(tanh_approx(h.x), tanh_approx(h.y)), h);
+      } else if constexpr (kAct == 2 && kMask) {   // as exact as the general kernel, which takes the other masks
+        acc.x = apply_act_rt(acc.x, a.act);
+        acc.y = apply_act_rt(acc.y, a.act);
       } else if constexpr (kAct == 2) {
         acc.x = apply_act_fast(acc.x, a.act);
         acc.y = apply_act_fast(acc.y, a.act);

@@ -171,6 +171,28 @@ def test_depthwise_conv1d_mask_of_the_rolling_kernel(dtype, K, T, C, masked, add
     torch.testing.assert_close(got.float().cpu(), want, rtol=2.0 ** (-8 if dtype == torch.bfloat16 else -11), atol=1e-5, equal_nan=True)
 
 
+@pytest.mark.parametrize("K", [9, 11, 15])
+def test_masked_depthwise_conv1d_swish_is_exact_to_the_rounding(K):
+    """The C entry point takes a mask together with swish: half an ulp of fp16 from the exact value, whichever kernel runs
+    (a swish by one tanh.approx, relative error 2^-11, is not)."""
+    from oasr_b200 import _lib
+
+    B, T, C = 2, 90, 64
+    x, w, b = _rand((B, T, C), torch.float16, 41), _rand((K, C), torch.float16, 42, 0.3), _rand((C,), torch.float16, 43)
+    mask = torch.arange(T)[None, :] < torch.tensor([T, 50])[:, None]
+    out = torch.empty(B, T, C, dtype=torch.float16, device="cuda")
+    dev = [t.cuda() for t in (x, w, b, mask)]
+    _lib.call("oasr_b200_depthwise_conv1d", out.data_ptr(), *(t.data_ptr() for t in dev[:3]), B, T, C, K, (K - 1) // 2, (K - 1) // 2,
+              dev[3].data_ptr(), 1, 0, 2, 1, torch.cuda.current_stream().cuda_stream)
+    m = mask[..., None].double()
+    y = torch.nn.functional.conv1d((x.double() * m).transpose(1, 2), w.double().t()[:, None], b.double(), padding=(K - 1) // 2,
+                                   groups=C).transpose(1, 2) * m
+    y = torch.nn.functional.silu(y)
+    half_ulp = torch.ldexp(torch.ones_like(y), torch.frexp(y)[1].clamp(min=-13) - 12)
+    # beside it: K + 1 fp32 additions and an exponential of 2 ulp on values of a few units, 16 * 2^-24 each
+    assert ((out.double().cpu() - y).abs() <= half_ulp + 1e-6 * (1 + y.abs())).all()
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("T", [16, 3, 1])
 def test_causal_conv1d_state(dtype, T):
