@@ -119,3 +119,22 @@ def test_512_point_kernel_at_other_framings_and_odd_frame_counts(length_ms, shif
         if n:
             assert (got[b, :n].cpu() - want[b, :n]).abs().max().item() < 3e-3     # fp32 FFT and summation order, as above
         assert torch.count_nonzero(got[b, n:]) == 0
+
+
+@pytest.mark.gpu
+def test_sample_counts_in_every_form_they_are_given():
+    """A column, more counts than waveforms, a list, another integer type, on the GPU: the frame counts come in that shape;
+    fewer counts than waveforms are refused."""
+    from oasr_b200 import features as F
+
+    wave = torch.randn(3, 1600, generator=torch.Generator().manual_seed(4)).cuda()
+    counts = torch.tensor([1600, 399, 700])
+    want, frames = F.batched_fbank(wave, counts)
+    assert frames.tolist() == [8, 0, 2] and frames.dtype == torch.int32
+    for form in (counts[:, None], counts.tolist(), counts.to(torch.int16).cuda(), list(counts), torch.cat([counts, counts[:2]])):
+        got, n = F.batched_fbank(wave, form)
+        assert torch.equal(got, want) and n.shape == torch.as_tensor(form).shape and n.dtype == torch.int32
+        assert n.reshape(-1)[:3].tolist() == [8, 0, 2] and n.device == wave.device
+    for form in (counts[:1], counts[:2].tolist(), 1600):
+        with pytest.raises(ValueError, match="sample counts"):
+            F.batched_fbank(wave, form)
