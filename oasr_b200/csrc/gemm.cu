@@ -904,6 +904,7 @@ int g_use_pairs = 2; // CTA pairs (cta_group::2) for dense problems: 0 never, 1 
 //   28000 rows: N 4096, K 1024 166.0 / 153.6;  N 1024, K 4096 155.6 / 145.4;  N 1024, K 1024 53.2 / 51.2;  GLU 1024, K 1024 82.0 / 75.8
 //    8000 rows: N 4096, K 1024 59.4 / 57.3;    N 1024, K 4096 61.4 / 57.3;    GLU 34.8 / 32.9
 //    4000 rows: N 1024, K 1024 (64 pair tiles) 18.4 / 20.5;   16722 rows: N 2048, K 512 43.0 / 47.1, N 1536, K 512 36.9 / 38.9
+bool pairs_can(int64_t M, int64_t n_acc, int64_t K) { return M >= 1024 && n_acc >= 256 && K >= 128; }
 bool pairs_ahead(int64_t M, int64_t n_acc, int64_t K) {
   const int64_t tiles = (M + 2 * BM - 1) / (2 * BM) * ((n_acc + 255) / 256);
   return K >= 1024 && tiles >= sm_count() / 2;
@@ -1127,7 +1128,7 @@ int run_typed(Problem& pr, int dtype, cudaStream_t s) {
   int bn = kEpi == kEpiLsm ? (g_force_bn ? g_force_bn : 256) : pick_bn(m_tiles_total, n_eff, pr.K);
   if (kEpi == kEpiGlu && bn < 128) bn = 128;  // half tiles of >= 64 columns
   constexpr bool kPairCapable = kSched == kSchedDense && (kEpi == kEpiStore || kEpi == kEpiGlu);
-  const bool pair = kPairCapable && g_use_pairs && g_force_bn == 0 && pr.M >= 1024 && n_eff >= 256 && pr.K >= 128 &&
+  const bool pair = kPairCapable && g_use_pairs && g_force_bn == 0 && pairs_can(pr.M, n_eff, pr.K) &&
                     (g_use_pairs == 1 || (pr.batch == 1 && bn == 256 && pairs_ahead(pr.M, n_eff, pr.K)));
   if (pair) bn = 256;
   p.num_m_tiles = static_cast<int>((pr.M + BM - 1) / BM);
@@ -1258,9 +1259,12 @@ extern "C" int oasr_b200_gemm_dup_first_supported(int64_t N, int64_t K, int64_t 
 namespace ob {
 
 namespace gemm {
-// Dense 16-bit problems of few rows go to gemm_small.cu; a forced tile width names a kernel of this file.
+// Dense 16-bit problems of few rows go to gemm_small.cu; a forced tile width, or pairs wherever they can run, names a kernel
+// of this file.
 static bool small_rows(int epi, int64_t M, int64_t N, int64_t K, int64_t dup_cols = 0) {
-  return g_force_bn == 0 && gsm::takes(epi, M, N, K, dup_cols);
+  if (g_force_bn != 0) return false;
+  if (g_use_pairs == 1 && (epi == gsm::kStore || epi == gsm::kGlu) && pairs_can(M, epi == gsm::kGlu ? 2 * N : N, K)) return false;
+  return gsm::takes(epi, M, N, K, dup_cols);
 }
 }  // namespace gemm
 

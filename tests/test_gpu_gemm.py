@@ -175,7 +175,11 @@ def test_gemm_cta_pairs_match_single_cta_tiles(dtype, M, N, K):
 
     A, B, C = _rand((M, K), dtype, 31), _rand((N, K), dtype, 32, K ** -0.5), _rand((N,), dtype, 33)
     want = O.gemm(A, B, C, 2)
-    got_single = ob.gemm_activation(A.cuda(), B.cuda(), C.cuda(), 2)
+    try:
+        tunables.set("gemm_bn", 256)        # names the single-CTA kernel, whatever the number of rows
+        got_single = ob.gemm_activation(A.cuda(), B.cuda(), C.cuda(), 2)
+    finally:
+        tunables.set("gemm_bn", 0)
     tunables.set("gemm_pairs", 1)
     try:
         got_pair = ob.gemm_activation(A.cuda(), B.cuda(), C.cuda(), 2)
@@ -183,7 +187,7 @@ def test_gemm_cta_pairs_match_single_cta_tiles(dtype, M, N, K):
             Bg, Cg = _rand((2 * N, K), dtype, 34, K ** -0.5), _rand((2 * N,), dtype, 35)
             _check(ob.gemm_glu(A.cuda(), Bg.cuda(), Cg.cuda()), O.gemm_glu(A, Bg, Cg), dtype)
     finally:
-        tunables.set("gemm_pairs", 0)
+        tunables.set("gemm_pairs", 2)
     _check(got_pair, want, dtype)
     _check(got_single, want, dtype)
     assert torch.equal(got_pair, got_single)   # fp32 accumulation order along K is the same
