@@ -81,6 +81,31 @@ def test_stem_and_depthwise_conv_in_one(dtype, B, T, Fb, C, lens):
     assert got.shape == want.shape and torch.equal(got, want)
 
 
+# (SL + T) * slab pieces of a block: one, two and four per thread, narrower slabs, the last size of the kernel and the first of
+# the two launches behind it; inputs shorter than the state
+@pytest.mark.parametrize("SL,T,C,dtype", [(8, 16, 256, torch.bfloat16), (14, 3, 72, torch.float16), (2, 40, 80, torch.float32),
+                                          (14, 100, 64, torch.bfloat16), (2, 300, 24, torch.float32), (2, 1022, 8, torch.bfloat16),
+                                          (2, 1023, 72, torch.bfloat16), (0, 5, 8, torch.float16)])
+def test_conv_state_is_concatenated_and_rolled(SL, T, C, dtype):
+    from oasr_b200 import _lib
+    from oasr_b200.functional import _DTYPE_ID
+
+    g = torch.Generator().manual_seed(SL + T)
+    state, x = torch.randn(5, SL, C, generator=g).to(dtype).cuda(), torch.randn(4, T, C, generator=g).to(dtype).cuda()
+    slots = [3, -1, 0, 7]                                   # two outside the buffer: zeros before the input, nothing kept
+    want_state = state.clone()
+    before = [state[s] if 0 <= s < 5 else torch.zeros_like(state[0]) for s in slots]
+    want = torch.stack([torch.cat([b, x[i]]) for i, b in enumerate(before)])
+    for i, s in enumerate(slots):
+        if 0 <= s < 5:
+            want_state[s] = want[i, T:]
+    got, ids = torch.full_like(want, 7.0), torch.tensor(slots).cuda()
+    held = state if SL else torch.empty(5, 1, C, dtype=dtype, device="cuda")       # an empty tensor has no address
+    _lib.call("oasr_b200_conv_state_concat", got.data_ptr(), held.data_ptr(), 5, ids.data_ptr(), x.data_ptr(), 4, SL, T, C,
+              _DTYPE_ID[dtype], torch.cuda.current_stream().cuda_stream)
+    assert torch.equal(got, want) and torch.equal(state, want_state)
+
+
 def test_other_kernel_sizes_keep_the_separate_steps():
     """A conv of 5 taps: packed batches native and composed agree bit for bit, streams continue their cached tail (chunks
     against the offline pass, tolerance of the streaming tests: the two attend through different kernels in bf16)."""

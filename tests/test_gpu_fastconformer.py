@@ -285,8 +285,9 @@ def test_streaming_from_feature_frames_matches_the_oracle():
     assert torch.equal(again, first)
 
 
+@pytest.mark.parametrize("longest", [128, 129, 200])         # from 129 frames on: attention inside its window, 14 + 4 launches per layer
 @pytest.mark.parametrize("quant", ["fp8", "int8"])
-def test_native_executor_with_8bit_linears_equals_the_composed_stack(quant):
+def test_native_executor_with_8bit_linears_equals_the_composed_stack(quant, longest):
     """With an 8-bit kind the native executor quantises every Linear's input per token and runs the fp8 / int8 GEMM on
     the weight quantised once per output channel -- the same two kernels per Linear as the Python composition, so
     the results are bit-identical, and they stay within the 8-bit gate (cosine >= 0.999) of the 16-bit stack."""
@@ -297,8 +298,8 @@ def test_native_executor_with_8bit_linears_equals_the_composed_stack(quant):
     args = (cfg.hidden, cfg.heads, cfg.ffn, cfg.layers, cfg.kernel, cfg.sliding_window, cfg.lookahead, P)
     model = FastConformerLayers(*args, quant=quant)
     assert model.native and model._native_model.quant_kind in (1, 2)
-    lengths = [61, 17, 128, 1]
-    hidden = torch.randn(len(lengths), 128, cfg.hidden, generator=torch.Generator().manual_seed(3)).cuda()
+    lengths = [61, 17, longest, 1]
+    hidden = torch.randn(len(lengths), longest, cfg.hidden, generator=torch.Generator().manual_seed(3)).cuda()
     before = _lib.launch_count()
     rows_native, index = model.forward_rows(hidden, lengths)
     launched = _lib.launch_count() - before
@@ -307,14 +308,15 @@ def test_native_executor_with_8bit_linears_equals_the_composed_stack(quant):
     model.native = True
     assert ob.device_status() == 0
     assert torch.equal(rows_native, rows_composed)
-    assert launched >= 21 * cfg.layers          # 17 + 4 per-token quantisations per layer (the other four ride in add + norm)
+    assert launched >= (21 if longest <= 128 else 18) * cfg.layers          # 17 + 4 per-token quantisations per layer (the other four ride in add + norm)
     rows16, _ = FastConformerLayers(*args).forward_rows(hidden, lengths)
     cos = torch.nn.functional.cosine_similarity(rows_native.flatten(), rows16.flatten(), dim=0).item()
     print(f"{quant} native stack vs 16-bit stack: cosine {cos:.6f}")
     assert cos >= 0.999
 
 
-def test_native_executor_equals_the_operator_by_operator_stack():
+@pytest.mark.parametrize("longest", [128, 129, 200])         # from 129 frames on: attention inside its window, 14 launches per layer
+def test_native_executor_equals_the_operator_by_operator_stack(longest):
     """oasr_b200_fastconformer_layers_packed enqueues the same kernels in the same order as the Python composition of
     the packed stack, so the two agree bit for bit; it refuses a workspace that is too small before launching."""
     import ctypes
@@ -325,8 +327,8 @@ def test_native_executor_equals_the_operator_by_operator_stack():
     P = OFC.init_params(cfg, 77)
     model = FastConformerLayers(cfg.hidden, cfg.heads, cfg.ffn, cfg.layers, cfg.kernel, cfg.sliding_window, cfg.lookahead, P)
     assert model.native
-    lengths = [61, 0, 17, 128, 1]
-    hidden = torch.randn(len(lengths), 128, cfg.hidden, generator=torch.Generator().manual_seed(2)).cuda()
+    lengths = [61, 0, 17, longest, 1]
+    hidden = torch.randn(len(lengths), longest, cfg.hidden, generator=torch.Generator().manual_seed(2)).cuda()
     before = _lib.launch_count()
     rows_native, index = model.forward_rows(hidden, lengths)
     launched = _lib.launch_count() - before
@@ -335,7 +337,7 @@ def test_native_executor_equals_the_operator_by_operator_stack():
     model.native = True
     assert ob.device_status() == 0
     assert torch.equal(index, index2) and torch.equal(rows_native, rows_composed)
-    assert launched >= 17 * cfg.layers
+    assert launched >= (17 if longest <= 128 else 14) * cfg.layers
     # 16-bit post-subsampling states (what the front end hands over): the same agreement
     hidden16 = hidden.bfloat16()
     native16, _ = model.forward_rows(hidden16, lengths)

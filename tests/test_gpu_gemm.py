@@ -93,7 +93,8 @@ def test_gemm_glu(dtype, M, N, K):
 
 
 @pytest.mark.parametrize("dtype", HALF)
-@pytest.mark.parametrize("M,N,K,alpha", [(1000, 512, 2048, 0.5), (333, 256, 256, 1.0), (129, 1024, 520, 1.0)])
+@pytest.mark.parametrize("M,N,K,alpha", [(1000, 512, 2048, 0.5), (333, 256, 256, 1.0), (129, 1024, 520, 1.0),
+                                           (2561, 136, 264, 1.0), (2700, 512, 2048, 0.5)])    # from 2561 rows on: gemm.cu
 def test_gemm_residual_f32(dtype, M, N, K, alpha):
     A, B, C = _rand((M, K), dtype, 12), _rand((N, K), dtype, 13, K ** -0.5), _rand((N,), dtype, 14)
     R = _rand((M, N), torch.float32, 15)
@@ -298,16 +299,15 @@ def test_gemm_dup_first_equals_the_gemm_with_the_repeated_weight_block(M):
 
 @pytest.mark.parametrize("M,N,K", [(9473, 512, 1024), (4737, 1024, 1032), (2561, 1024, 1024), (1024, 4864, 1024), (18689, 272, 1024)])
 def test_gemm_rule_for_cta_pairs(M, N, K):
-    """Both sides of the rule's tile count (74 pair tiles on 148 SMs) and ragged rows, columns and K: whichever kernel a
-    product runs on, the bits are those of single-CTA tiles."""
+    """Both sides of the rule's tile count (74 pair tiles on 148 SMs), ragged rows, columns and K, and an unsplit product of few
+    rows: whichever kernel a product runs on, the bits are those of single-CTA tiles."""
     from oasr_b200 import tunables
 
     A, B, C = (t.cuda() for t in (_rand((M, K), torch.bfloat16, 41), _rand((N, K), torch.bfloat16, 42, K ** -0.5), _rand((N,), torch.bfloat16, 43)))
+    by_size, by_size_glu = ob.gemm_activation(A, B, C, 2), ob.gemm_glu(A, B, C)
     try:
-        tunables.set("gemm_pairs", 2)
-        by_size, by_size_glu = ob.gemm_activation(A, B, C, 2), ob.gemm_glu(A, B, C)
-        tunables.set("gemm_pairs", 0)
+        tunables.set("gemm_bn", 256)        # names the single-CTA kernel
         assert torch.equal(by_size, ob.gemm_activation(A, B, C, 2))
         assert torch.equal(by_size_glu, ob.gemm_glu(A, B, C))
     finally:
-        tunables.set("gemm_pairs", 2)
+        tunables.set("gemm_bn", 0)

@@ -43,10 +43,31 @@ def test_duplicated_block(M):
     assert torch.equal(fused.gemm_dup_first(A, B, C, d), ob.gemm(A, torch.cat([B[:d], B]), C))
 
 
-@pytest.mark.parametrize("N,K", [(2048, 512), (512, 2048), (512, 9728)])
+@pytest.mark.parametrize("N,K", [(2048, 512), (512, 2048), (512, 9728), (4096, 512), (4096, 1024)])   # the last two change kernels
 def test_a_row_does_not_depend_on_its_batch(N, K):
-    """The split of K and the order of a row's sums depend on N and K only: bit-identical rows from 1 row to the whole range."""
+    """Outputs of up to 512 columns stay on the kernel, unsplit products give the bits of the one that takes over: bit-identical
+    rows from 1 row to the whole range."""
     A, B = _rand((2560, K), torch.bfloat16, 5).cuda(), _rand((N, K), torch.bfloat16, 6, K ** -0.5).cuda()
     full = ob.gemm(A, B)
     for m in (1, 17, 100, 700):
         assert torch.equal(ob.gemm(A[:m].contiguous(), B), full[:m])
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 512, 512), (100, 4096, 512), (700, 4096, 1024), (1500, 2048, 520), (2560, 520, 968)])
+def test_unsplit_products_have_the_bits_of_the_persistent_kernel(M, N, K):
+    """What lets a product change kernels with its rows: store, swish, GLU and fp32 residual against a forced tile width, which
+    names the kernel of gemm.cu."""
+    from oasr_b200 import tunables
+
+    A, B, C = _rand((M, K), torch.bfloat16, 7).cuda(), _rand((N, K), torch.bfloat16, 8, K ** -0.5).cuda(), _rand((N,), torch.bfloat16, 9).cuda()
+    R = _rand((M, N), torch.float32, 10).cuda()
+    every = lambda: [ob.gemm(A, B, C), ob.gemm_activation(A, B, C, 2), ob.gemm_residual_f32(R, A, B, C, 0.5)] + (
+        [ob.gemm_glu(A, B, C)] if N % 16 == 0 else [])
+    by_size = every()
+    try:
+        tunables.set("gemm_bn", 128)
+        forced = every()
+    finally:
+        tunables.set("gemm_bn", 0)
+    assert ob.device_status() == 0
+    assert all(torch.equal(a, b) for a, b in zip(by_size, forced))
