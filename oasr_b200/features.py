@@ -102,14 +102,13 @@ def batched_fbank(waveforms: torch.Tensor, lengths: torch.Tensor, cfg: FbankConf
     L, hop = cfg.frame_length_samples, cfg.frame_shift_samples
     num_frames = max(0, (T - L) // hop + 1)
     # sample counts and frame counts in one small host array, one copy to the device
-    lengths = torch.as_tensor(lengths).cpu()
-    if lengths.numel() < B:
-        raise ValueError(f"{B} waveforms need as many sample counts, got {lengths.numel()}")
-    counts = np.empty((2, lengths.numel()), dtype=np.int32)
-    counts[0] = lengths.reshape(-1).numpy()
+    host = (lengths if isinstance(lengths, torch.Tensor) else torch.as_tensor(lengths)).cpu().numpy()
+    if host.size < B:
+        raise ValueError(f"{B} waveforms need as many sample counts, got {host.size}")
+    counts = np.empty((2, *host.shape), dtype=np.int32)
+    counts[0] = host
     counts[1] = np.maximum((counts[0].astype(np.int64) - L) // hop + 1, 0)
     len_dev, feat_len = torch.from_numpy(counts).to(dev, non_blocking=True)
-    feat_len = feat_len.view(lengths.shape)
     out = torch.empty(B, num_frames, cfg.num_mel_bins, device=dev, dtype=torch.float32)
     if B == 0 or num_frames == 0:
         return out, feat_len
