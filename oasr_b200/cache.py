@@ -43,7 +43,8 @@ def write_kv_chunk(k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: to
         new_v = new_v.contiguous()
         new_k = new_k.contiguous()
     offset = offset.contiguous()
-    _lib.call("oasr_b200_paged_kv_write", _p(k_cache), _p(v_cache), _p(new_k), _p(new_v), _p(block_table), _p(offset), B, Hkv, T, D, new_k.stride(0), new_k.stride(1), new_k.stride(2),
+    _lib.call("oasr_b200_paged_kv_write", _p(k_cache), _p(v_cache), _p(new_k), _p(new_v), _p(block_table), _p(offset),
+              B, Hkv, T, D, new_k.stride(0), new_k.stride(1), new_k.stride(2),
               block_table.size(1), bs, num_blocks, k_cache.element_size(), _stream(new_k))
 
 

@@ -7,7 +7,7 @@
 //
 // One CTA owns 128 query rows of one (batch|segment, head) and walks the keys
 // in tiles of 128.  160 threads:
-//   warp 4, one thread: TMA producer and tcgen05.mma issuer
+//   warp 4: TMA producer and tcgen05.mma issuer (the whole warp, one elected lane issuing)
 //       S[b]  = Q . K_j^T      (M=128, N=128, K = 64 per atom, 1-2 atoms)  -> TMEM
 //       O[b]  = P_j . V_j      (M=128, N=D,   K = 128)                      -> TMEM
 //     K/V tiles are double-buffered in shared memory (128-byte swizzle), S and

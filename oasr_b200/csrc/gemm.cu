@@ -1270,7 +1270,8 @@ static bool small_rows(int epi, int64_t M, int64_t N, int64_t K, int64_t dup_col
 
 bool starts_late(int epi, int64_t M, int64_t N, int64_t K) { return gemm::small_rows(epi, M, N, K) && !gemm::use_simt(M, N, K); }
 
-int gemm_op(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int activation, int dtype, void* stream, Chain chain) {
+int gemm_op(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int activation,
+            int dtype, void* stream, Chain chain) {
   using namespace ob;
   using namespace ob::gemm;
   if (int rc = validate_common("gemm", D, A, B, bias, M, N, K)) return rc;
@@ -1292,7 +1293,8 @@ int gemm_op(void* D, const void* A, const void* B, const void* bias, int64_t M, 
   return run<kSchedDense, kEpiStore>(pr, dtype, s);
 }
 
-int gemm_dup_first_op(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int64_t dup_cols, int dtype, void* stream, Chain chain) {
+int gemm_dup_first_op(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K,
+                      int64_t dup_cols, int dtype, void* stream, Chain chain) {
   using namespace ob;
   using namespace ob::gemm;
   if (int rc = validate_common("gemm_dup_first", D, A, B, bias, M, N, K)) return rc;
@@ -1343,7 +1345,8 @@ int gemm_dup_first_op(void* D, const void* A, const void* B, const void* bias, i
   });
 }
 
-int gemm_residual_f32_op(float* R_out, const float* R_in, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, double alpha, int dtype, void* stream, Chain chain) {
+int gemm_residual_f32_op(float* R_out, const float* R_in, const void* A, const void* B, const void* bias, int64_t M,
+                         int64_t N, int64_t K, double alpha, int dtype, void* stream, Chain chain) {
   using namespace ob;
   using namespace ob::gemm;
   if (int rc = validate_common("gemm_residual_f32", R_out, A, B, bias, M, N, K)) return rc;
@@ -1363,7 +1366,8 @@ int gemm_residual_f32_op(float* R_out, const float* R_in, const void* A, const v
   return run<kSchedDense, kEpiResid>(pr, dtype, static_cast<cudaStream_t>(stream));
 }
 
-int gemm_glu_op(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int dtype, void* stream, Chain chain) {
+int gemm_glu_op(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int dtype,
+                void* stream, Chain chain) {
   using namespace ob;
   using namespace ob::gemm;
   if (int rc = validate_common("gemm_glu", D, A, B, bias, M, N, K)) return rc;
@@ -1382,7 +1386,8 @@ int gemm_glu_op(void* D, const void* A, const void* B, const void* bias, int64_t
   return run<kSchedDense, kEpiGlu>(pr, dtype, static_cast<cudaStream_t>(stream));
 }
 
-int gemm_log_softmax_op(void* out, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int dtype, int out_dtype, int32_t* argmax, void* stream, Chain chain) {
+int gemm_log_softmax_op(void* out, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K,
+                        int dtype, int out_dtype, int32_t* argmax, void* stream, Chain chain) {
   using namespace ob;
   using namespace ob::gemm;
   // out == NULL with argmax != NULL: only the per-row index of the first maximum is wanted (greedy CTC search);
@@ -1405,12 +1410,12 @@ int gemm_log_softmax_op(void* out, const void* A, const void* B, const void* bia
       a.b_static = chain.b_static; a.late_launch = chain.late_launch;
       if (int rc = gsm::run(gsm::kResid, a, dtype, static_cast<cudaStream_t>(stream))) return rc;
     } else {
-    Problem pg{};
-    pg.sched = kSchedDense; pg.epi = kEpiResid;
-    pg.M = M; pg.N = N; pg.K = K; pg.batch = 1; pg.A = A; pg.B = B;
-    pg.p.M = (int)M; pg.p.N = (int)N; pg.p.K = (int)K; pg.p.batch = 1;
-    pg.p.D = out; pg.p.R_in = nullptr; pg.p.bias = bias; pg.p.act = OASR_ACT_NONE; pg.p.alpha = 1.f;
-    if (int rc = run<kSchedDense, kEpiResid>(pg, dtype, static_cast<cudaStream_t>(stream))) return rc;
+      Problem pg{};
+      pg.sched = kSchedDense; pg.epi = kEpiResid;
+      pg.M = M; pg.N = N; pg.K = K; pg.batch = 1; pg.A = A; pg.B = B;
+      pg.p.M = (int)M; pg.p.N = (int)N; pg.p.K = (int)K; pg.p.batch = 1;
+      pg.p.D = out; pg.p.R_in = nullptr; pg.p.bias = bias; pg.p.act = OASR_ACT_NONE; pg.p.alpha = 1.f;
+      if (int rc = run<kSchedDense, kEpiResid>(pg, dtype, static_cast<cudaStream_t>(stream))) return rc;
     }
     int64_t g = M < static_cast<int64_t>(sm_count()) * 8 ? M : static_cast<int64_t>(sm_count()) * 8;
     launch_pdl(log_softmax_rows_f32_kernel, dim3(static_cast<unsigned>(g)), dim3(256), 0, static_cast<cudaStream_t>(stream),
@@ -1432,7 +1437,8 @@ int gemm_log_softmax_op(void* out, const void* A, const void* B, const void* bia
 
 extern "C" {
 
-int oasr_b200_gemm(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int activation, int dtype, void* stream) {
+int oasr_b200_gemm(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int activation,
+                   int dtype, void* stream) {
   return ob::gemm_op(D, A, B, bias, M, N, K, activation, dtype, stream, ob::Chain{});
 }
 
@@ -1440,7 +1446,8 @@ int oasr_b200_gemm_dup_first_supported(int64_t N, int64_t K, int64_t dup_cols) {
   return N > 0 && K >= 16 && K % 8 == 0 && dup_cols > 0 && dup_cols <= N && N % 256 == 0 && dup_cols % 256 == 0 ? 1 : 0;
 }
 
-int oasr_b200_gemm_dup_first(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int64_t dup_cols, int dtype, void* stream) {
+int oasr_b200_gemm_dup_first(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K,
+                             int64_t dup_cols, int dtype, void* stream) {
   return ob::gemm_dup_first_op(D, A, B, bias, M, N, K, dup_cols, dtype, stream, ob::Chain{});
 }
 
@@ -1476,11 +1483,13 @@ int oasr_b200_gemm_q8(void* D, const void* A_q, const float* a_scale, const void
   });
 }
 
-int oasr_b200_gemm_residual_f32(float* R_out, const float* R_in, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, double alpha, int dtype, void* stream) {
+int oasr_b200_gemm_residual_f32(float* R_out, const float* R_in, const void* A, const void* B, const void* bias, int64_t M,
+                                int64_t N, int64_t K, double alpha, int dtype, void* stream) {
   return ob::gemm_residual_f32_op(R_out, R_in, A, B, bias, M, N, K, alpha, dtype, stream, ob::Chain{});
 }
 
-int oasr_b200_gemm_glu(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int dtype, void* stream) {
+int oasr_b200_gemm_glu(void* D, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int dtype,
+                       void* stream) {
   return ob::gemm_glu_op(D, A, B, bias, M, N, K, dtype, stream, ob::Chain{});
 }
 
@@ -1597,7 +1606,8 @@ int oasr_b200_subsample_conv2(void* out, const void* x1, const void* w2, const v
   });
 }
 
-int oasr_b200_gemm_log_softmax(void* out, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K, int dtype, int out_dtype, int32_t* argmax, void* stream) {
+int oasr_b200_gemm_log_softmax(void* out, const void* A, const void* B, const void* bias, int64_t M, int64_t N, int64_t K,
+                               int dtype, int out_dtype, int32_t* argmax, void* stream) {
   return ob::gemm_log_softmax_op(out, A, B, bias, M, N, K, dtype, out_dtype, argmax, stream, ob::Chain{});
 }
 

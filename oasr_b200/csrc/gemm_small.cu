@@ -13,9 +13,6 @@
 //     (b_static) before this one has finished; only the A tiles wait for the previous kernel.
 //   * narrow tiles (BN 32 / 64 / 128) chosen so that as many SMs as possible pull operand bytes: an SM takes about 50 B
 //     per clock from L2, and operand bytes per SM are what is left of the time.
-// The number of splits depends on N and K only, and a tile's K order never depends on M, so a row's result does not
-// depend on the rows that share its batch (as long as the batch stays on this kernel).
-//
 //   * few barriers: a stage is several K blocks, fetched by one TMA instruction per operand (the K blocks are a tensor
 //     dimension of their own; only rows that exist are fetched), and where the grid leaves SMs free the whole K slice is
 //     resident, so that nothing is ever refilled.  A successful mbarrier wait costs its thread about 0.2k clocks and a
@@ -23,8 +20,9 @@
 //   * the exchange is pushed (st.async credited to the owner's mbarrier), so that an owner waits for its data and not for
 //     a cluster-wide barrier.
 // The number of splits depends on N and K only, and a tile's K order never depends on M; unsplit products give the bits of
-// gemm.cu.  So up to kMaxRows a row's result does not depend on the rows that share its batch, for all outputs of up to 512
-// columns and all unsplit ones.
+// gemm.cu.  So a row's result does not depend on the rows that share its batch for all unsplit products, and up to kMaxRows
+// for all outputs of up to 512 columns.  A split product of a wider output changes its order of sums where takes() hands it
+// to gemm.cu.
 //
 // Roles: warp 0 TMA producer, warp 1 MMA issuer and tensor-memory owner, the other 4 (128-wide tiles: 8) epilogue, a
 // thread per row (and column half); output goes through padded shared memory so that global accesses are coalesced.
