@@ -14,6 +14,12 @@
 // own A box and half of the weight rows of every instruction, 48 KB per 1024 tensor clocks.  With K = 9 * C_in = 4608
 // the main loop is 72 K blocks long, so that the epilogue, which cannot overlap the next tile's main loop (the 128 x
 // 512 fp32 accumulator is all of a CTA's tensor memory), is a small share.  No multicast; every wait is bounded.
+//
+// A few utterances or streams fill few pairs, and then the main loop of one tile over all N channels is all of the time: 72
+// blocks of 1024 tensor clocks for N = 512.  So where pairs are free they share a tile's columns, down to 64 each (grid.y;
+// the order of K, hence every bit, stays): N = 512, 1 to 37 output frames 50 -> 22 us (256 columns 27, 128 columns 22.5; a
+// K block then costs its operands' trip from L2, not its products), 16 streams of 16 frames 57 -> 33 us; N = 256 16.5 ->
+// 12.6 us.  With more tiles than half of the pairs nothing changes.
 #include <cuda.h>
 
 #include <type_traits>
@@ -33,7 +39,7 @@ constexpr int kEpiWarps = 8;
 constexpr int kThreads = 64 + 32 * kEpiWarps;
 
 struct Params {
-  int N;                    // output channels
+  int N;                    // output channels; a pair computes the columns blockIdx.y * (tile width) .. of them
   int groups;               // utterances
   const int32_t* offsets;   // cu[0..groups]: packed output frame offsets
   int conv_f2;              // output positions per output frame
@@ -106,6 +112,7 @@ conv2_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   constexpr uint32_t kIdesc = ptx::umma_idesc_f16(kBf16, 2 * BM, kNI);
   constexpr uint32_t kTmemCols = N;
   const uint32_t cta_rank = ptx::cluster_ctarank();
+  const int n0 = static_cast<int>(blockIdx.y) * N;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -178,7 +185,7 @@ conv2_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 #pragma unroll
             for (int j = 0; j < kHalves; ++j)
               ptx::tma_load_3d_pair(sB + stage * S::kBBytes + j * S::kBHalfBytes, &tmap_b, kb * BK,
-                                    j * kNI + static_cast<int>(cta_rank) * (kNI / 2), 0, lead_full);
+                                    n0 + j * kNI + static_cast<int>(cta_rank) * (kNI / 2), 0, lead_full);
           }
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
@@ -226,7 +233,7 @@ conv2_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     const int slice = ew >> 2;
     const uint32_t lane_base = static_cast<uint32_t>(q * 32) << 16;
     const int tile_row = q * 32 + lane;
-    const T* bias = static_cast<const T*>(p.bias);
+    const T* bias = p.bias ? static_cast<const T*>(p.bias) + n0 : nullptr;
     constexpr int kCols = N / 2;                   // columns per warp
     uint32_t tile_phase = 0;
     bool ok = true;
@@ -240,7 +247,7 @@ conv2_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       ptx::tc_fence_after_sync();
       const int64_t row = mine.out_row + tile_row;
       const bool row_ok = have && tile_row < p.conv_tpt * p.conv_f2 && row < mine.row_end;
-      T* drow = static_cast<T*>(p.D) + row * N;
+      T* drow = static_cast<T*>(p.D) + row * p.N + n0;
 #pragma unroll 1
       for (int c0 = 0; c0 < kCols; c0 += 32) {
         const int col = slice * kCols + c0;
@@ -295,7 +302,9 @@ template <int N> struct StagesFor;
 template <> struct StagesFor<512> { static constexpr int v = 4; };   // 48 KB per stage
 template <> struct StagesFor<256> { static constexpr int v = 6; };   // 32 KB per stage
 template <> struct StagesFor<128> { static constexpr int v = 8; };   // 24 KB per stage
+template <> struct StagesFor<64> { static constexpr int v = 10; };   // 20 KB per stage
 
+// N: columns of a pair's tile, a divisor of p.N.
 template <typename T, int N>
 int launch(const CUtensorMap& ta, const void* w2, int64_t K, const Params& p, int64_t max_items, int dtype, cudaStream_t s) {
   constexpr int kStages = StagesFor<N>::v;
@@ -306,15 +315,15 @@ int launch(const CUtensorMap& ta, const void* w2, int64_t K, const Params& p, in
   if (e != cudaSuccess) return set_error(OASR_ERR_CUDA, "subsample_conv2: cannot reserve %d bytes of shared memory: %s",
                                          S::kDynamic, cudaGetErrorString(e));
   CUtensorMap tb;
-  uint64_t bdims[3] = {(uint64_t)K, (uint64_t)N, 1};
-  uint64_t bstr[3] = {0, (uint64_t)K * 2, (uint64_t)K * 2 * (uint64_t)N};
+  uint64_t bdims[3] = {(uint64_t)K, (uint64_t)p.N, 1};
+  uint64_t bstr[3] = {0, (uint64_t)K * 2, (uint64_t)K * 2 * (uint64_t)p.N};
   uint32_t bbox[3] = {BK, (uint32_t)(S::kNI / 2), 1};
   if (int rc = make_tensor_map(&tb, tma_dtype(dtype), 3, w2, bdims, bstr, bbox)) return rc;
   int64_t clusters = sm_count() / 2;
   const int64_t pairs = (max_items + 1) / 2;
   if (pairs < clusters) clusters = pairs;
   if (clusters < 1) clusters = 1;
-  launch_pdl(kern, dim3(static_cast<unsigned>(2 * clusters)), dim3(kThreads), S::kDynamic, s, ta, tb, p);
+  launch_pdl(kern, dim3(static_cast<unsigned>(2 * clusters), static_cast<unsigned>(p.N / N)), dim3(kThreads), S::kDynamic, s, ta, tb, p);
   return check_launch("subsample_conv2 (CTA pairs) launch");
 }
 
@@ -327,11 +336,17 @@ int run(const CUtensorMap& ta, void* out, const void* w2, const void* bias, cons
   p.num_k_blocks = 9 * p.conv_cblocks;
   p.D = out; p.bias = bias; p.status = device_status_ptr();
   const int64_t max_items = total_frames / tpt + B;   // upper bound of the conv tiles (the kernel finds the exact end)
+  // Few tiles: a tile's columns are halved as long as every half still finds a free pair of SMs (a second round would cost
+  // what the halving saves).
+  const int64_t pairs = (max_items + 1) / 2;
+  int64_t tile = N;
+  while (tile > 64 && pairs * (N / tile) * 2 <= sm_count() / 2) tile /= 2;
   return OB_DISPATCH_HALF(dtype, T, [&]() -> int {
-    switch (N) {
+    switch (tile) {
       case 512: return launch<T, 512>(ta, w2, 9 * C, p, max_items, dtype, s);
       case 256: return launch<T, 256>(ta, w2, 9 * C, p, max_items, dtype, s);
-      default: return launch<T, 128>(ta, w2, 9 * C, p, max_items, dtype, s);
+      case 128: return launch<T, 128>(ta, w2, 9 * C, p, max_items, dtype, s);
+      default: return launch<T, 64>(ta, w2, 9 * C, p, max_items, dtype, s);
     }
   });
 }

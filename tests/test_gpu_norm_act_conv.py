@@ -321,3 +321,40 @@ def test_packed_depthwise_conv_kernels_agree_with_each_other_and_with_fp32(K, ca
         for path in (2, 0):
             err = (outs[path][a:a + n].cpu() - want).abs().max().item()
             assert err < 3e-2 * max(1.0, want.abs().max().item()), (path, s, n, err)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("C,N,frames", [(512, 512, [1]), (512, 512, [6]), (512, 512, [7, 0, 5]), (512, 512, [102]), (512, 512, [108]), (512, 512, [216]),
+                                        (512, 512, [438]), (512, 512, [444]), (512, 512, [16] * 12), (64, 256, [13, 40]), (128, 128, [9, 1, 3])])
+def test_subsampling_second_conv_at_every_tile_width(C, N, frames, dtype):
+    """Few tiles deal their output columns to several pairs of SMs: every width, the last sizes before each line and partial
+    tiles, against fp64.  Bound: one rounding to 16 bits of the result and K fp32 additions of the products."""
+    from oasr_b200 import fused
+
+    g = torch.Generator(device="cuda").manual_seed(sum(frames) + C)
+    F1, F2, B = 39, 19, len(frames)
+    T1 = 2 * max(frames) + 1
+    x = torch.randn(B, T1, F1, C, generator=g, device="cuda").to(dtype)
+    w = (torch.randn(N, 3, 3, C, generator=g, device="cuda") * (9 * C) ** -0.5).to(dtype)
+    b = (torch.randn(N, generator=g, device="cuda") * 0.1).to(dtype)
+    split = torch.zeros(B, (T1 + 1) // 2, 4, (F1 + 1) // 2, C, dtype=dtype, device="cuda")
+    for plane in range(4):
+        part = x[:, plane >> 1::2, plane & 1::2]
+        split[:, :part.size(1), plane, :part.size(2)] = part
+    cu = torch.tensor([0] + list(np.cumsum(frames)), dtype=torch.int32, device="cuda")
+    got = fused.subsample_conv2(split, T1, F1, w, b, cu, sum(frames)).view(-1, F2, N).double()
+    assert ob.device_status() == 0
+    at = 0
+    for i, n in enumerate(frames):
+        want = b.double().expand(n, F2, N).clone()
+        size = b.double().abs().expand(n, F2, N).clone()
+        for kh in range(3):
+            for kw in range(3):
+                rows = x[i, kh:kh + 2 * n - 1:2, kw:kw + 2 * F2 - 1:2].double() if n else x[i, :0, :F2].double()
+                want += rows @ w[:, kh, kw].double().t()
+                size += rows.abs() @ w[:, kh, kw].double().abs().t()
+        want = want.relu()
+        eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+        bound = eps * want.abs() + 9 * C * 2.0 ** -24 * size
+        assert bool(((got[at:at + n] - want).abs() <= bound).all()), (i, ((got[at:at + n] - want).abs() - bound).max().item())
+        at += n
