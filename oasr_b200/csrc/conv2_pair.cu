@@ -18,8 +18,8 @@
 // A few utterances or streams fill few pairs, and then the main loop of one tile over all N channels is all of the time: 72
 // blocks of 1024 tensor clocks for N = 512.  So where pairs are free they share a tile's columns, down to 64 each (grid.y;
 // the order of K, hence every bit, stays): N = 512, 1 to 37 output frames 50 -> 22 us (256 columns 27, 128 columns 22.5; a
-// K block then costs its operands' trip from L2, not its products), 16 streams of 16 frames 57 -> 33 us; N = 256 16.5 ->
-// 12.6 us.  With more tiles than half of the pairs nothing changes.
+// K block then costs its operands' trip from L2, not its products), 16 streams of 16 frames 57 -> 31 us; N = 256 16.5 ->
+// 13 us.  With more tiles than half of the pairs nothing changes.
 #include <cuda.h>
 
 #include <type_traits>
@@ -82,22 +82,37 @@ struct Item {
   bool valid;
 };
 
-// w-th conv tile in (utterance, frame block) order; invalid past the last one.
+// w-th conv tile in (utterance, frame block) order; invalid past the last one.  By a whole warp, a lane per utterance: one
+// after the other, each of a full step's 256 utterances cost an L2 or L1 latency before the tile's first load could go out.
+// N 512, 16 frames each: 256 utterances 476 -> 319 us, 64 121 -> 104, 37 65 -> 57; N 256: 256 utterances 273 -> 104 us, 64 of 249
+// frames 391 -> 318.
 __device__ __forceinline__ Item find_item(const Params& p, int64_t w) {
+  const int lane = threadIdx.x & 31;
   Item it{0, 0, 0, 0, false};
-  for (int b = 0; b < p.groups; ++b) {
-    const int lo = p.offsets[b], hi = p.offsets[b + 1];
+  for (int base = 0; base < p.groups; base += 32) {
+    const int b = base + lane;
+    const int lo = b < p.groups ? p.offsets[b] : 0, hi = b < p.groups ? p.offsets[b + 1] : 0;
     const int frames = hi - lo;
     const int tiles = (frames + p.conv_tpt - 1) / p.conv_tpt;
-    if (w < tiles) {
-      it.b = b;
-      it.t0 = static_cast<int>(w) * p.conv_tpt;
-      it.out_row = static_cast<int64_t>(lo + it.t0) * p.conv_f2;
-      it.row_end = static_cast<int64_t>(lo + min(it.t0 + p.conv_tpt, frames)) * p.conv_f2;
+    int upto = tiles;                                      // tiles of these 32 utterances up to and with this one
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const uint32_t reach = __ballot_sync(0xffffffffu, w < upto);
+    if (reach) {
+      const int at = __ffs(reach) - 1;
+      const int lo_at = __shfl_sync(0xffffffffu, lo, at), frames_at = __shfl_sync(0xffffffffu, frames, at);
+      const int before = __shfl_sync(0xffffffffu, upto - tiles, at);
+      it.b = base + at;
+      it.t0 = static_cast<int>(w - before) * p.conv_tpt;
+      it.out_row = static_cast<int64_t>(lo_at + it.t0) * p.conv_f2;
+      it.row_end = static_cast<int64_t>(lo_at + min(it.t0 + p.conv_tpt, frames_at)) * p.conv_f2;
       it.valid = true;
       return it;
     }
-    w -= tiles;
+    w -= __shfl_sync(0xffffffffu, upto, 31);
   }
   return it;
 }
@@ -189,6 +204,7 @@ conv2_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           }
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
+        ok = __all_sync(0xffffffffu, ok);                  // the warp goes on, or gives up, as a whole (find_item)
       }
       if (!ok && issuer && p.status) atomicOr(p.status, kStatusGemmProducer);
     }
@@ -202,7 +218,8 @@ conv2_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       bool ok = true;
       for (int64_t w = first; ok; w += num_clusters) {
         if (!find_item(p, 2 * w).valid) break;
-        if (!ptx::mbar_wait(tempty_bar, acc_phase ^ 1u, abort_flag)) { ok = false; break; }
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait(tempty_bar, acc_phase ^ 1u, abort_flag));
+        if (!ok) break;
         ptx::tc_fence_after_sync();
         for (int kb = 0; kb < p.num_k_blocks; ++kb) {
           if (!ptx::mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
@@ -220,6 +237,7 @@ conv2_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           }
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
+        ok = __all_sync(0xffffffffu, ok);
         if (ok && issuer) ptx::umma_commit_pair(tfull_bar, 3);
         acc_phase ^= 1u;
       }
@@ -242,7 +260,8 @@ conv2_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       if (!lead.valid) break;
       Item mine = cta_rank == 0 ? lead : find_item(p, 2 * w + 1);
       const bool have = mine.valid;
-      if (!ptx::mbar_wait(tfull_bar, tile_phase, abort_flag)) { ok = false; break; }
+      ok = __all_sync(0xffffffffu, ptx::mbar_wait(tfull_bar, tile_phase, abort_flag));
+      if (!ok) break;
       tile_phase ^= 1u;
       ptx::tc_fence_after_sync();
       const int64_t row = mine.out_row + tile_row;

@@ -325,10 +325,11 @@ def test_packed_depthwise_conv_kernels_agree_with_each_other_and_with_fp32(K, ca
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("C,N,frames", [(512, 512, [1]), (512, 512, [6]), (512, 512, [7, 0, 5]), (512, 512, [102]), (512, 512, [108]), (512, 512, [216]),
-                                        (512, 512, [438]), (512, 512, [444]), (512, 512, [16] * 12), (64, 256, [13, 40]), (128, 128, [9, 1, 3])])
+                                        (512, 512, [438]), (512, 512, [444]), (512, 512, [16] * 12), (64, 256, [13, 40]), (128, 128, [9, 1, 3]),
+                                        (64, 256, [7, 0, 1] * 11), (64, 512, [0] * 31 + [6] + [0] * 33 + [20, 3])])
 def test_subsampling_second_conv_at_every_tile_width(C, N, frames, dtype):
     """Few tiles deal their output columns to several pairs of SMs: every width, the last sizes before each line and partial
-    tiles, against fp64.  Bound: one rounding to 16 bits of the result and K fp32 additions of the products."""
+    tiles; more utterances than lanes look for a tile at a time, empty ones among them; against fp64.  Bound: one rounding to 16 bits of the result and K fp32 additions of the products."""
     from oasr_b200 import fused
 
     g = torch.Generator(device="cuda").manual_seed(sum(frames) + C)
