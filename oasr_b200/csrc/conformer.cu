@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "fmha_chunk_append.cuh"
 #include "gemm_small.cuh"
 
 namespace ob {
@@ -468,9 +469,13 @@ int oasr_b200_conformer_chunk_paged(const oasr_b200_conformer_model* model, cons
     } else {
       OB_CHUNK_LINEAR_H("qkv4", 2.0 * M * 3 * d * d, w.qkv4, l.qkv4_w, l.qkv4_b, l, 2, 4 * d, OASR_ACT_NONE);
     }
-    if (kv_scales) {   // fp8 pages: per-head scales of this layer, K then V
-      const float* ks = kv_scales + static_cast<int64_t>(i) * 2 * m.heads;
-      const float* vs = ks + m.heads;
+    const float* ks = kv_scales ? kv_scales + static_cast<int64_t>(i) * 2 * m.heads : nullptr;   // fp8 pages: scales of K, then V
+    const float* vs = ks ? ks + m.heads : nullptr;
+    if (fmha_chunk_append::applies(B, m.heads, T, block_size, blocks_per_seq, k_pools[i], v_pools[i])) {   // few streams: in one kernel
+      OB_STEP("fmha_paged_relpos", 0, fmha_chunk_append::run(w.att, w.qkv4, k_pools[i], v_pools[i], ks, vs,
+                                       static_cast<const uint8_t*>(m.pos_proj) + i * d * 2, m.pos_proj_rows, L * d, pos_start, block_table,
+                                       total_seqlens, B, T, m.heads, blocks_per_seq, block_size, num_blocks, scale, dt, static_cast<cudaStream_t>(stream), cache_seqlens));
+    } else if (kv_scales) {
       OB_STEP("paged_kv_write", 0, oasr_b200_paged_kv_write_fp8(k_pools[i], v_pools[i], w.qkv4 + 2 * d * 2, w.qkv4 + 3 * d * 2,
                                        ks, vs, block_table, cache_seqlens, B, m.heads, T, 64, T * 4 * d, 64, 4 * d,
                                        blocks_per_seq, block_size, num_blocks, dt, stream));

@@ -1,0 +1,18 @@
+// Host interface of the streaming-chunk attention of few streams (fmha_chunk_append.cu): paged_kv_write(_fp8) and
+// fmha_paged_relpos(_fp8) in one kernel.
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace ob {
+namespace fmha_chunk_append {
+
+bool applies(int64_t B, int64_t H, int64_t Tq, int64_t block_size, int64_t blocks_per_seq, const void* k_pool, const void* v_pool);
+// The chunk's keys and values go to the pages from position append_at[b] on; k_scale null: 16-bit pages.
+int run(void* out, const void* qkv4, void* k_pool, void* v_pool, const float* k_scale, const float* v_scale, const void* pos,
+        int64_t pos_rows, int64_t pos_stride, const int32_t* pos_start, const int32_t* block_table, const int32_t* seqlens,
+        int64_t B, int64_t Tq, int64_t H, int64_t blocks_per_seq, int64_t block_size, int64_t num_blocks, double scale,
+        int dtype, cudaStream_t stream, const int32_t* append_at);
+
+}  // namespace fmha_chunk_append
+}  // namespace ob

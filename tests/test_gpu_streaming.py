@@ -187,3 +187,35 @@ def test_streaming_with_8bit_linears_reaches_the_cosine_gate_against_the_16_bit_
     agree = (a.argmax(-1) == b.argmax(-1)).float().mean().item()
     print(f"{mode} streaming Linears vs 16-bit: cosine {cos:.6f}, argmax agreement {agree:.4f}, max-abs {(a - b).abs().max().item():.3e}")
     assert cos >= 0.999, cos
+
+
+@pytest.mark.parametrize("history,block_size", [(64, 16), (48, 16)])
+def test_appended_pages_equal_the_page_write(history, block_size):
+    """The chunk kernel appends the chunk's keys and values itself.  The first layer's do not depend on attention: its pages are
+    bit-equal to those of the path that writes them with a launch of its own, for slices that hold cached keys only, new ones
+    only and both, with eviction; fp8 pages hold the rounded codes of the 16-bit ones."""
+    from oasr_b200 import tunables
+
+    case = cases.STREAM_CASE
+    cfg, chunk = case["cfg"], case["chunk_size"]
+    model = ConformerCTC(_cfg(cfg), OC.init_params(cfg, case["weight_seed"], case["perturb"]))
+    feats = cases.make_stream_features(case).cuda()
+    scales = torch.rand(cfg.layers, 2, cfg.heads, device="cuda") * 0.02 + 0.01
+    new = lambda **kw: model.new_streaming_cache(3, history, chunk_frames=chunk, block_size=block_size, seed=2, **kw)
+    a, b, c = new(), new(), new(kv_scales=scales)
+    for i in range(case["chunks"]):
+        xs = feats[:, i * case["step"]: i * case["step"] + case["window"]]
+        got = model.forward_chunk_paged(xs, [2, 0], a)
+        model.forward_chunk_paged(xs, [2, 0], c)
+        tunables.set("fmha_chunk_path", 0)
+        try:
+            want = model.forward_chunk_paged(xs, [2, 0], b)
+        finally:
+            tunables.set("fmha_chunk_path", 1)
+        assert ob.device_status() == 0
+        assert (got - want).abs().max().item() < 2e-2
+        for pool, ref, codes, which in ((a.k_pool, b.k_pool, c.k_pool, 0), (a.v_pool, b.v_pool, c.v_pool, 1)):
+            assert torch.equal(pool[0], ref[0])
+            inv = (1.0 / scales[0, which]).view(1, 1, -1, 1)
+            want8 = (pool[0].float() * inv).clamp(-448, 448).to(torch.float8_e4m3fn).view(torch.uint8)
+            assert torch.equal(codes[0], want8)
