@@ -856,6 +856,27 @@ OASR_API int oasr_b200_conformer_chunk_paged(const oasr_b200_conformer_model* mo
                                              int64_t workspace_bytes, float* log_probs /*nullable*/,
                                              int32_t* argmax /*nullable*/, void* stream);
 
+/* The same step with the page write and the attention of every layer as two
+ * launches whatever the number of streams.  oasr_b200_conformer_chunk_paged
+ * runs both as one kernel while few streams leave the GPU room, and that
+ * kernel adds the keys in another order.  For callers whose results must not
+ * depend on which side of that line they are: the fp8 page scales are
+ * calibrated with it, since every later session rests on them. */
+OASR_API int oasr_b200_conformer_chunk_paged_split(const oasr_b200_conformer_model* model,
+                                                   const void* rows, int64_t B, int64_t T,
+                                                   void* const* k_pools /*host*/,
+                                                   void* const* v_pools /*host*/,
+                                                   const int32_t* block_table,
+                                                   const int32_t* cache_seqlens,
+                                                   const int32_t* total_seqlens,
+                                                   const int32_t* pos_start, int64_t blocks_per_seq,
+                                                   int64_t block_size, int64_t num_blocks,
+                                                   const float* kv_scales /*nullable: fp8 pages, fp32 (num_layers, 2, heads) K then V scales*/,
+                                                   void* cnn_state, int64_t num_slots,
+                                                   const int64_t* slot_ids, void* workspace,
+                                                   int64_t workspace_bytes, float* log_probs /*nullable*/,
+                                                   int32_t* argmax /*nullable*/, void* stream);
+
 /* This entry point has no counterpart in the reference.  It does what
  * oasr_b200_conformer_encode_packed does for callers that must not allocate
  * device memory (a plugin inside a process whose own pool already owns the

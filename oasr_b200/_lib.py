@@ -154,6 +154,7 @@ _SIGNATURES["oasr_b200_conformer_encode_packed"] = [POINTER(ConformerModel), P, 
 _SIGNATURES["oasr_b200_conformer_encode_packed_noalloc"] = [POINTER(ConformerModel), P, P, P, I, I, I, P, P, P]
 _SIGNATURES["oasr_b200_conformer_chunk_paged"] = [POINTER(ConformerModel), P, I, I, POINTER(c_void_p), POINTER(c_void_p),
                                                  P, P, P, P, I, I, I, P, P, I, P, P, I, P, P, P]
+_SIGNATURES["oasr_b200_conformer_chunk_paged_split"] = _SIGNATURES["oasr_b200_conformer_chunk_paged"]
 _SIGNATURES["oasr_b200_profile_enable"] = [c_int]
 _SIGNATURES["oasr_b200_profile_get"] = [c_int, POINTER(c_char_p), POINTER(c_double), POINTER(c_double)]
 

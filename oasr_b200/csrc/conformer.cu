@@ -389,14 +389,12 @@ int64_t oasr_b200_conformer_chunk_workspace_bytes(const oasr_b200_conformer_mode
   return ob::carve_chunk(*model, B, T, nullptr).bytes;
 }
 
-int oasr_b200_conformer_chunk_paged(const oasr_b200_conformer_model* model, const void* rows, int64_t B, int64_t T,
-                                    void* const* k_pools, void* const* v_pools, const int32_t* block_table,
-                                    const int32_t* cache_seqlens, const int32_t* total_seqlens,
-                                    const int32_t* pos_start, int64_t blocks_per_seq, int64_t block_size,
-                                    int64_t num_blocks, const float* kv_scales, void* cnn_state, int64_t num_slots,
-                                    const int64_t* slot_ids,
-                                    void* workspace, int64_t workspace_bytes, float* log_probs, int32_t* argmax,
-                                    void* stream) {
+// merged: attention that appends the chunk's keys and values itself, where it applies (few streams)
+static int chunk_paged(const oasr_b200_conformer_model* model, const void* rows, int64_t B, int64_t T,
+                       void* const* k_pools, void* const* v_pools, const int32_t* block_table, const int32_t* cache_seqlens,
+                       const int32_t* total_seqlens, const int32_t* pos_start, int64_t blocks_per_seq, int64_t block_size,
+                       int64_t num_blocks, const float* kv_scales, void* cnn_state, int64_t num_slots, const int64_t* slot_ids,
+                       void* workspace, int64_t workspace_bytes, float* log_probs, int32_t* argmax, void* stream, bool merged) {
   using namespace ob;
   OB_REQUIRE(model && model->layers, OASR_ERR_INVALID, "conformer_chunk_paged: null model");
   const oasr_b200_conformer_model& m = *model;
@@ -471,7 +469,7 @@ int oasr_b200_conformer_chunk_paged(const oasr_b200_conformer_model* model, cons
     }
     const float* ks = kv_scales ? kv_scales + static_cast<int64_t>(i) * 2 * m.heads : nullptr;   // fp8 pages: scales of K, then V
     const float* vs = ks ? ks + m.heads : nullptr;
-    if (fmha_chunk_append::applies(B, m.heads, T, block_size, blocks_per_seq, k_pools[i], v_pools[i])) {   // few streams: in one kernel
+    if (merged && fmha_chunk_append::applies(B, m.heads, T, block_size, blocks_per_seq, k_pools[i], v_pools[i])) {   // few streams: in one kernel
       OB_STEP("fmha_paged_relpos", 0, fmha_chunk_append::run(w.att, w.qkv4, k_pools[i], v_pools[i], ks, vs,
                                        static_cast<const uint8_t*>(m.pos_proj) + i * d * 2, m.pos_proj_rows, L * d, pos_start, block_table,
                                        total_seqlens, B, T, m.heads, blocks_per_seq, block_size, num_blocks, scale, dt, static_cast<cudaStream_t>(stream), cache_seqlens));
@@ -514,6 +512,30 @@ int oasr_b200_conformer_chunk_paged(const oasr_b200_conformer_model* model, cons
                                        argmax, stream, inner));
   }
   return OASR_OK;
+}
+
+int oasr_b200_conformer_chunk_paged(const oasr_b200_conformer_model* model, const void* rows, int64_t B, int64_t T,
+                                    void* const* k_pools, void* const* v_pools, const int32_t* block_table,
+                                    const int32_t* cache_seqlens, const int32_t* total_seqlens,
+                                    const int32_t* pos_start, int64_t blocks_per_seq, int64_t block_size,
+                                    int64_t num_blocks, const float* kv_scales, void* cnn_state, int64_t num_slots,
+                                    const int64_t* slot_ids,
+                                    void* workspace, int64_t workspace_bytes, float* log_probs, int32_t* argmax,
+                                    void* stream) {
+  return chunk_paged(model, rows, B, T, k_pools, v_pools, block_table, cache_seqlens, total_seqlens, pos_start, blocks_per_seq, block_size,
+                     num_blocks, kv_scales, cnn_state, num_slots, slot_ids, workspace, workspace_bytes, log_probs, argmax, stream, true);
+}
+
+int oasr_b200_conformer_chunk_paged_split(const oasr_b200_conformer_model* model, const void* rows, int64_t B, int64_t T,
+                                          void* const* k_pools, void* const* v_pools, const int32_t* block_table,
+                                          const int32_t* cache_seqlens, const int32_t* total_seqlens,
+                                          const int32_t* pos_start, int64_t blocks_per_seq, int64_t block_size,
+                                          int64_t num_blocks, const float* kv_scales, void* cnn_state, int64_t num_slots,
+                                          const int64_t* slot_ids,
+                                          void* workspace, int64_t workspace_bytes, float* log_probs, int32_t* argmax,
+                                          void* stream) {
+  return chunk_paged(model, rows, B, T, k_pools, v_pools, block_table, cache_seqlens, total_seqlens, pos_start, blocks_per_seq, block_size,
+                     num_blocks, kv_scales, cnn_state, num_slots, slot_ids, workspace, workspace_bytes, log_probs, argmax, stream, false);
 }
 
 }  // extern "C"

@@ -336,21 +336,23 @@ class ConformerCTC:
     def calibrate_kv_scales(self, windows, chunk_frames: int = 16, margin: float = 1.0) -> torch.Tensor:
         """Per (layer, head) fp8 scales ``amax / 448`` of the keys and values seen while the feature windows
         ``windows`` (an iterable of ``(B, window, F)`` tensors, consecutive chunks of the same B streams) run through
-        a 16-bit cache.  Returns ``(layers, 2, heads)`` fp32."""
+        a 16-bit cache.  Returns ``(layers, 2, heads)`` fp32.  The bits of the scales do not depend on whether B is small
+        enough for the attention kernel of few streams."""
         c = self.cfg
         windows = list(windows)
         B = windows[0].size(0)
         cache = self.new_streaming_cache(B, max_past_frames=chunk_frames * len(windows), chunk_frames=chunk_frames, seed=None)
         for xs in windows:
-            self.forward_chunk_paged(xs.to(self.device), list(range(B)), cache)
+            self._chunk_step(xs.to(self.device), list(range(B)), cache, "oasr_b200_conformer_chunk_paged_split")
         k = cache.k_pool.float().abs().amax(dim=(1, 2, 4))     # (L, H)
         v = cache.v_pool.float().abs().amax(dim=(1, 2, 4))
         scales = torch.stack([k, v], dim=1) * (margin / 448.0)
         return torch.clamp(scales, min=1e-8).contiguous()
 
-    def _chunk_launch(self, xs: torch.Tensor, cache, table, cached, total, pos_start, slot_ids):
+    def _chunk_launch(self, xs: torch.Tensor, cache, table, cached, total, pos_start, slot_ids,
+                      entry: str = "oasr_b200_conformer_chunk_paged"):
         """The device work of one streaming step on the current stream: subsampling convolutions + ONE native call
-        (oasr_b200_conformer_chunk_paged).  No host synchronisation, no host-to-device copy: capturable."""
+        (``entry``).  No host synchronisation, no host-to-device copy: capturable."""
         import ctypes
 
         from . import _lib
@@ -371,7 +373,7 @@ class ConformerCTC:
         kp, vp = cache.pool_pointers()
         log_probs = torch.empty(B, T, self.cfg.vocab_padded, device=xs.device, dtype=torch.float32)
         argmax = torch.empty(B, T, device=xs.device, dtype=torch.int32)
-        _lib.call("oasr_b200_conformer_chunk_paged", ctypes.byref(self._native_model), _p(rows), B, T, kp, vp, _p(table),
+        _lib.call(entry, ctypes.byref(self._native_model), _p(rows), B, T, kp, vp, _p(table),
                   _p(cached), _p(total), _p(pos_start), table.size(1), cache.block_size, cache.num_blocks,
                   _p(cache.kv_scales), _p(cache.cnn_state), cache.max_streams, _p(slot_ids), ctypes.c_void_p(ws.data_ptr() + off),
                   ws.numel() - off, _p(log_probs), _p(argmax),
@@ -389,6 +391,10 @@ class ConformerCTC:
         oasr/models/conformer/model.py:913-1023, oasr/models/base.py:763-777).  K/V pages and the conv
         left context in ``cache`` are updated in place; page allocation, eviction and the commit of
         ``cache_seqlens`` happen around the single native call."""
+        log_probs, argmax = self._chunk_step(xs, slots, cache)
+        return (log_probs, argmax) if return_argmax else log_probs
+
+    def _chunk_step(self, xs: torch.Tensor, slots, cache, entry: str = "oasr_b200_conformer_chunk_paged"):
         import ctypes
 
         from . import _lib
@@ -410,9 +416,9 @@ class ConformerCTC:
         if len(slots) != B:
             raise RuntimeError(f"{B} feature windows for {len(slots)} slots")
         table, cached, total, pos_start, slot_ids = cache.prepare(slots)
-        log_probs, argmax = self._chunk_launch(xs, cache, table, cached, total, pos_start, slot_ids)
+        log_probs, argmax = self._chunk_launch(xs, cache, table, cached, total, pos_start, slot_ids, entry)
         cache.commit(slots)
-        return (log_probs, argmax) if return_argmax else log_probs
+        return log_probs, argmax
 
     def _forward(self, features: torch.Tensor, lengths, padded_semantics: bool, padded_output: bool,
                  return_argmax: bool, tokens_only: bool = False):

@@ -219,3 +219,17 @@ def test_appended_pages_equal_the_page_write(history, block_size):
             inv = (1.0 / scales[0, which]).view(1, 1, -1, 1)
             want8 = (pool[0].float() * inv).clamp(-448, 448).to(torch.float8_e4m3fn).view(torch.uint8)
             assert torch.equal(codes[0], want8)
+
+
+def test_calibrated_scales_do_not_depend_on_the_attention_kernel_of_few_streams():
+    """The most streams that the attention kernel of few streams takes, and one more: the further stream repeats the first
+    one, so the largest keys and values are the same and the fp8 scales must be too, bit for bit."""
+    cfg = _cfg(OC.CONFIG3)
+    model = ConformerCTC(cfg, OC.init_params(OC.CONFIG3, 1234))
+    few = 2 * torch.cuda.get_device_properties(0).multi_processor_count // cfg.heads
+    g = torch.Generator(device="cuda").manual_seed(29)
+    windows = [torch.randn(few, 67, 80, generator=g, device="cuda") for _ in range(4)]
+    want = model.calibrate_kv_scales([torch.cat((w, w[:1])) for w in windows])
+    got = model.calibrate_kv_scales(windows)
+    assert ob.device_status() == 0
+    assert torch.equal(got, want)
