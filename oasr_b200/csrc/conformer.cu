@@ -407,6 +407,12 @@ static int chunk_paged(const oasr_b200_conformer_model* model, const void* rows,
              OASR_ERR_INVALID, "conformer_chunk_paged: null pointer argument");
   OB_REQUIRE(m.pos_proj && m.pos_proj_rows > 0, OASR_ERR_INVALID,
              "conformer_chunk_paged: the model has no projected positional table (pos_proj)");
+  OB_REQUIRE(is_aligned(m.pos_proj, 16), OASR_ERR_ALIGN, "conformer_chunk_paged: pos_proj must be 16-byte aligned");
+  OB_REQUIRE(blocks_per_seq > 0 && block_size > 0 && num_blocks > 0, OASR_ERR_INVALID,
+             "conformer_chunk_paged: bad page geometry (%lld pages of %lld frames per stream, %lld in all)", (long long)blocks_per_seq,
+             (long long)block_size, (long long)num_blocks);
+  for (int64_t i = 0; i < m.num_layers; ++i)
+    OB_REQUIRE(k_pools[i] && v_pools[i], OASR_ERR_INVALID, "conformer_chunk_paged: null page pool of layer %lld", (long long)i);
   OB_REQUIRE(is_aligned(workspace, 256), OASR_ERR_ALIGN, "conformer_chunk_paged: workspace must be 256-byte aligned");
   const int qk = m.quant_kind;
   OB_REQUIRE(qk == 0 || qk == OASR_Q8_FP8_E4M3 || qk == OASR_Q8_INT8, OASR_ERR_INVALID, "conformer_chunk_paged: bad quant_kind %d", qk);
