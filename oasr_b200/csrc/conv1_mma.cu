@@ -27,6 +27,7 @@
 #include "common.cuh"
 #include "device_status.cuh"
 #include "sm100_ptx.cuh"
+#include "smem_limit.cuh"
 #include "tma_host.cuh"
 
 namespace ob {
@@ -346,13 +347,10 @@ int launch(void* out, const Params& p, int dtype, cudaStream_t s) {
   using S = Smem<C>;
   static_assert(S::kDynamic <= 232448, "shared memory budget of one CTA");
   auto kern = conv1_mma_kernel<T, C>;
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kDynamic);
-    if (e != cudaSuccess) return set_error(OASR_ERR_CUDA, "subsample_conv1_s2d: cannot reserve %d bytes of shared memory: %s",
-                                           S::kDynamic, cudaGetErrorString(e));
-    attr_done = true;
-  }
+  static SmemLimit smem_limit;
+  const cudaError_t e = smem_limit.raise(kern, S::kDynamic);
+  if (e != cudaSuccess) return set_error(OASR_ERR_CUDA, "subsample_conv1_s2d: cannot reserve %d bytes of shared memory: %s",
+                                         S::kDynamic, cudaGetErrorString(e));
   CUtensorMap to;
   const uint64_t slots = static_cast<uint64_t>(p.TH) * 4 * p.FH;
   uint64_t dims[3] = {static_cast<uint64_t>(C), slots, static_cast<uint64_t>(p.B)};

@@ -37,6 +37,7 @@
 #include "common.cuh"
 #include "device_status.cuh"
 #include "sm100_ptx.cuh"
+#include "smem_limit.cuh"
 #include "tma_host.cuh"
 
 namespace ob {
@@ -605,14 +606,11 @@ template <typename T, int D, int kAtoms, bool kGeneral>
 int launch_k(const Maps& maps, const Params& p, dim3 grid, cudaStream_t s) {
   using S = Smem<D, kAtoms>;
   auto kern = fmha_tcgen05_kernel<T, D, kAtoms, kGeneral>;
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kDynamic);
-    if (e != cudaSuccess)
-      return set_error(OASR_ERR_CUDA, "fmha: cannot reserve %d bytes of shared memory: %s", S::kDynamic,
-                       cudaGetErrorString(e));
-    attr_done = true;
-  }
+  static SmemLimit smem_limit;
+  const cudaError_t e = smem_limit.raise(kern, S::kDynamic);
+  if (e != cudaSuccess)
+    return set_error(OASR_ERR_CUDA, "fmha: cannot reserve %d bytes of shared memory: %s", S::kDynamic,
+                     cudaGetErrorString(e));
   launch_pdl(kern, grid, dim3(kThreads), S::kDynamic, s, maps, p);
   return check_launch("fmha launch");
 }

@@ -23,6 +23,7 @@
 #include "common.cuh"
 #include "device_status.cuh"
 #include "sm100_ptx.cuh"
+#include "smem_limit.cuh"
 #include "tma_host.cuh"
 
 namespace ob {
@@ -376,14 +377,11 @@ bool applies_fp8(int64_t Tq, int64_t block_size, int64_t blocks_per_seq) {
 template <typename T, bool kFp8>
 int launch(const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mp, const Params& p, unsigned grid, cudaStream_t stream) {
   auto kern = fmha_chunk_kernel<T, kFp8>;
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemDynamic);
-    if (e != cudaSuccess)
-      return set_error(OASR_ERR_CUDA, "fmha_paged_relpos: cannot reserve %d bytes of shared memory: %s", kSmemDynamic,
-                       cudaGetErrorString(e));
-    attr_done = true;
-  }
+  static SmemLimit smem_limit;
+  const cudaError_t e = smem_limit.raise(kern, kSmemDynamic);
+  if (e != cudaSuccess)
+    return set_error(OASR_ERR_CUDA, "fmha_paged_relpos: cannot reserve %d bytes of shared memory: %s", kSmemDynamic,
+                     cudaGetErrorString(e));
   launch_pdl(kern, dim3(grid), dim3(kWarps * 32), kSmemDynamic, stream, mk, mv, mp, p);
   return check_launch("fmha_paged_relpos (chunk kernel) launch");
 }

@@ -30,6 +30,7 @@
 #include "device_status.cuh"
 #include "gemm_small.cuh"
 #include "sm100_ptx.cuh"
+#include "smem_limit.cuh"
 #include "tma_host.cuh"
 
 namespace ob {
@@ -915,13 +916,10 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, 
            cudaStream_t s) {
   using S = Smem<BN, kStages>;
   auto kern = gemm_tcgen05_kernel<T, BN, kStages, kSched, kEpi>;
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kDynamic);
-    if (e != cudaSuccess) return set_error(OASR_ERR_CUDA, "gemm: cannot reserve %d bytes of shared memory: %s",
-                                           S::kDynamic, cudaGetErrorString(e));
-    attr_done = true;
-  }
+  static SmemLimit smem_limit;
+  const cudaError_t e = smem_limit.raise(kern, S::kDynamic);
+  if (e != cudaSuccess) return set_error(OASR_ERR_CUDA, "gemm: cannot reserve %d bytes of shared memory: %s",
+                                         S::kDynamic, cudaGetErrorString(e));
   int64_t grid = work_items < sm_count() ? work_items : sm_count();
   if (grid < 1) grid = 1;
   launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(threads_for<kSched, kEpi>()), S::kDynamic, s, ta, tb, td, p);
@@ -933,13 +931,10 @@ int launch_q8(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& t
               cudaStream_t s) {
   using S = Smem<BN, kStages>;
   auto kern = gemm_tcgen05_q8_kernel<T, BN, kStages, kEpi, kKind>;
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kDynamic);
-    if (e != cudaSuccess) return set_error(OASR_ERR_CUDA, "gemm_q8: cannot reserve %d bytes of shared memory: %s",
-                                           S::kDynamic, cudaGetErrorString(e));
-    attr_done = true;
-  }
+  static SmemLimit smem_limit;
+  const cudaError_t e = smem_limit.raise(kern, S::kDynamic);
+  if (e != cudaSuccess) return set_error(OASR_ERR_CUDA, "gemm_q8: cannot reserve %d bytes of shared memory: %s",
+                                         S::kDynamic, cudaGetErrorString(e));
   int64_t grid = work_items < sm_count() ? work_items : sm_count();
   if (grid < 1) grid = 1;
   launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(threads_for<kSchedDense, kEpi>()), S::kDynamic, s, ta, tb, td, p);
@@ -953,13 +948,10 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
                 int64_t work_items, cudaStream_t s) {
   using S = Smem<256, kPairStages, 2>;
   auto kern = gemm_tcgen05_pair_kernel<T, kPairStages, kEpi>;
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kDynamic);
-    if (e != cudaSuccess) return set_error(OASR_ERR_CUDA, "gemm: cannot reserve %d bytes of shared memory: %s",
-                                           S::kDynamic, cudaGetErrorString(e));
-    attr_done = true;
-  }
+  static SmemLimit smem_limit;
+  const cudaError_t e = smem_limit.raise(kern, S::kDynamic);
+  if (e != cudaSuccess) return set_error(OASR_ERR_CUDA, "gemm: cannot reserve %d bytes of shared memory: %s",
+                                         S::kDynamic, cudaGetErrorString(e));
   int64_t clusters = sm_count() / 2;
   if (work_items < clusters) clusters = work_items;
   if (clusters < 1) clusters = 1;
@@ -1330,13 +1322,10 @@ int gemm_dup_first_op(void* D, const void* A, const void* B, const void* bias, i
     if (int rc = make_tensor_map(&td, tma_dtype(dtype), 3, D, ddims, dstr, dbox, CU_TENSOR_MAP_SWIZZLE_64B)) return rc;
     using S = Smem<256, 4>;
     auto kern = gemm_tcgen05_dup_kernel<T>;
-    static bool attr_done = false;
-    if (!attr_done) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kDynamic);
-      if (e != cudaSuccess) return set_error(OASR_ERR_CUDA, "gemm_dup_first: cannot reserve %d bytes of shared memory: %s",
-                                             S::kDynamic, cudaGetErrorString(e));
-      attr_done = true;
-    }
+    static SmemLimit smem_limit;
+    const cudaError_t e = smem_limit.raise(kern, S::kDynamic);
+    if (e != cudaSuccess) return set_error(OASR_ERR_CUDA, "gemm_dup_first: cannot reserve %d bytes of shared memory: %s",
+                                           S::kDynamic, cudaGetErrorString(e));
     const int64_t work = static_cast<int64_t>(p.num_m_tiles) * p.num_n_tiles;
     int64_t grid = work < sm_count() ? work : sm_count();
     if (grid < 1) grid = 1;

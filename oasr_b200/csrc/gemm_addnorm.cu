@@ -38,6 +38,7 @@
 #include "common.cuh"
 #include "device_status.cuh"
 #include "sm100_ptx.cuh"
+#include "smem_limit.cuh"
 #include "tma_host.cuh"
 
 namespace ob {
@@ -582,13 +583,10 @@ int launch(const Call& c, cudaStream_t s) {
   using S = Smem<N, kStages>;
   static_assert(S::kDynamic <= 232448, "shared memory budget of one CTA");
   auto kern = gemm_addnorm_kernel<T, N, kStages>;
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kDynamic);
-    if (e != cudaSuccess) return set_error(OASR_ERR_CUDA, "gemm_add_norm_f32: cannot reserve %d bytes of shared memory: %s",
-                                           S::kDynamic, cudaGetErrorString(e));
-    attr_done = true;
-  }
+  static SmemLimit smem_limit;
+  const cudaError_t e = smem_limit.raise(kern, S::kDynamic);
+  if (e != cudaSuccess) return set_error(OASR_ERR_CUDA, "gemm_add_norm_f32: cannot reserve %d bytes of shared memory: %s",
+                                         S::kDynamic, cudaGetErrorString(e));
   CUtensorMap ta, tb, th;
   const uint64_t M = static_cast<uint64_t>(c.M), K = static_cast<uint64_t>(c.K);
   {

@@ -34,6 +34,7 @@
 #include "device_status.cuh"
 #include "gemm_small.cuh"
 #include "sm100_ptx.cuh"
+#include "smem_limit.cuh"
 #include "tma_host.cuh"
 
 namespace ob {
@@ -527,12 +528,9 @@ int launch(const Args& a, Params& p, int m_tiles, int dtype, cudaStream_t s) {
   const uint32_t bbox[4] = {BK, (uint32_t)(kGluE ? BN / 2 : BN), kGluE ? 2u : 1u, (uint32_t)p.kg};
   if (int rc = make_tensor_map(&tb, tma_dtype(dtype), 4, a.B, bdims, bstr, bbox)) return rc;
   auto kern = gemm_small_kernel<T, BN, S, kEpi>;
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (e != cudaSuccess) return set_error(OASR_ERR_CUDA, "gemm_small: cannot reserve shared memory: %s", cudaGetErrorString(e));
-    attr_done = true;
-  }
+  static SmemLimit smem_limit;
+  const cudaError_t e = smem_limit.raise(kern, 227 * 1024);
+  if (e != cudaSuccess) return set_error(OASR_ERR_CUDA, "gemm_small: cannot reserve shared memory: %s", cudaGetErrorString(e));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>(n_tiles * S), static_cast<unsigned>(m_tiles));
   cfg.blockDim = dim3(G::kThreads);
