@@ -207,3 +207,46 @@ def test_length_sorted_sweep_through_packs_matches_the_fp32_oracle():
         ids = lp[:n, :cfg.vocab].argmax(-1).cpu().numpy()
         assert results[i] == ConformerCTC._collapse(ids, [n])[0]       # the pack's tokens = this utterance's own tokens
     assert worst_mean <= 2.0e-3
+
+
+@pytest.mark.parametrize("kv", ["bf16", "fp8"])
+def test_streaming_of_many_streams_at_real_width_matches_the_oracle(kv):
+    """More streams than the attention kernel of few streams takes: the step with page write and attention as two launches, at
+    d 512, eager and replayed as a graph, through eviction.  Gates of the test of fewer streams above."""
+    import dataclasses
+
+    chunks, window, step, chunk, max_past = 8, 67, 64, 16, 64
+    ocfg = dataclasses.replace(OC.CONFIG3, layers=4)
+    streams = 2 * torch.cuda.get_device_properties(0).multi_processor_count // ocfg.heads + 3
+    P = OC.init_params(ocfg, 1234)
+    feats = torch.randn(streams, step * (chunks - 1) + window, 80, generator=torch.Generator().manual_seed(18))
+    model = ConformerCTC(_cfg(ocfg), P, device="cuda", dtype=torch.bfloat16)
+    windows = [feats[:, c * step: c * step + window] for c in range(chunks)]
+    scales = model.calibrate_kv_scales([w.cuda() for w in windows[:4]], chunk, margin=1.5) if kv == "fp8" else None
+    new = lambda: model.new_streaming_cache(streams + 2, max_past, chunk_frames=chunk, seed=5, kv_scales=scales)
+    cache, replayed = new(), new()
+    slots = [int(s) for s in np.random.default_rng(4).permutation(streams + 2)[:streams]]
+    check = [0, streams // 2, streams - 1]
+    states = {s: OC.StreamState(ocfg) for s in check}
+    PR = {k: (v.to(torch.bfloat16).float() if v.ndim >= 2 else v) for k, v in P.items()}
+    floor_states = {s: OC.StreamState(ocfg) for s in check}
+    got_rows, want_rows, floor_rows, graph = [], [], [], None
+    for c in range(chunks):
+        lp = model.forward_chunk_paged(windows[c].cuda(), slots, cache)
+        if graph is None:
+            graph = model.graphed_chunk_forward(replayed, streams, window)
+        assert torch.equal(graph(windows[c].cuda(), slots)[0], lp), c
+        assert ob.device_status() == 0
+        lp = lp.cpu()
+        for s in check:
+            with torch.no_grad():
+                want_rows.append(OC.forward_chunk(P, ocfg, states[s], windows[c][s], max_past))
+                floor_rows.append(OC.forward_chunk(PR, ocfg, floor_states[s], windows[c][s], max_past))
+            got_rows.append(lp[s])
+    got, want, floor = torch.cat(got_rows), torch.cat(want_rows), torch.cat(floor_rows)
+    mx, mean, _, agree_clear = _stats(got, want, ocfg.vocab, f"streaming d512 x4, {streams} streams x {chunks} chunks, {kv} pages")
+    _, fmean, _, _ = _stats(floor, want, ocfg.vocab, "same streams, fp32 oracle with bf16 weight matrices")
+    slack = 1.3 if kv == "bf16" else 1.6
+    assert mx <= (MAX_ABS if kv == "bf16" else 3e-2)
+    assert mean <= max(MEAN_ABS, slack * fmean), (mean, fmean)
+    assert agree_clear >= (ARGMAX_AGREE if kv == "bf16" else 0.99)
