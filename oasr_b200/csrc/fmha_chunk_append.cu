@@ -204,7 +204,8 @@ fmha_chunk_append_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
         const T* src = reinterpret_cast<const T*>(p.qkv4) + static_cast<int64_t>(b) * p.Tq * p.ld + h * D;
         const int64_t d = static_cast<int64_t>(p.H) * D;
         for (int i = threadIdx.x; i < p.Tq * 8; i += kWarps * 32) {       // eight values of a key and of a value
-          const int t_new = i >> 3, part = i & 7, at = cached + t_new, logical = at / p.block_size;
+          const int t_new = i >> 3, part = i & 7;
+          const int64_t at = static_cast<int64_t>(cached) + t_new, logical = at / p.block_size;   // any int32 may be in the table
           if (at < 0 || logical >= p.blocks_per_seq) continue;            // outside the table: dropped, never written
           const int page = row[logical];
           if (page < 0 || page >= p.num_blocks) continue;

@@ -117,3 +117,23 @@ def test_pages_and_attention_of_a_step(entry, dtype, fp8, block, pages, T):
         bound = vv.abs().max() * (2 * p_unit + 2 * score + n * 2.0 ** -24) + unit * out.abs() + 1e-5
         err = (got[b].double().view(T, H, D) - out).abs()
         assert bool((err <= bound).all()), (b, cached[b], (err - bound).max().item(), err.max().item())
+
+
+@pytest.mark.parametrize("entry", ENTRIES)
+def test_append_positions_that_leave_32_bits_or_begin_below_zero(entry):
+    """No row outside the table is written, and none inside it by a position that wrapped round."""
+    block, pages, T, d = 16, 4, 16, CFG.d_model
+    cached = [2 ** 31 - 5, 2 ** 31 - 1, -3, -2 ** 31]
+    B = len(cached)
+    g = torch.Generator(device="cuda").manual_seed(41)
+    model = ConformerCTC(ConformerConfig(**{f: getattr(CFG, f) for f in ConformerConfig.__dataclass_fields__}), OC.init_params(CFG, 77, 0.1))
+    model.forward_chunk_paged(torch.zeros(1, 67, 80, device="cuda"), [0], model.new_streaming_cache(1, 16))
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    table = torch.randperm(B * pages, generator=g, device="cuda").view(B, pages).int()
+    k, v = (torch.randn(CFG.layers, B * pages, block, CFG.heads, 64, generator=g, device="cuda").bfloat16() for _ in range(2))
+    want_k, want_v = k[-1].clone(), v[-1].clone()
+    qkv4, _ = _step(entry, model, torch.randn(B * T, model._native_model.embed_in, generator=g, device="cuda").bfloat16(), B, T, list(k), list(v),
+                    table, ints(cached), ints([T] * B), ints([0] * B), None, torch.zeros(CFG.layers, B, CFG.kernel - 1, d, device="cuda").bfloat16())
+    fresh = qkv4.view(B, T, 4, CFG.heads, 64)
+    want_k[table[2, 0].long(), :T - 3], want_v[table[2, 0].long(), :T - 3] = fresh[2, 3:, 2], fresh[2, 3:, 3]
+    assert torch.equal(k[-1], want_k) and torch.equal(v[-1], want_v)
