@@ -8,7 +8,7 @@
 #include <vector>
 
 #include "common.cuh"
-#include "fmha_chunk_append.cuh"
+#include "fmha_chunk.cuh"
 #include "gemm_small.cuh"
 
 namespace ob {
@@ -475,8 +475,8 @@ static int chunk_paged(const oasr_b200_conformer_model* model, const void* rows,
     }
     const float* ks = kv_scales ? kv_scales + static_cast<int64_t>(i) * 2 * m.heads : nullptr;   // fp8 pages: scales of K, then V
     const float* vs = ks ? ks + m.heads : nullptr;
-    if (merged && fmha_chunk_append::applies(B, m.heads, T, block_size, blocks_per_seq, k_pools[i], v_pools[i])) {   // few streams: in one kernel
-      OB_STEP("fmha_paged_relpos", 0, fmha_chunk_append::run(w.att, w.qkv4, k_pools[i], v_pools[i], ks, vs,
+    if (merged && fmha_chunk::applies_append(B, m.heads, T, block_size, blocks_per_seq, k_pools[i], v_pools[i])) {   // few streams: in one kernel
+      OB_STEP("fmha_paged_relpos", 0, fmha_chunk::run(w.att, w.qkv4, k_pools[i], v_pools[i], ks, vs,
                                        static_cast<const uint8_t*>(m.pos_proj) + i * d * 2, m.pos_proj_rows, L * d, pos_start, block_table,
                                        total_seqlens, B, T, m.heads, blocks_per_seq, block_size, num_blocks, scale, dt, static_cast<cudaStream_t>(stream), cache_seqlens));
     } else if (kv_scales) {

@@ -36,6 +36,7 @@
 
 #include "common.cuh"
 #include "device_status.cuh"
+#include "fmha_chunk.cuh"
 #include "sm100_ptx.cuh"
 #include "smem_limit.cuh"
 #include "tma_host.cuh"
@@ -644,15 +645,6 @@ int plan(void* plan_buf, const int32_t* cu_seqlens, int64_t num_segs, int64_t H,
 }  // namespace fmha_relpos
 extern int g_fmha_relpos_path;
 
-namespace fmha_chunk {   // fmha_chunk.cu: warp-per-(stream, head) kernel for <= 16 query frames
-bool applies(int64_t Tq, int64_t block_size, int64_t blocks_per_seq);
-bool applies_fp8(int64_t Tq, int64_t block_size, int64_t blocks_per_seq);
-int run(void* out, const void* qkv4, void* k_pool, void* v_pool, const float* k_scale, const float* v_scale, const void* pos,
-        int64_t pos_rows, int64_t pos_stride, const int32_t* pos_start, const int32_t* block_table, const int32_t* seqlens,
-        int64_t B, int64_t Tq, int64_t H, int64_t blocks_per_seq, int64_t block_size, int64_t num_blocks, double scale,
-        int dtype, cudaStream_t stream);
-}  // namespace fmha_chunk
-
 }  // namespace ob
 
 extern "C" {
@@ -755,7 +747,7 @@ int oasr_b200_fmha_paged_relpos(void* out, const void* qkv4, void* k_pool, void*
   if (fmha_chunk::applies(Tq, block_size, blocks_per_seq))
     return fmha_chunk::run(out, qkv4, k_pool, v_pool, nullptr, nullptr, pos, pos_rows, pos_stride, pos_start, block_table,
                            seqlens, B, Tq, H, blocks_per_seq, block_size, num_blocks, scale, dtype,
-                           static_cast<cudaStream_t>(stream));
+                           static_cast<cudaStream_t>(stream), nullptr);
   const int64_t d = H * D, ld = 4 * d;
   const uint8_t* base = static_cast<const uint8_t*>(qkv4);
   Maps maps;
@@ -798,7 +790,7 @@ int oasr_b200_fmha_paged_relpos_fp8(void* out, const void* qkv4, void* k_pool, v
              OASR_ERR_ALIGN, "fmha_paged_relpos_fp8: operands must be 16-byte aligned");
   return fmha_chunk::run(out, qkv4, k_pool, v_pool, k_scale, v_scale, pos, pos_rows, pos_stride, pos_start, block_table,
                          seqlens, B, Tq, H, blocks_per_seq, block_size, num_blocks, scale, dtype,
-                         static_cast<cudaStream_t>(stream));
+                         static_cast<cudaStream_t>(stream), nullptr);
 }
 
 static int fmha_dense_or_paged(void* out, const void* q, const void* k, const void* v, const int64_t* q_strides,

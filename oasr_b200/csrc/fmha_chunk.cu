@@ -5,12 +5,17 @@
 //
 // With 16 query rows the contraction is tiny (about 24 flop per byte of K/V/P read) and the
 // kernel is bound by how fast pages stream out of HBM, so the layout is chosen for memory-level
-// parallelism, not for the tensor pipe: one WARP owns one (stream, head) and runs its own
-// two-stage TMA ring of 32-key slices (K page rows, the matching rows of the projected position
-// table, V page rows; 128-byte swizzle) behind per-warp mbarriers -- no block-wide barrier after
-// set-up, eight independent pipelines per CTA, ~100 KB of loads in flight per SM.  The 16-row
-// products run on warp-level m16n8k16 MMAs fed by ldmatrix (a 128-row tcgen05 tile would waste 7/8
-// of its rows here); the softmax is the usual online form in the log2 domain with fp32 state.
+// parallelism, not for the tensor pipe: every WARP runs its own two-stage TMA ring of 32-key
+// slices (K page rows, the matching rows of the projected position table, V page rows; 128-byte
+// swizzle) behind per-warp mbarriers, ~100 KB of loads in flight per block.  The 16-row products
+// run on warp-level m16n8k16 MMAs fed by ldmatrix (a 128-row tcgen05 tile would waste 7/8 of its
+// rows here); the softmax is the usual online form in the log2 domain with fp32 state.
+// Two forms of one kernel:
+//   a warp per (stream, head), eight of them per block, no block-wide barrier after set-up;
+//   kAppend, few streams, where one item's chain of slices is all of the time: a block of four warps per (stream, head), two
+//   blocks per SM.  Warp w takes the slices w, w + 4, ...; the four partial results are added in warp order at the end.  The
+//   block also appends the chunk's keys and values to their pages, while its first slices of cached keys are on their way (a
+//   launch of its own otherwise).  The sums run in another order than with a warp per item, so the two forms differ in last bits.
 //
 // Reference semantics: RelPositionMultiHeadedAttention.forward_paged
 // (oasr/layers/attention/attention.py:388-470) + paged fmha (oasr/functionals/attention.py:369-551):
@@ -22,6 +27,8 @@
 
 #include "common.cuh"
 #include "device_status.cuh"
+#include "e4m3.cuh"
+#include "fmha_chunk.cuh"
 #include "sm100_ptx.cuh"
 #include "smem_limit.cuh"
 #include "tma_host.cuh"
@@ -31,14 +38,17 @@ int g_fmha_chunk_path = 1;  // 1 = this kernel where it applies; 0 = always the 
 
 namespace fmha_chunk {
 
-constexpr int kWarps = 8;
 constexpr int kKeys = 32;                   // keys per pipeline stage
 constexpr int kStages = 2;
 constexpr int kTileBytes = kKeys * 128;     // 32 rows x 64 x 2 B
 constexpr int kStageBytes = 3 * kTileBytes; // K | pos | V
-constexpr int kSmemBars = kWarps * kStages * kStageBytes;
-constexpr int kSmemTotal = kSmemBars + kWarps * kStages * 8 + 16;
-constexpr int kSmemDynamic = kSmemTotal + 1024;
+template <bool kAppend>
+struct Form {
+  static constexpr int kWarps = kAppend ? 4 : 8;
+  static constexpr int kSmemBars = kWarps * kStages * kStageBytes;
+  static constexpr int kSmemMl = kSmemBars + kWarps * kStages * 8 + 16;   // kAppend: running maximum and sum of 16 rows per warp
+  static constexpr int kSmemDynamic = kSmemMl + (kAppend ? kWarps * 16 * 8 : 0) + 1024;
+};
 constexpr int D = 64;
 
 struct Params {
@@ -54,6 +64,8 @@ struct Params {
   uint32_t* status;
   const float* k_scale;  // fp8 pages: [H] per-head scales of the K / V codes (x ~ code * scale)
   const float* v_scale;
+  const int32_t* append_at;   // kAppend: the chunk's keys / values (columns 2 d.., 3 d.. of qkv4) go to these positions first
+  uint8_t *k_pool, *v_pool;
 };
 
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
@@ -93,20 +105,22 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 // K scale once when it loads it (as fp16) and the output by the V scale once at the end.  The content product and
 // P.V then run as fp16 MMAs, the position product stays in T; all accumulate in the same fp32 registers.
 // Per warp: 2 stages x 8 KB + 2 x 4 KB working tiles = the same 24 KB as the 16-bit ring.
-template <typename T, bool kFp8>
-__global__ void __launch_bounds__(kWarps * 32, 1)
+template <typename T, bool kFp8, bool kAppend>
+__global__ void __launch_bounds__(Form<kAppend>::kWarps * 32, kAppend ? 2 : 1)
 fmha_chunk_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                   const __grid_constant__ CUtensorMap map_pos, const Params p) {
+  using F = Form<kAppend>;
+  constexpr int kWarps = F::kWarps;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int kStageB = kFp8 ? 2 * (kTileBytes / 2) + kTileBytes : kStageBytes;   // fp8: K8 2 KB | V8 2 KB | pos 4 KB
-  constexpr int kPosOff = kFp8 ? kTileBytes : kTileBytes;                           // position rows sit 4 KB into a stage either way
+  constexpr int kPosOff = kTileBytes;                                               // position rows sit 4 KB into a stage either way
   using TC = typename std::conditional<kFp8, __half, T>::type;                      // operand type of the content / P.V MMAs
   uint8_t* ring = smem + warp * kStages * kStageBytes;
   uint8_t* work = ring + kStages * kStageB;                                         // fp8 only: K and V working tiles (fp16)
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kSmemBars) + warp * kStages;
-  volatile uint32_t* abort_flag = reinterpret_cast<uint32_t*>(smem + kSmemBars + kWarps * kStages * 8);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + F::kSmemBars) + warp * kStages;
+  volatile uint32_t* abort_flag = reinterpret_cast<uint32_t*>(smem + F::kSmemBars + kWarps * kStages * 8);
   if (threadIdx.x == 0) *abort_flag = 0;
   if (lane == 0) {
     for (int s = 0; s < kStages; ++s) ptx::mbar_init(&bars[s], 1);
@@ -117,17 +131,19 @@ fmha_chunk_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
   ptx::grid_dep_launch();   // no-ops unless launched with programmatic stream serialisation
   ptx::grid_dep_wait();
   bool ok = true;
-  const int item = blockIdx.x * kWarps + warp;
-  const bool live = item < p.B * p.H;   // warp-uniform; dead warps skip to the common exit
-  if (live) {
+  const int item = kAppend ? blockIdx.x : blockIdx.x * kWarps + warp;
+  if (kAppend || item < p.B * p.H) {   // warp-uniform; warps without an item skip to the common exit
     const int b = item / p.H, h = item - b * p.H;
     const int kv_len = min(max(p.seqlens[b], 0), p.blocks_per_seq * p.block_size);
-    const int n_it = (kv_len + kKeys - 1) / kKeys;
+    const int slices = (kv_len + kKeys - 1) / kKeys;
+    const int n_it = !kAppend ? slices : slices > warp ? (slices - warp + kWarps - 1) / kWarps : 0;
+    const int key_lo = kAppend ? warp * kKeys : 0;                     // first key of the slice of iteration `it`: key_lo + it * kStep
+    constexpr int kStep = kAppend ? kWarps * kKeys : kKeys;
     const int pos0 = p.pos_start[b];
     const int g = lane >> 2, t = lane & 3;
     T* out = static_cast<T*>(p.out) + (static_cast<int64_t>(b) * p.Tq * p.H + h) * D;
     const int64_t out_ld = static_cast<int64_t>(p.H) * D;
-    if (n_it == 0) {   // no visible key: zero rows
+    if (!kAppend && n_it == 0) {   // no visible key: zero rows
       for (int i = lane; i < p.Tq * (D / 8); i += 32)
         *reinterpret_cast<uint4*>(out + (i / (D / 8)) * out_ld + (i % (D / 8)) * 8) = make_uint4(0, 0, 0, 0);
     } else {
@@ -139,7 +155,7 @@ fmha_chunk_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
       pg_hi = min(max(pg_hi, 0), p.num_blocks - 1);
       const bool small_pages = p.block_size == 16;   // else block_size is a multiple of 32
       auto issue = [&](int it, int s) {   // warp-collective: shuffles by all lanes, TMA by lane 0
-        const int key0 = it * kKeys;
+        const int key0 = key_lo + it * kStep;
         int col0 = min(key0 / p.block_size, p.blocks_per_seq - 1);
         int col1 = min(col0 + 1, p.blocks_per_seq - 1);
         const int a0 = __shfl_sync(0xffffffffu, pg_lo, col0 & 31), a1 = __shfl_sync(0xffffffffu, pg_hi, col0 & 31);
@@ -173,8 +189,40 @@ fmha_chunk_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
           ptx::tma_load_4d(dst + kPosOff, &map_pos, 0, pos0 + key0, h, 0, &bars[s]);
         }
       };
-      issue(0, 0);
-      if (n_it > 1) issue(1, 1);
+      if constexpr (kAppend) {
+        // slices of cached keys only go out before the chunk's own keys and values are in their pages
+        const int cached = p.append_at[b];
+        const bool early0 = n_it > 0 && key_lo + kKeys <= cached, early1 = n_it > 1 && key_lo + kStep + kKeys <= cached;
+        if (early0) issue(0, 0);
+        if (early1) issue(1, 1);
+        const T* src = reinterpret_cast<const T*>(p.qkv4) + static_cast<int64_t>(b) * p.Tq * p.ld + h * D;
+        const int64_t d = static_cast<int64_t>(p.H) * D;
+        for (int i = threadIdx.x; i < p.Tq * 8; i += kWarps * 32) {       // eight values of a key and of a value
+          const int t_new = i >> 3, part = i & 7;
+          const int64_t at = static_cast<int64_t>(cached) + t_new, logical = at / p.block_size;   // any int32 may be in the table
+          if (at < 0 || logical >= p.blocks_per_seq) continue;            // outside the table: dropped, never written
+          const int page = row[logical];
+          if (page < 0 || page >= p.num_blocks) continue;
+          const int64_t dst = ((static_cast<int64_t>(page) * p.block_size + at % p.block_size) * p.H + h) * D + part * 8;
+          const Pack<T> kv = ld128(src + t_new * p.ld + 2 * d + part * 8);
+          const Pack<T> vv = ld128(src + t_new * p.ld + 3 * d + part * 8);
+          if constexpr (kFp8) {
+            *reinterpret_cast<uint2*>(p.k_pool + dst) = to_e4m3x8<T>(kv, 1.f / p.k_scale[h]);
+            *reinterpret_cast<uint2*>(p.v_pool + dst) = to_e4m3x8<T>(vv, 1.f / p.v_scale[h]);
+          } else {
+            st128(reinterpret_cast<T*>(p.k_pool) + dst, kv);
+            st128(reinterpret_cast<T*>(p.v_pool) + dst, vv);
+          }
+        }
+        __threadfence();                                                  // written here, read back by TMA
+        asm volatile("fence.proxy.async;" ::: "memory");
+        __syncthreads();
+        if (n_it > 0 && !early0) issue(0, 0);
+        if (n_it > 1 && !early1) issue(1, 1);
+      } else {
+        issue(0, 0);
+        if (n_it > 1) issue(1, 1);
+      }
 
       // Q fragments (A operand, 16 x 64 each) straight from global memory; rows >= Tq are zero
       uint32_t qu[4][4], qv[4][4];
@@ -262,7 +310,7 @@ fmha_chunk_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
           }
         }
         // ---- online softmax (log2 domain); rows g and g+8 ----
-        const int key0 = it * kKeys;
+        const int key0 = key_lo + it * kStep;
         float tmax[2] = {-INFINITY, -INFINITY};
 #pragma unroll
         for (int n = 0; n < 4; ++n) {
@@ -318,12 +366,61 @@ fmha_chunk_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
         __syncwarp();
         if (it + kStages < n_it) issue(it + kStages, s);
       }
-      if (ok) {
+      auto whole_row = [&] {   // the sum of a row's four lanes
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
           l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 1);
           l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 2);
         }
+      };
+      if constexpr (kAppend) {
+        whole_row();
+        if (!ok && lane == 0 && p.status) atomicOr(p.status, kStatusFmhaLoad);
+        // the warps' parts meet in shared memory (this warp's ring, which it has read for the last time)
+        float2* ml = reinterpret_cast<float2*>(smem + F::kSmemMl);
+        float4* mine = reinterpret_cast<float4*>(ring);
+        __syncwarp();
+#pragma unroll
+        for (int n = 0; n < 8; ++n) mine[n * 32 + lane] = make_float4(o[n][0], o[n][1], o[n][2], o[n][3]);
+        if (t == 0) {
+          ml[warp * 16 + g] = make_float2(m_run[0], l_run[0]);
+          ml[warp * 16 + g + 8] = make_float2(m_run[1], l_run[1]);
+        }
+        __syncthreads();
+        if (!*abort_flag) {
+          float f[kWarps][2], inv[2];
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            float m_all = -INFINITY, l_all = 0.f;
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) m_all = fmaxf(m_all, ml[w * 16 + g + r * 8].x);
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) {
+              const float2 part = ml[w * 16 + g + r * 8];
+              f[w][r] = part.x == -INFINITY ? 0.f : exp2f(part.x - m_all);
+              l_all = fmaf(part.y, f[w][r], l_all);
+            }
+            inv[r] = l_all > 0.f ? 1.f / l_all : 0.f;                       // no visible key: zero rows
+            if constexpr (kFp8) inv[r] *= p.v_scale[h];
+          }
+#pragma unroll
+          for (int i = 0; i < 8 / kWarps; ++i) {                            // a warp finishes two blocks of eight columns
+            const int n = warp * (8 / kWarps) + i, c = n * 8 + 2 * t;
+            float a[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) {
+              const float4 v = reinterpret_cast<const float4*>(smem + w * kStages * kStageBytes)[n * 32 + lane];
+              a[0] = fmaf(v.x, f[w][0], a[0]);
+              a[1] = fmaf(v.y, f[w][0], a[1]);
+              a[2] = fmaf(v.z, f[w][1], a[2]);
+              a[3] = fmaf(v.w, f[w][1], a[3]);
+            }
+            if (g < p.Tq) *reinterpret_cast<uint32_t*>(out + g * out_ld + c) = pack2<T>(a[0] * inv[0], a[1] * inv[0]);
+            if (g + 8 < p.Tq) *reinterpret_cast<uint32_t*>(out + (g + 8) * out_ld + c) = pack2<T>(a[2] * inv[1], a[3] * inv[1]);
+          }
+        }
+      } else if (ok) {
+        whole_row();
         float inv0 = l_run[0] > 0.f ? 1.f / l_run[0] : 0.f;
         float inv1 = l_run[1] > 0.f ? 1.f / l_run[1] : 0.f;
         if constexpr (kFp8) {
@@ -368,15 +465,25 @@ int make_map_u8(CUtensorMap* m, const void* base, int64_t block_size, int64_t he
 }
 
 bool applies(int64_t Tq, int64_t block_size, int64_t blocks_per_seq) {
-  return g_fmha_chunk_path && Tq <= 16 && (block_size == 16 || block_size % 32 == 0) && blocks_per_seq <= 64;
+  return g_fmha_chunk_path && applies_fp8(Tq, block_size, blocks_per_seq);
 }
 bool applies_fp8(int64_t Tq, int64_t block_size, int64_t blocks_per_seq) {
   return Tq <= 16 && (block_size == 16 || block_size % 32 == 0) && blocks_per_seq <= 64;
 }
+// A block per (stream, head) is ahead while all of them are resident at once (two per SM): one stream 8.8 us and a page write
+// of 2.7 us before, a step of 12 chunks 11.5 -> 10.9 ms; 37 streams 24.1 -> 22.5 ms.  Beyond that the pages' bandwidth sets the
+// time, a block's own latencies come on top of every wave, and a warp per item (fmha_chunk.cu) is ahead: 256 streams with fp8
+// pages 52.8 ms there, 58.6 ms here.
+bool applies_append(int64_t B, int64_t H, int64_t Tq, int64_t block_size, int64_t blocks_per_seq, const void* k_pool, const void* v_pool) {
+  return applies(Tq, block_size, blocks_per_seq) && B * H <= 2 * sm_count() && Tq >= 1 && block_size > 0 && 128 % block_size == 0 &&
+         blocks_per_seq >= 1 && is_aligned(k_pool, 16) && is_aligned(v_pool, 16);
+}
 
-template <typename T, bool kFp8>
-int launch(const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mp, const Params& p, unsigned grid, cudaStream_t stream) {
-  auto kern = fmha_chunk_kernel<T, kFp8>;
+template <typename T, bool kFp8, bool kAppend>
+int launch(const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mp, const Params& p, cudaStream_t stream) {
+  constexpr int kWarps = Form<kAppend>::kWarps, kSmemDynamic = Form<kAppend>::kSmemDynamic;
+  const unsigned grid = static_cast<unsigned>(kAppend ? p.B * p.H : (p.B * p.H + kWarps - 1) / kWarps);
+  auto kern = fmha_chunk_kernel<T, kFp8, kAppend>;
   static SmemLimit smem_limit;
   const cudaError_t e = smem_limit.raise(kern, kSmemDynamic);
   if (e != cudaSuccess)
@@ -386,11 +493,10 @@ int launch(const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mp, 
   return check_launch("fmha_paged_relpos (chunk kernel) launch");
 }
 
-// k_scale / v_scale null: 16-bit pools; otherwise the pools hold fp8 e4m3 codes with per-head scales.
 int run(void* out, const void* qkv4, void* k_pool, void* v_pool, const float* k_scale, const float* v_scale, const void* pos,
         int64_t pos_rows, int64_t pos_stride, const int32_t* pos_start, const int32_t* block_table, const int32_t* seqlens,
         int64_t B, int64_t Tq, int64_t H, int64_t blocks_per_seq, int64_t block_size, int64_t num_blocks, double scale,
-        int dtype, cudaStream_t stream) {
+        int dtype, cudaStream_t stream, const int32_t* append_at) {
   const int64_t d = H * D;
   const int box_rows = block_size == 16 ? 16 : 32;
   const bool fp8 = k_scale != nullptr;
@@ -412,9 +518,10 @@ int run(void* out, const void* qkv4, void* k_pool, void* v_pool, const float* k_
   p.blocks_per_seq = (int)blocks_per_seq; p.block_size = (int)block_size; p.num_blocks = (int)num_blocks;
   p.out = out; p.status = device_status_ptr();
   p.k_scale = k_scale; p.v_scale = v_scale;
-  const unsigned grid = (unsigned)((B * H + kWarps - 1) / kWarps);
+  p.append_at = append_at; p.k_pool = static_cast<uint8_t*>(k_pool); p.v_pool = static_cast<uint8_t*>(v_pool);
   return OB_DISPATCH_HALF(dtype, T, [&]() -> int {
-    return fp8 ? launch<T, true>(mk, mv, mp, p, grid, stream) : launch<T, false>(mk, mv, mp, p, grid, stream);
+    if (append_at) return fp8 ? launch<T, true, true>(mk, mv, mp, p, stream) : launch<T, false, true>(mk, mv, mp, p, stream);
+    return fp8 ? launch<T, true, false>(mk, mv, mp, p, stream) : launch<T, false, false>(mk, mv, mp, p, stream);
   });
 }
 

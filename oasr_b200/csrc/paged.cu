@@ -5,9 +5,8 @@
 // Index rule (oasr/cache/paged_kv.py:23-40 in the reference): logical frame
 // pos = offsets[b] + t of stream b lives at physical pool row
 //   block_table[b, pos / block_size] * block_size + pos % block_size.
-#include <cuda_fp8.h>
-
 #include "common.cuh"
+#include "e4m3.cuh"
 #include "sm100_ptx.cuh"
 
 namespace ob {
@@ -140,20 +139,6 @@ struct PagedWriteFp8Args {
   int64_t stride_b, stride_h, stride_t;  // elements
   int64_t blocks_per_seq, block_size, num_blocks;
 };
-
-template <typename T>
-__device__ __forceinline__ uint2 to_e4m3x8(const Pack<T>& v, float inv) {
-  uint32_t w[2];
-#pragma unroll
-  for (int hh = 0; hh < 2; ++hh) {
-    const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(Elem<T>::to_f(v.v[hh * 4]) * inv, Elem<T>::to_f(v.v[hh * 4 + 1]) * inv),
-                                                 __NV_SATFINITE, __NV_E4M3);
-    const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(Elem<T>::to_f(v.v[hh * 4 + 2]) * inv, Elem<T>::to_f(v.v[hh * 4 + 3]) * inv),
-                                                 __NV_SATFINITE, __NV_E4M3);
-    w[hh] = lo | (hi << 16);
-  }
-  return make_uint2(w[0], w[1]);
-}
 
 template <typename T>
 __global__ void __launch_bounds__(256) paged_kv_write_fp8_kernel(PagedWriteFp8Args a) {
