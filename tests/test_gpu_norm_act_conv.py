@@ -359,3 +359,28 @@ def test_subsampling_second_conv_at_every_tile_width(C, N, frames, dtype):
         bound = eps * want.abs() + 9 * C * 2.0 ** -24 * size
         assert bool(((got[at:at + n] - want).abs() <= bound).all()), (i, ((got[at:at + n] - want).abs() - bound).max().item())
         at += n
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("C,N", [(64, 128), (64, 256), (512, 512)])
+def test_subsampling_second_conv_gives_an_utterance_the_same_bits_in_every_batch(C, N, dtype):
+    """A batch's size chooses the columns of a tile, 64 to N; the first utterances' rows are those of each of them alone."""
+    from oasr_b200 import fused
+
+    g = torch.Generator(device="cuda").manual_seed(N)
+    F1, F2, n, most = 39, 19, 6, 96
+    T1 = 2 * n + 1
+    x = torch.randn(most, (T1 + 1) // 2, 4, (F1 + 1) // 2, C, generator=g, device="cuda").to(dtype)      # parity planes
+    w = (torch.randn(N, 3, 3, C, generator=g, device="cuda") * (9 * C) ** -0.5).to(dtype)
+    b = (torch.randn(N, generator=g, device="cuda") * 0.1).to(dtype)
+
+    def conv(utts):
+        cu = torch.arange(0, (utts + 1) * n, n, dtype=torch.int32, device="cuda")
+        return fused.subsample_conv2(x[:utts].contiguous(), T1, F1, w, b, cu, utts * n).clone()
+
+    want = conv(most)
+    assert ob.device_status() == 0 and torch.isfinite(want).all()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for utts in (1, sms // 16, sms // 16 + 1, sms // 8, sms // 8 + 1, sms // 4, sms // 4 + 1, most - 1):
+        got = conv(utts)
+        assert torch.equal(got, want[:got.size(0)]), utts
