@@ -106,16 +106,19 @@ OASR_API unsigned long long oasr_b200_launch_count(void);
 /* Process-wide integer tunables.  "gemm_bn": 0 = heuristic tile width, or 64 /
  * 128 / 256 to force it; "gemm_pairs": dense GEMMs on CTA pairs
  * (tcgen05 cta_group::2) where they are ahead (2, default), wherever they can run (1), never (0);
- * "dwconv_path": 0 (default) = register-streaming depthwise conv where it
- * applies, 1 = the shared-memory tiled kernel; "fmha_chunk_path": 1 (default)
- * = paged rel-pos attention with <= 16 query frames runs the warp-per-(stream,
- * head) kernel, 0 = always the 128-row tcgen05 kernel; "fmha_relpos_path": 1 (default) =
+ * "dwconv_path": 2 (default) = the rolling depthwise conv for kernel sizes 9 and
+ * 15, 0 = the register-streaming one, 1 = the shared-memory tiled one;
+ * "fmha_chunk_path": 1 (default) = paged rel-pos attention with <= 16 query
+ * frames runs the streaming-chunk kernel: a warp per (stream, head), or inside
+ * oasr_b200_conformer_chunk_paged with few streams a block that also appends the
+ * chunk to its pages; 0 = the 128-row tcgen05 kernel behind a page write (fp8
+ * pages: the warp-per-(stream, head) form behind one); "fmha_relpos_path": 1 (default) =
  * packed relative-position attention on the two-CTAs-per-SM kernel (64-key tiles),
  * 0 = on the general kernel; "lsm_path": the CTC head, 0 (default) = by size, 1 = the fused two-sweep
  * kernel, 2 = fp32 logits GEMM + in-place row log-softmax kernel (fp32 output only); "pdl": 1 launches
  * the GEMM, attention, add+norm, depthwise-conv and quantise kernels with
  * programmatic stream serialisation (their set-up overlaps the previous
- * kernel's tail), 0 (default) = plain stream order (no reference counterpart; the reference selects tiles
+ * kernel's tail; default), 0 = plain stream order (no reference counterpart; the reference selects tiles
  * through its JIT variant names, oasr/jit/gemm.py:863-880). */
 OASR_API int oasr_b200_set_tunable(const char* name, int value);
 

@@ -17,9 +17,15 @@
 //
 // A few utterances or streams fill few pairs, and then the main loop of one tile over all N channels is all of the time: 72
 // blocks of 1024 tensor clocks for N = 512.  So where pairs are free they share a tile's columns, down to 64 each (grid.y;
-// the order of K, hence every bit, stays): N = 512, 1 to 37 output frames 50 -> 22 us (256 columns 27, 128 columns 22.5; a
-// K block then costs its operands' trip from L2, not its products), 16 streams of 16 frames 57 -> 31 us; N = 256 16.5 ->
-// 13 us.  With more tiles than half of the pairs nothing changes.
+// the order of K, hence every bit, stays).  Launches in a row, us by the width of a tile:
+//   output frames          512    256    128     64
+//   N 512    1 x 6         50.0   26.6   21.7   21.1     (from 128 on a K block costs its operands' trip from L2, not its products)
+//            1 x 74        50.7   27.3   22.8   22.1
+//            8 x 16        50.6   27.9   22.9   43.4     (64: a second wave)
+//           16 x 16        52.8   28.8   45.5
+//   N 256    1 x 6                17.1   13.3   12.5
+//           16 x 16               17.7   14.5   26.3
+// With more tiles than half of the pairs nothing changes.
 #include <cuda.h>
 
 #include <type_traits>

@@ -15,7 +15,8 @@
 //   kAppend, few streams, where one item's chain of slices is all of the time: a block of four warps per (stream, head), two
 //   blocks per SM.  Warp w takes the slices w, w + 4, ...; the four partial results are added in warp order at the end.  The
 //   block also appends the chunk's keys and values to their pages, while its first slices of cached keys are on their way (a
-//   launch of its own otherwise).  The sums run in another order than with a warp per item, so the two forms differ in last bits.
+//   launch of its own otherwise).  The sums run in another order than with a warp per item, so the two forms differ in last
+//   bits; against fp64 this one's rms error is 0.965 to 1.000 of the other's (16 to 1024 keys, both types and page kinds).
 //
 // Reference semantics: RelPositionMultiHeadedAttention.forward_paged
 // (oasr/layers/attention/attention.py:388-470) + paged fmha (oasr/functionals/attention.py:369-551):
@@ -470,10 +471,14 @@ bool applies(int64_t Tq, int64_t block_size, int64_t blocks_per_seq) {
 bool applies_fp8(int64_t Tq, int64_t block_size, int64_t blocks_per_seq) {
   return Tq <= 16 && (block_size == 16 || block_size % 32 == 0) && blocks_per_seq <= 64;
 }
-// A block per (stream, head) is ahead while all of them are resident at once (two per SM): one stream 8.8 us and a page write
-// of 2.7 us before, a step of 12 chunks 11.5 -> 10.9 ms; 37 streams 24.1 -> 22.5 ms.  Beyond that the pages' bandwidth sets the
-// time, a block's own latencies come on top of every wave, and a warp per item (fmha_chunk.cu) is ahead: 256 streams with fp8
-// pages 52.8 ms there, 58.6 ms here.
+// Few streams: all blocks resident at once, two per SM.  A graph-replayed step of 8 heads and 12 layers with 272 keys per
+// stream, in us, page write and a warp per item -> this form:
+//   streams           1             37             38             48             74            100            256
+//   16-bit pages   905 -> 778   1165 -> 1055   1171 -> 1123   1214 -> 1166   1483 -> 1483   1697 -> 1782   2625 -> 2964
+//   fp8 pages      979 -> 797   1254 -> 1065   1256 -> 1178   1290 -> 1211   1546 -> 1495   1749 -> 1802   2676 -> 3004
+// Each further wave of blocks pays a block's own latencies again; in the third (100 streams) the warp per item, which asks
+// for more pages at a time, is ahead.  The line lies at the end of the first wave, where the gain is largest; the second,
+// up to 74 streams, still gains 0-6 % and is not taken.
 bool applies_append(int64_t B, int64_t H, int64_t Tq, int64_t block_size, int64_t blocks_per_seq, const void* k_pool, const void* v_pool) {
   return applies(Tq, block_size, blocks_per_seq) && B * H <= 2 * sm_count() && Tq >= 1 && block_size > 0 && 128 % block_size == 0 &&
          blocks_per_seq >= 1 && is_aligned(k_pool, 16) && is_aligned(v_pool, 16);

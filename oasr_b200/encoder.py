@@ -560,7 +560,7 @@ class ConformerCTC:
 class GraphedChunkForward:
     """One streaming step of ``batch`` streams x ``window`` feature frames, captured once into a CUDA graph and
     replayed per chunk (the reference captures its streaming encoder the same way: ``GraphedEncoderForward``,
-    oasr/engine/graph_cache.py:24-29).  The step is about 170 launches of a few microseconds each, so replaying one
+    oasr/engine/graph_cache.py:24-29).  The step is about 190 launches of a few microseconds each, so replaying one
     graph instead of enqueueing them takes the launch path off the host.  Everything that changes from chunk to chunk
     is data in fixed device buffers: the feature windows, the block-table rows, the cached / total lengths, the
     position starts and the slot ids; the page pools and conv states are the cache's own.  Outputs are the graph's

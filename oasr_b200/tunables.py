@@ -7,8 +7,9 @@ an in-place row log-softmax kernel (fp32 output only).
 (1) or never (0).
 ``dwconv_path``: 2 (default) runs the depthwise conv of kernel size 9 / 15 on the rolling register-window kernel (other sizes
 up to 15 on the run-at-once register-streaming kernel), 0 all of them on the run-at-once kernel, 1 on the shared-memory tiled one.
-``fmha_chunk_path``: 1 (default) runs paged rel-pos attention with <= 16 query frames on the warp-per-(stream, head)
-kernel, 0 always on the 128-row tcgen05 kernel.
+``fmha_chunk_path``: 1 (default) runs paged rel-pos attention with <= 16 query frames on the streaming-chunk kernel: a warp
+per (stream, head), or inside the Conformer's step of few streams a block that also appends the chunk to its pages; 0 on the
+128-row tcgen05 kernel behind a page write (fp8 pages: the warp-per-(stream, head) form behind one).
 ``fmha_relpos_path``: 1 (default) runs packed relative-position attention on the two-CTAs-per-SM kernel, 0 on the general one.
 ``conv1_mma``: 1 (default) runs the first subsampling convolution (parity-split output, 256 / 512 channels) as a K = 32
 split-bf16 GEMM on the tensor cores, 0 as the fp32 stencil kernel.
